@@ -1321,10 +1321,10 @@ static void run_pecvel(mx_ctx* c, const mx_grids* g, float redshift, cudaStream_
   pa.delta_T = g->delta_T;
   pa.TS = g->TS_box;
   pa.mode = p.flag_pecvel;
-  pa.H_z = H_z;
-  pa.redshift = redshift;
+  pa.inv_H = 1.0 / (double)H_z;
   pa.max_v_deriv = std::fabs((double)(0.2f * H_z));  // fabs(MAX_DVDR * H_z), MAX_DVDR = (float)0.2
   pa.T_rad = k::TCMB * (1. + redshift);
+  pa.mK = 1000. / (1. + (double)redshift);
   {
     Prof pr(c, "k_pecvel_cells", (p.flag_pecvel > 1 ? 16.0 : 12.0) * (double)gd.N, s);
     launch_pecvel_cells(pa, gd, s);
@@ -1342,8 +1342,9 @@ static void run_pecvel(mx_ctx* c, const mx_grids* g, float redshift, cudaStream_
       ra.x_pos_offset[i] = (float)(ra.subcell_width * (float)i + ra.subcell_width / 2.);
       ra.x_pos[i] = (float)(ra.x_pos_offset[i] / (ra.box / (float)gd.D));
     }
+    ra.inv_cell = (double)(float)gd.D / ra.box;
     ra.H_z = H_z;
-    Prof pr(c, "k_rsd_columns", 20.0 * (double)gd.N, s);
+    Prof pr(c, "k_rsd_columns", 16.0 * (double)gd.N, s);
     launch_rsd(ra, gd, s);
   }
 }

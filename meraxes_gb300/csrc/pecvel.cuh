@@ -15,10 +15,10 @@ struct PecvelArgs
   float* delta_T;     // REAL
   const float* TS;    // REAL
   int mode;           // Flag_IncludePecVelsFor21cm
-  float H_z;
-  float redshift;
+  double inv_H;        // 1 / H_z
   double max_v_deriv;  // fabs(MAX_DVDR * H_z)
   double T_rad;
+  double mK;           // 1000 / (1 + z)
 };
 
 struct RsdArgs
@@ -26,11 +26,12 @@ struct RsdArgs
   const float* vel;      // converted velocities, padded
   const float* delta_T;  // REAL, read
   const float* xH;       // REAL
-  float* los;            // REAL scratch (one column per thread)
-  float* delta_T_out;    // REAL, receives the remapped columns
+  float* los;            // REAL scratch of the columns that are remapped sequentially
+  float* delta_T_out;    // REAL, receives the remapped columns (may be delta_T)
   float x_pos[RSD_STEPS], x_pos_offset[RSD_STEPS];
   double box;            // BoxSize / h [Mpc]
   double subcell_width;
+  double inv_cell;       // cells per Mpc
   float H_z;
 };
 
