@@ -1,0 +1,596 @@
+// Frequency-integral tables of ComputeTs (ComputeTs.c:517-664) on the device:
+// per shell the frequency of unit optical depth (nu_tau_one,
+// XRayHeatingFunctions.c:229-375), then for every x_HII node the heating,
+// ionisation and Ly-alpha integrals over frequency (integrate_over_nu,
+// :672-800).  All in FP64 with the quadrature (QUADPACK QAG, 61 points) and
+// the root finder (Brent) of host_physics.cpp, so that the same intervals are
+// bisected and the same root is stepped to; build_freq_integrals there is
+// the same computation on host threads, for tables whose adaptive intervals
+// outgrow FREQ_INTERVALS (FreqDevResult::fail).
+//
+//   k_tau_lower       a block per shell: the 61 nodes of tau_X(nu) in 61
+//                     threads; their redshift factors do not depend on nu and
+//                     are kept over the steps of the root finder.
+//   k_freq_integrals  a block per (shell, table, x_HII node), the two halves
+//                     of a bisected interval in its two pairs of warps.
+//
+// Shells below unit optical depth at E0 share their lower limit, so their
+// integrals are the same numbers: the first of them is computed for all.
+//
+// On 16 host threads the tables took 8.4 ms per snapshot, longer than the
+// shells' transforms of any grid below 512^3.
+#include <cfloat>
+#include <cmath>
+#include <cstring>
+
+#include "freq_tables.cuh"
+#include "gk61.h"
+
+namespace mx {
+
+namespace {
+// per host thread: a call counts its own launches when contexts run concurrently
+thread_local int freq_launches = 0;
+
+constexpr int FREQ_INTERVALS = 128;
+constexpr int TAU_THREADS = 64;
+constexpr int INT_THREADS = 128;
+
+// Node and weight of the 61-point rule for thread j < 61 of a panel: 0..29
+// below the centre, 30..59 above, 60 the centre (x = 0).
+struct Rule
+{
+  double x, wk, wg;
+};
+
+__constant__ Gk61 c_rule = GK61;
+
+__device__ __forceinline__ Rule rule_of(int j)
+{
+  Rule r{ 0.0, 0.0, 0.0 };
+  if (j < 61) {
+    const int i = j < 30 ? j : (j < 60 ? j - 30 : 30);
+    r.x = j < 30 ? -c_rule.x[i] : (j < 60 ? c_rule.x[i] : 0.0);
+    r.wk = c_rule.wk[i];
+    r.wg = (i & 1) ? c_rule.wg[i >> 1] : 0.0;  // i = 30 has no Gauss weight
+  }
+  return r;
+}
+
+struct Panel
+{
+  double result, abserr, resabs, resasc;
+};
+
+// Sum of NV values over the 64 threads of a panel (two warps); every thread
+// of the block calls it.  `sh` holds 2 x NV doubles per panel.
+template <int NV>
+__device__ __forceinline__ void panel_sum(double (&v)[NV], double* sh)
+{
+#pragma unroll
+  for (int q = 0; q < NV; q++)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int q = 0; q < NV; q++)
+      sh[((threadIdx.x >> 5) & 1) * NV + q] = v[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; q++)
+    v[q] = sh[q] + sh[NV + q];
+}
+
+__device__ double rescale_err(double err, double res_abs, double res_asc)
+{
+  err = fabs(err);
+  if (res_asc != 0 && err != 0) {
+    const double t = 200 * err / res_asc;
+    const double scale = t * sqrt(t);
+    err = scale < 1 ? res_asc * scale : res_asc;
+  }
+  if (res_abs > DBL_MIN / (50 * DBL_EPSILON)) {
+    const double min_err = 50 * DBL_EPSILON * res_abs;
+    if (min_err > err)
+      err = min_err;
+  }
+  return err;
+}
+
+// The panel's sums from the 61 threads' integrand values f (0 in the others).
+__device__ Panel panel_of(double f, const Rule& w, double a, double b, double* sh)
+{
+  const double half = 0.5 * (b - a), ahalf = fabs(half);
+  double v[3] = { w.wk * f, w.wg * f, w.wk * fabs(f) };
+  panel_sum<3>(v, sh);
+  double u[1] = { w.wk * fabs(f - v[0] * 0.5) };
+  panel_sum<1>(u, sh);
+  Panel p;
+  p.result = v[0] * half;
+  p.resabs = v[2] * ahalf;
+  p.resasc = u[0] * ahalf;
+  p.abserr = rescale_err((v[0] - v[1]) * half, p.resabs, p.resasc);
+  return p;
+}
+
+// Interval list in QUADPACK's partially sorted order (qpsrt) and the running
+// state of one adaptive integral, kept by thread 0.
+struct Qag
+{
+  double a[FREQ_INTERVALS], b[FREQ_INTERVALS], r[FREQ_INTERVALS], e[FREQ_INTERVALS];
+  int order[FREQ_INTERVALS];
+  int size, nrmax, i, rt1, rt2, etype, more;
+  double area, errsum, tol, epsrel, result;
+  double red[16];    // panel_sum scratch
+  Panel second;      // the upper half's panel
+
+  __device__ void sort_errors()
+  {
+    const int last = size - 1;
+    int i_nrmax = nrmax;
+    const int i_maxerr = order[i_nrmax];
+    if (last < 2) {
+      order[0] = 0;
+      order[1] = 1;
+      i = i_maxerr;
+      return;
+    }
+    const double errmax = e[i_maxerr];
+    while (i_nrmax > 0 && errmax > e[order[i_nrmax - 1]]) {
+      order[i_nrmax] = order[i_nrmax - 1];
+      i_nrmax--;
+    }
+    const int top = last;
+    int ii = i_nrmax + 1;
+    while (ii < top && errmax < e[order[ii]]) {
+      order[ii - 1] = order[ii];
+      ii++;
+    }
+    order[ii - 1] = i_maxerr;
+    const double errmin = e[last];
+    int kk = top - 1;
+    while (kk > ii - 2 && errmin >= e[order[kk]]) {
+      order[kk + 1] = order[kk];
+      kk--;
+    }
+    order[kk + 1] = last;
+    i = order[i_nrmax];
+    nrmax = i_nrmax;
+  }
+
+  // after the first panel; more: bisect on
+  __device__ void begin(const Panel& p, double lo, double hi, double eps)
+  {
+    epsrel = eps;
+    result = p.result;
+    tol = epsrel * fabs(p.result);
+    more = 1;
+    const double round_off = 50 * DBL_EPSILON * p.resabs;
+    if ((p.abserr <= round_off && p.abserr > tol) || (p.abserr <= tol && p.abserr != p.resasc) || p.abserr == 0.0)
+      more = 0;
+    a[0] = lo;
+    b[0] = hi;
+    r[0] = p.result;
+    e[0] = p.abserr;
+    order[0] = 0;
+    size = 1;
+    nrmax = i = rt1 = rt2 = etype = 0;
+    area = p.result;
+    errsum = p.abserr;
+  }
+
+  // the two halves of interval i
+  __device__ void step(const Panel& p1, const Panel& p2, int* fail)
+  {
+    const double ai = a[i], bi = b[i], ri = r[i], ei = e[i];
+    const double b1 = 0.5 * (ai + bi);
+    const double area12 = p1.result + p2.result, err12 = p1.abserr + p2.abserr;
+    errsum += err12 - ei;
+    area += area12 - ri;
+    if (p1.resasc != p1.abserr && p2.resasc != p2.abserr) {
+      const double delta = ri - area12;
+      if (fabs(delta) <= 1.0e-5 * fabs(area12) && err12 >= 0.99 * ei)
+        rt1++;
+      if (size >= 10 && err12 > ei)
+        rt2++;
+    }
+    tol = epsrel * fabs(area);
+    if (errsum > tol) {
+      if (rt1 >= 6 || rt2 >= 20)
+        etype = 2;
+      const double tmp = (1 + 100 * DBL_EPSILON) * (fabs(b1) + 1000 * DBL_MIN);
+      if (fabs(ai) <= tmp && fabs(bi) <= tmp)
+        etype = 3;
+    }
+    const int imax = i, n = size;
+    const bool swap = p2.abserr > p1.abserr;
+    a[imax] = swap ? b1 : ai;
+    b[imax] = swap ? bi : b1;
+    r[imax] = swap ? p2.result : p1.result;
+    e[imax] = swap ? p2.abserr : p1.abserr;
+    a[n] = swap ? ai : b1;
+    b[n] = swap ? b1 : bi;
+    r[n] = swap ? p1.result : p2.result;
+    e[n] = swap ? p1.abserr : p2.abserr;
+    size++;
+    sort_errors();
+    more = !etype && errsum > tol;
+    if (more && size == FREQ_INTERVALS) {
+      *fail = 1;
+      more = 0;
+    }
+    if (!more) {
+      double s = 0;
+      for (int q = 0; q < size; q++)
+        s += r[q];
+      result = s;
+    }
+  }
+};
+
+// ---------------------------------------------------------- cross sections
+// XRayHeatingFunctions.c:823-900; eps = sqrt(nu / nu0 - 1)
+__device__ double xs_hydrogenic(double nu, double nu0, double sigma)
+{
+  if (nu < nu0)
+    return 0;
+  if (nu == nu0)
+    nu += k::TINY;
+  const double q = nu0 / nu, q2 = q * q;
+  const double eps = sqrt(nu / nu0 - 1), ieps = 1.0 / eps;
+  return sigma * (q2 * q2) * exp(4 - (4 * atan(eps) * ieps)) / (1 - exp(-2 * k::PI * ieps));
+}
+__device__ __forceinline__ double xs_HI(double nu) { return xs_hydrogenic(nu, k::NU_HI, k::SIGMA_HI); }
+__device__ __forceinline__ double xs_HeII(double nu) { return xs_hydrogenic(nu, k::NU_HEII, 6.3e-18 / 4); }
+__device__ double xs_HeI(double nu)
+{
+  if (nu < k::NU_HEI)
+    return 0;
+  const double x = nu * (1.0 / k::NU_OVER_EV / 13.61) - 0.4434;
+  const double y = sqrt(x * x + 2.136 * 2.136);
+  // y^(0.5 * 3.188 - 5.5) (1 + sqrt(y / 1.469))^-3.188
+  return 9.492e-16 * ((x - 1) * (x - 1) + 2.039 * 2.039) *
+         exp((0.5 * 3.188 - 5.5) * log(y) - 3.188 * log(1.0 + sqrt(y * (1.0 / 1.469))));
+}
+
+// ---------------------------------------------------------- optical depth
+// dtdz (XRayHeatingFunctions.c:377-392) times C n HI at redshift zhat
+__device__ double tau_factor(const FreqArgs& a, double zhat, double fcoll1, double x_e_ave)
+{
+  const double opz = (double)(1 + (float)zhat);
+  const double s = sqrt(a.ol / a.om), ir = 1.0 / (opz * sqrt(opz));
+  const double x = s * ir, dxdz = s * (ir / opz) * (-3.0 / 2.0);
+  const double root = sqrt(x * x + 1);
+  const double const1 = 2 * sqrt(1 + a.om / a.ol) / (3.0 * k::HUBBLE * a.hubble_h);
+  const double dtdz = const1 * (dxdz * (1 + x / root)) / (x + root);
+  const double o = 1 + zhat;
+  const double n = a.n_b0 * (o * o * o);
+  double fc = fcoll1;
+  if (!a.first_snapshot)
+    fc = a.fcoll0 + (zhat - a.z0) * (fcoll1 - a.fcoll0) / (a.z1 - a.z0);
+  if (fc < 0.0)
+    fc = 0.0;
+  double HI = fc < 1e-20 ? 1 : 1 - (a.eff * fc) / (1.0 - x_e_ave);
+  if (HI < 1e-4)
+    HI = 1e-4;
+  return k::C * dtdz * n * HI;
+}
+
+__global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant__ FreqArgs a)
+{
+  __shared__ Qag q;
+  const int r = blockIdx.x, j = threadIdx.x;
+  const double x_e = a.sums[1] / a.total, fcoll1 = a.sums[0] / a.total;
+  if (x_e > 0.9999) {
+    if (j == 0)
+      a.out->nu1[r] = -1.0;
+    return;
+  }
+  const Rule w = rule_of(j);
+  const double zpp = a.zpp[r], zp = a.zp;
+  const double z0 = 0.5 * (zpp + zp) + 0.5 * (zp - zpp) * w.x;
+  const double factor0 = j < 61 ? tau_factor(a, z0, fcoll1, x_e) : 0.0;
+  const double sH = a.f_h * (1 - x_e), sHe = a.f_he * (1 - x_e), sHe2 = a.f_he * x_e;
+  // tau_X(nu): the integral from zpp to zp
+  auto tau = [&](double nu) {
+    const double nu0 = nu / (1 + zp);
+    auto value = [&](double zhat, double factor) {
+      if (j >= 61)
+        return 0.0;
+      const double nuhat = nu0 * (1 + zhat);
+      return factor * (sH * xs_HI(nuhat) + sHe * xs_HeI(nuhat) + sHe2 * xs_HeII(nuhat));
+    };
+    const Panel p = panel_of(value(z0, factor0), w, zpp, zp, q.red);
+    __syncthreads();
+    if (j == 0)
+      q.begin(p, zpp, zp, 0.005);
+    __syncthreads();
+    while (q.more) {
+      const double lo = q.a[q.i], hi = q.b[q.i], mid = 0.5 * (lo + hi);
+      Panel half[2];
+#pragma unroll 1
+      for (int h = 0; h < 2; h++) {
+        const double pa = h ? mid : lo, pb = h ? hi : mid;
+        const double z = 0.5 * (pa + pb) + 0.5 * (pb - pa) * w.x;
+        half[h] = panel_of(value(z, tau_factor(a, z, fcoll1, x_e)), w, pa, pb, q.red);
+      }
+      __syncthreads();
+      if (j == 0)
+        q.step(half[0], half[1], &a.out->fail);
+      __syncthreads();
+    }
+    return q.result;
+  };
+  // nu_tau_one: every thread steps the same bracket (the same sums in each)
+  double root = k::NU_HEI;
+  const double f_lo = tau(k::NU_HEI);
+  if (!(f_lo < 1)) {
+    double xa = k::NU_HEI, xb = 1e6 * k::NU_OVER_EV, fa = f_lo - 1, fb = tau(xb) - 1;
+    double xc = xb, fc = fb, d = xb - xa, e = d, xl = xa, xu = xb;
+    root = 0.5 * (xa + xb);
+    for (int iter = 1; iter <= 100; iter++) {
+      bool two_points = false;
+      if ((fb < 0 && fc < 0) || (fb > 0 && fc > 0)) {
+        two_points = true;
+        xc = xa;
+        fc = fa;
+        d = e = xb - xa;
+      }
+      if (fabs(fc) < fabs(fb)) {
+        two_points = true;
+        xa = xb;
+        xb = xc;
+        xc = xa;
+        fa = fb;
+        fb = fc;
+        fc = fa;
+      }
+      const double tol = 0.5 * DBL_EPSILON * fabs(xb), m = 0.5 * (xc - xb);
+      if (fb == 0) {
+        root = xl = xu = xb;
+        break;
+      }
+      if (fabs(m) <= tol) {
+        root = xb;
+        break;
+      }
+      if (fabs(e) < tol || fabs(fa) <= fabs(fb)) {
+        d = e = m;
+      } else {
+        const double s = fb / fa;
+        double pp, qq;
+        if (two_points) {
+          pp = 2 * m * s;
+          qq = 1 - s;
+        } else {
+          const double t = fa / fc, rr = fb / fc;
+          pp = s * (2 * m * t * (t - rr) - (xb - xa) * (rr - 1));
+          qq = (t - 1) * (rr - 1) * (s - 1);
+        }
+        if (pp > 0)
+          qq = -qq;
+        else
+          pp = -pp;
+        if (2 * pp < fmin(3 * m * qq - fabs(tol * qq), fabs(e * qq))) {
+          e = d;
+          d = pp / qq;
+        } else {
+          d = e = m;
+        }
+      }
+      xa = xb;
+      fa = fb;
+      xb += fabs(d) > tol ? d : (m > 0 ? tol : -tol);
+      fb = tau(xb) - 1;
+      root = xb;
+      double other = xc;
+      if ((fb < 0 && fc < 0) || (fb > 0 && fc > 0))
+        other = xa;
+      xl = fmin(xb, other);
+      xu = fmax(xb, other);
+      const double min_abs = (xl > 0 && xu > 0) || (xl < 0 && xu < 0) ? fmin(fabs(xl), fabs(xu)) : 0.0;
+      if (fabs(xu - xl) < 0.02 * min_abs)
+        break;
+    }
+  }
+  if (j == 0)
+    a.out->nu1[r] = root;
+}
+
+// ----------------------------------------------------- frequency integrals
+// interp_tab (XRayHeatingFunctions.c:914-1190): the energy's bin and the float
+// interpolation in it, then (at the last x_HII node only, which is looked up
+// just below itself) between two x_HII rows.
+struct EnergyBin
+{
+  int n;  // -1: below the table
+  float dE, width;
+};
+__device__ EnergyBin energy_bin(const FreqDevTables& t, double E)
+{
+  EnergyBin b;
+  float En = (float)E;
+  if (En > 0.999 * t.energy[k::NENERGY - 1]) {
+    En = (float)(t.energy[k::NENERGY - 1] * 0.999);
+  } else if (En < t.energy[0]) {
+    b.n = -1;
+    return b;
+  }
+  int n = En < 1008.88f ? (int)(logf(En * 0.1f) * (float)(1 / 1.98026273e-2))
+                        : 232 + (int)(logf(En * (float)(1 / 1008.88)) * (float)(1 / 9.53101798e-2));
+  n = min(max(n, 0), k::NENERGY - 2);
+  while (n > 0 && En < t.edge[n])
+    n--;
+  while (n < k::NENERGY - 2 && En >= t.edge[n + 1])
+    n++;
+  b.n = n;
+  b.width = t.energy[n + 1] - t.energy[n];
+  b.dE = En - t.energy[n];
+  return b;
+}
+__device__ __forceinline__ float in_energy(const float* row, const EnergyBin& b)
+{
+  float v = (row[b.n + 1] - row[b.n]) / b.width;
+  v *= b.dE;
+  return v + row[b.n];
+}
+__device__ float interp(const FreqDevTables& t, const float (*tab)[k::NENERGY], float below, const EnergyBin& b, int xi)
+{
+  if (b.n < 0)
+    return below;
+  if (xi < k::NXHII - 1)
+    return in_energy(tab[xi], b);
+  const int m0 = k::NXHII - 2;
+  const float x = (float)(t.xhii[k::NXHII - 1] * 0.999);
+  const float lo = in_energy(tab[m0], b), hi = in_energy(tab[m0 + 1], b);
+  float v = (hi - lo) / (t.xhii[m0 + 1] - t.xhii[m0]);
+  v *= x - t.xhii[m0];
+  return v + lo;
+}
+
+__device__ double integrand(const FreqArgs& a, double nu, int flag, int xi, double E0nu)
+{
+  const FreqDevTables& t = *a.tables;
+  const double xe = t.xhii[xi];
+  const double nus[3] = { k::NU_HI, k::NU_HEI, k::NU_HEII };
+  const double xs[3] = { a.f_h * (1 - xe) * xs_HI(nu), a.f_he * (1 - xe) * xs_HeI(nu), a.f_he * xe * xs_HeII(nu) };
+  double s = 0;
+#pragma unroll 1
+  for (int q = 0; q < 3; q++) {
+    const EnergyBin b = energy_bin(t, (nu - nus[q]) * (1.0 / k::NU_OVER_EV));
+    double c;
+    if (flag == 0)
+      c = (double)interp(t, t.fheat, 1.0f, b, xi) * k::PLANCK * (nu - nus[q]);
+    else if (flag == 1)
+      c = (double)(interp(t, t.nion[0], 0.0f, b, xi) + interp(t, t.nion[1], 0.0f, b, xi) +
+                   interp(t, t.nion[2], 0.0f, b, xi) + 1);
+    else
+      c = (double)interp(t, t.nlya, 0.0f, b, xi);
+    s += c * xs[q];
+  }
+  return s * exp((-a.alpha - 1) * log(nu / E0nu));
+}
+
+__global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_constant__ FreqArgs a)
+{
+  __shared__ Qag q;
+  // the Ly-alpha tables of the most ionised nodes bisect longest: first
+  int blk = blockIdx.x;
+  const int r = blk % a.S;
+  blk /= a.S;
+  const int set = blk % a.n_sets;
+  blk /= a.n_sets;
+  const int xi = k::NXHII - 1 - blk % k::NXHII, flag = 2 - blk / k::NXHII;
+  const double E0nu = a.E0[set] * k::NU_OVER_EV;
+  // shells whose lower limit is E0 share their integrals: the first computes
+  const bool at_E0 = !(a.out->nu1[r] > E0nu);
+  if (at_E0)
+    for (int o = 0; o < r; o++)
+      if (!(a.out->nu1[o] > E0nu))
+        return;
+  const double lower = at_E0 ? E0nu : a.out->nu1[r];
+  const int j = threadIdx.x & 63, h = threadIdx.x >> 6;
+  const Rule w = rule_of(j);
+  auto panel = [&](double pa, double pb) {
+    const double f = j < 61 ? integrand(a, 0.5 * (pa + pb) + 0.5 * (pb - pa) * w.x, flag, xi, E0nu) : 0.0;
+    return panel_of(f, w, pa, pb, q.red + 8 * h);
+  };
+  {
+    const Panel p = panel(lower, a.numax);
+    __syncthreads();
+    if (threadIdx.x == 0)
+      q.begin(p, lower, a.numax, 0.01);
+  }
+  __syncthreads();
+  while (q.more) {
+    const double lo = q.a[q.i], hi = q.b[q.i], mid = 0.5 * (lo + hi);
+    const Panel p = panel(h ? mid : lo, h ? hi : mid);
+    if (threadIdx.x == 64)
+      q.second = p;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      q.step(p, q.second, &a.out->fail);
+    __syncthreads();
+  }
+  if (threadIdx.x < a.S) {
+    const int o = threadIdx.x;
+    double res = q.result;
+    if (flag == 2)
+      res = res * k::C / (4 * k::PI) / k::LYA_HZ / a.hubble;
+    if (o == r || (at_E0 && !(a.out->nu1[o] > E0nu)))
+      a.out->tab[set][(flag * k::NXHII + xi) * a.S + o] = res;
+  }
+}
+}  // namespace
+
+void fill_freq_dev_tables(const HeatTables& ht, FreqDevTables* t)
+{
+  std::memcpy(t->energy, ht.energy, sizeof(t->energy));
+  std::memcpy(t->xhii, ht.xhii, sizeof(t->xhii));
+  std::memcpy(t->fheat, ht.fheat, sizeof(t->fheat));
+  std::memcpy(t->nlya, ht.nlya, sizeof(t->nlya));
+  std::memcpy(t->nion[0], ht.nion_hi, sizeof(t->nion[0]));
+  std::memcpy(t->nion[1], ht.nion_hei, sizeof(t->nion[1]));
+  std::memcpy(t->nion[2], ht.nion_heii, sizeof(t->nion[2]));
+  // loc_energy does not decrease with the energy: bisect the float at which
+  // it reaches n
+  const float top = ht.energy[k::NENERGY - 1];
+  t->edge[0] = 0.0f;
+  for (int n = 1; n <= k::NENERGY; n++) {
+    if (loc_energy(top) < n) {
+      t->edge[n] = INFINITY;
+      continue;
+    }
+    float lo = ht.energy[0], hi = top;
+    if (loc_energy(lo) >= n)
+      hi = lo;
+    while (std::nextafter(lo, hi) < hi) {
+      const float mid = lo + 0.5f * (hi - lo);
+      (loc_energy(mid) >= n ? hi : lo) = mid;
+    }
+    t->edge[n] = hi;
+  }
+}
+
+FreqArgs make_freq_args(const mx_params& p, const Derived& d, const std::vector<double>& zz, const double* stored_fcoll,
+                        int snapshot, const ShellPlan& sp)
+{
+  FreqArgs a{};
+  a.S = sp.S;
+  a.n_sets = 1;
+  a.zp = zz[snapshot];
+  for (int r = 0; r < sp.S; r++)
+    a.zpp[r] = shell_redshift(sp, a.zp, r);
+  a.E0[0] = p.nu_xray_gal_threshold;
+  a.alpha = p.spec_index_xray_gal;
+  a.numax = p.nu_xray_max * k::NU_OVER_EV;
+  a.hubble = hubble(p, (float)a.zp);
+  a.om = p.omega_m;
+  a.ol = p.omega_lambda;
+  a.hubble_h = p.hubble_h;
+  a.n_b0 = d.n_b0;
+  a.f_h = d.f_h;
+  a.f_he = d.f_he;
+  a.eff = p.reion_efficiency;
+  a.first_snapshot = snapshot == 0;
+  if (snapshot > 0) {
+    a.fcoll0 = stored_fcoll[snapshot - 1];
+    a.z0 = zz[snapshot - 1];
+  }
+  a.z1 = a.zp;
+  return a;
+}
+
+void launch_freq_tables(const FreqArgs& a, cudaStream_t s)
+{
+  cudaMemsetAsync(&a.out->fail, 0, sizeof(int), s);
+  k_tau_lower<<<a.S, TAU_THREADS, 0, s>>>(a);
+  k_freq_integrals<<<a.S * a.n_sets * FREQ_TAB, INT_THREADS, 0, s>>>(a);
+  freq_launches += 2;
+}
+
+int freq_kernel_launches() { return freq_launches; }
+
+}  // namespace mx

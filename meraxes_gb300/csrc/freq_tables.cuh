@@ -1,0 +1,56 @@
+// Frequency-integral tables of ComputeTs on the device (see freq_tables.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "host_physics.h"
+#include "kernels.cuh"
+
+namespace mx {
+
+constexpr int FREQ_SETS = 3;  // X-ray thresholds E0 of one call (the adjoint needs three)
+constexpr int FREQ_TAB = 3 * k::NXHII;  // rows of a set: tab[(flag * 14 + x) * S + r]
+
+// The secondary-electron tables and the bin edges of their energy index.
+struct FreqDevTables
+{
+  float energy[k::NENERGY];
+  float edge[k::NENERGY + 1];  // smallest energy whose index (loc_energy) is n
+  float xhii[k::NXHII];
+  float fheat[k::NXHII][k::NENERGY], nlya[k::NXHII][k::NENERGY];
+  float nion[3][k::NXHII][k::NENERGY];
+};
+void fill_freq_dev_tables(const HeatTables& ht, FreqDevTables* t);
+
+// What the kernels write: the frequency of unit optical depth of each shell,
+// the tables (S entries per row), and whether an integral needed more
+// intervals than the kernels hold (then the host builds the tables).
+struct FreqDevResult
+{
+  double nu1[MAX_SHELLS];
+  double tab[FREQ_SETS][FREQ_TAB * MAX_SHELLS];
+  int fail;
+};
+
+struct FreqArgs
+{
+  const FreqDevTables* tables;  // device
+  const double* sums;           // device: sum of f_coll and of x_e over the cells
+  double total;                 // cells
+  int S, n_sets;
+  double zp, zpp[MAX_SHELLS];
+  double E0[FREQ_SETS];  // NuXrayGalThreshold [eV]
+  double alpha, numax, hubble;
+  double om, ol, hubble_h, n_b0, f_h, f_he, eff;
+  // collapse fraction over redshift (interpolate_fcoll): linear from fcoll0 at
+  // z0 to this snapshot's at z1; constant for the first snapshot
+  int first_snapshot;
+  double fcoll0, z0, z1;
+  FreqDevResult* out;  // device
+};
+FreqArgs make_freq_args(const mx_params& p, const Derived& d, const std::vector<double>& zz, const double* stored_fcoll,
+                        int snapshot, const ShellPlan& sp);
+void launch_freq_tables(const FreqArgs& a, cudaStream_t s);
+int freq_kernel_launches();
+
+}  // namespace mx

@@ -1,6 +1,8 @@
 // Host-side FP64 physics tables of the reionization step (see host_physics.h).
 #include "host_physics.h"
 
+#include "gk61.h"
+
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
@@ -72,41 +74,9 @@ double NaturalSpline::eval(double xv) const
 
 // ================================================================ QAG-GK61
 namespace {
-// Kronrod abscissae (xk), Kronrod weights (wk) and Gauss weights (wg) of the
-// 61-point rule, QUADPACK (Piessens et al. 1983), qk61.
-const double XK[31] = {
-  0.999484410050490637571325895705811, 0.996893484074649540271630050918695, 0.991630996870404594858628366109486,
-  0.983668123279747209970032581605663, 0.973116322501126268374693868423707, 0.960021864968307512216871025581798,
-  0.944374444748559979415831324037439, 0.926200047429274325879324277080474, 0.905573307699907798546522558925958,
-  0.882560535792052681543116462530226, 0.857205233546061098958658510658944, 0.829565762382768397442898119732502,
-  0.799727835821839083013668942322683, 0.767777432104826194917977340974503, 0.733790062453226804726171131369528,
-  0.697850494793315796932292388026640, 0.660061064126626961370053668149271, 0.620526182989242861140477556431189,
-  0.579345235826361691756024932172540, 0.536624148142019899264169793311073, 0.492480467861778574993693061207709,
-  0.447033769538089176780609900322854, 0.400401254830394392535476211542661, 0.352704725530878113471037207089374,
-  0.304073202273625077372677107199257, 0.254636926167889846439805129817805, 0.204525116682309891438957671002025,
-  0.153869913608583546963794672743256, 0.102806937966737030147096751318001, 0.051471842555317695833025213166723,
-  0.000000000000000000000000000000000
-};
-const double WG[15] = {
-  0.007968192496166605615465883474674, 0.018466468311090959142302131912047, 0.028784707883323369349719179611292,
-  0.038799192569627049596801936446348, 0.048402672830594052902938140422808, 0.057493156217619066481721689402056,
-  0.065974229882180495128128515115962, 0.073755974737705206268243850022191, 0.080755895229420215354694938460530,
-  0.086899787201082979802387530715126, 0.092122522237786128717632707087619, 0.096368737174644259639468626351810,
-  0.099593420586795267062780282103569, 0.101762389748405504596428952168554, 0.102852652893558840341285636705415
-};
-const double WK[31] = {
-  0.001389013698677007624551591226760, 0.003890461127099884051267201844516, 0.006630703915931292173319826369750,
-  0.009273279659517763428441146892024, 0.011823015253496341742232898853251, 0.014369729507045804812451432443580,
-  0.016920889189053272627572289420322, 0.019414141193942381173408951050128, 0.021828035821609192297167485738339,
-  0.024191162078080601365686370725232, 0.026509954882333101610601709335075, 0.028754048765041292843978785354334,
-  0.030907257562387762472884252943092, 0.032981447057483726031814191016854, 0.034979338028060024137499670731468,
-  0.036882364651821229223911065617136, 0.038678945624727592950348651532281, 0.040374538951535959111995279752468,
-  0.041969810215164246147147541285970, 0.043452539701356069316831728117073, 0.044814800133162663192355551616723,
-  0.046059238271006988116271735559374, 0.047185546569299153945261478181099, 0.048185861757087129140779492298305,
-  0.049055434555029778887528165367238, 0.049795683427074206357811569379942, 0.050405921402782346840893085653585,
-  0.050881795898749606492297473049805, 0.051221547849258772170656282604944, 0.051426128537459025933862879215781,
-  0.051494729429451567558340433647099
-};
+const double (&XK)[31] = GK61.x;
+const double (&WG)[15] = GK61.wg;
+const double (&WK)[31] = GK61.wk;
 
 double rescale_err(double err, double res_abs, double res_asc)
 {
@@ -935,12 +905,16 @@ double xs_HeI(double nu)
          std::pow(1.0 + std::sqrt(y / 1.469), -3.188);
 }
 
+}  // namespace
+
 int loc_energy(float En)
 {
   if (En < 1008.88)
     return (int)(std::log(En / 10.0) / 1.98026273e-2);
   return 232 + (int)(std::log(En / 1008.88) / 9.53101798e-2);
 }
+
+namespace {
 int loc_xhii(const HeatTables& ht, float x)
 {
   int m = k::NXHII - 1;
@@ -1018,22 +992,26 @@ void parallel_for(int n, int nthreads, const std::function<void(int)>& fn)
 }
 }  // namespace
 
-void build_freq_tables(const mx_params& p,
-                       const Derived& d,
-                       const HeatTables& ht,
-                       const std::vector<double>& zz,
-                       const double* stored_fcoll,
-                       int snapshot,
-                       const ShellPlan& sp,
-                       double x_e_ave,
-                       double weight_in,
-                       int nthreads,
-                       FreqTables* out)
+double shell_redshift(const ShellPlan& sp, double zp, int r)
+{
+  const double prev_zpp = r == 0 ? zp : sp.zpp_edge[r - 1];
+  return (sp.zpp_edge[r] + prev_zpp) * 0.5;
+}
+
+void build_freq_integrals(const mx_params& p,
+                          const Derived& d,
+                          const HeatTables& ht,
+                          const std::vector<double>& zz,
+                          const double* stored_fcoll,
+                          int snapshot,
+                          const ShellPlan& sp,
+                          double x_e_ave,
+                          int nthreads,
+                          FreqTables* out)
 {
   const int S = sp.S;
   const double zp = zz[snapshot];
   out->tab.assign((size_t)3 * k::NXHII * S, 0.0);
-  out->sum_lyn.assign(S, 0.0);
   const double eff = p.reion_efficiency;
 
   // interpolate_fcoll (XRayHeatingFunctions.c:1884-1900)
@@ -1076,10 +1054,8 @@ void build_freq_tables(const mx_params& p,
   };
 
   std::vector<double> zpp_mid(S), lower(S);
-  for (int r = 0; r < S; r++) {
-    const double prev_zpp = r == 0 ? zp : sp.zpp_edge[r - 1];
-    zpp_mid[r] = (sp.zpp_edge[r] + prev_zpp) * 0.5;
-  }
+  for (int r = 0; r < S; r++)
+    zpp_mid[r] = shell_redshift(sp, zp, r);
   const double E0 = p.nu_xray_gal_threshold, alpha = p.spec_index_xray_gal;
   parallel_for(S, nthreads, [&](int r) {
     lower[r] = std::fmax(nu_tau_one(zpp_mid[r], x_e_ave), E0 * k::NU_OVER_EV);
@@ -1140,6 +1116,23 @@ void build_freq_tables(const mx_params& p,
       res = res * k::C / (4 * k::PI) / k::LYA_HZ / hub;
     out->tab[((size_t)flag * k::NXHII + xi) * S + r] = res;
   });
+}
+
+void build_freq_scalars(const mx_params& p,
+                        const HeatTables& ht,
+                        const std::vector<double>& zz,
+                        int snapshot,
+                        const ShellPlan& sp,
+                        double weight_in,
+                        FreqTables* out)
+{
+  const int S = sp.S;
+  const double zp = zz[snapshot];
+  const double E0 = p.nu_xray_gal_threshold, alpha = p.spec_index_xray_gal;
+  out->sum_lyn.assign(S, 0.0);
+  float zmax[k::NSPEC_MAX + 1];
+  for (int n = 2; n <= k::NSPEC_MAX; n++)
+    zmax[n] = zmax_f((float)zp, n);
 
   // Ly-n sums and the kink correction (ComputeTs.c:585-663)
   bool first_radii = true, first_zero = true;
@@ -1148,10 +1141,10 @@ void build_freq_tables(const mx_params& p,
   for (int r = 0; r < S; r++) {
     const double prev_zpp = r == 0 ? zp : sp.zpp_edge[r - 1];
     const double prev_R = r == 0 ? 0 : sp.R[r - 1];
-    const double zpp = zpp_mid[r];
+    const double zpp = shell_redshift(sp, zp, r);
     double s = 0;
     for (int n_ct = k::NSPEC_MAX; n_ct >= 2; n_ct--) {
-      if (zpp > zmax_f((float)zp, n_ct))
+      if (zpp > zmax[n_ct])
         continue;
       const double nuprime = nu_n(n_ct) * (1 + zpp) / (1.0 + zp);
       s += frecycle(n_ct) * spectral_emissivity(ht, nuprime);
@@ -1167,7 +1160,7 @@ void build_freq_tables(const mx_params& p,
         const double tz = tmin + (tmax - tmin) * (float)ii / ((float)n_pts_radii - 1.);
         int counter = 0;
         for (int n_ct = k::NSPEC_MAX; n_ct >= 2; n_ct--) {
-          if (tz > zmax_f((float)zp, n_ct))
+          if (tz > zmax[n_ct])
             continue;
           counter++;
         }

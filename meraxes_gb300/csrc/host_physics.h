@@ -175,16 +175,28 @@ struct FreqTables
   double const_zp_prefactor = 0;
   double growth_zp = 0, dgrowth_dzp = 0, dt_dzp = 0;
 };
-void build_freq_tables(const mx_params& p,
-                       const Derived& d,
-                       const HeatTables& ht,
-                       const std::vector<double>& zz,
-                       const double* stored_fcoll,
-                       int snapshot,
-                       const ShellPlan& sp,
-                       double x_e_ave,
-                       double weight_in,
-                       int nthreads,
-                       FreqTables* out);
+// The mid redshift of shell r.
+double shell_redshift(const ShellPlan& sp, double zp, int r);
+// tab, on host threads (the device computes it in freq_tables.cu).
+void build_freq_integrals(const mx_params& p,
+                          const Derived& d,
+                          const HeatTables& ht,
+                          const std::vector<double>& zz,
+                          const double* stored_fcoll,
+                          int snapshot,
+                          const ShellPlan& sp,
+                          double x_e_ave,
+                          int nthreads,
+                          FreqTables* out);
+// Everything else of FreqTables.
+void build_freq_scalars(const mx_params& p,
+                        const HeatTables& ht,
+                        const std::vector<double>& zz,
+                        int snapshot,
+                        const ShellPlan& sp,
+                        double weight_in,
+                        FreqTables* out);
+// Energy-table bin of a photoelectron energy (XRayHeatingFunctions.c:914-940).
+int loc_energy(float En);
 
 }  // namespace mx

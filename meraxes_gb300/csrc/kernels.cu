@@ -10,6 +10,7 @@
 #include "kernels.cuh"
 #include "deposit.cuh"
 #include "fft3d.cuh"
+#include "freq_tables.cuh"
 #include "lightcone.cuh"
 #include "pecvel.cuh"
 #include "ps.cuh"
@@ -102,7 +103,7 @@ void launch_adjoint_axpy(float* grad, const float* v, const float* u0, float a_f
 int kernel_launch_count()
 {
   return g_launches + ts_kernel_launches() + fft_kernel_launches() + ps_kernel_launches() + pecvel_kernel_launches() +
-         lightcone_kernel_launches() + deposit_kernel_launches();
+         lightcone_kernel_launches() + deposit_kernel_launches() + freq_kernel_launches();
 }
 void reset_kernel_launch_count() { g_launches = 0; }
 

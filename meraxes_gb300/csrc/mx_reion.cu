@@ -12,7 +12,6 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
-#include <future>
 #include <map>
 #include <mutex>
 #include <memory>
@@ -24,6 +23,7 @@
 #include "bulk.cuh"
 #include "deposit.cuh"
 #include "fft3d.cuh"
+#include "freq_tables.cuh"
 #include "lightcone.cuh"
 #include "pecvel.cuh"
 #include "ps.cuh"
@@ -75,8 +75,9 @@ struct mx_ctx
   double stored_fcoll[1000];
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // host-pointer mx_step: copies that overlap the compute
-  // host-pointer mx_step: ComputeTs's collapse fraction and <x_e> beside the
-  // shells (they wait for other uploads); ev_cf marks their sums on the host
+  // ComputeTs beside its shells: the frequency-integral tables, and in a
+  // host-pointer mx_step the collapse fraction and <x_e> that they need (which
+  // wait for other uploads); ev_cf marks the results on the host
   cudaStream_t aux_stream = nullptr;
   cudaEvent_t ev_cf = nullptr;
   bool early_shells = true;  // MX_TS_EARLY_SHELLS=0: the collapse fraction first
@@ -133,6 +134,10 @@ struct mx_ctx
   float* d_shells = nullptr;    // S x N (spin temperature)
   unsigned int* d_err = nullptr;
   float* d_xe_last = nullptr;
+  // frequency-integral tables of ComputeTs (freq_tables.cu)
+  FreqDevTables* d_ft_tables = nullptr;
+  FreqDevResult* d_ft = nullptr;
+  FreqDevResult* h_ft = nullptr;  // pinned copy
   // device mirror used by the host-pointer entry points
   mx_grids mirror{};
   std::vector<void*> mirror_allocs;
@@ -298,6 +303,9 @@ mx_ctx::~mx_ctx()
   cudaFree(d_shells);
   cudaFree(d_err);
   cudaFree(d_xe_last);
+  cudaFree(d_ft_tables);
+  cudaFree(d_ft);
+  cudaFreeHost(h_ft);
   cudaFree(d_rr_x);
   cudaFree(d_rr_y);
   cudaFree(d_rr_c);
@@ -398,6 +406,12 @@ void mx_ctx::alloc_scratch()
     MX_CUDA(cudaMallocHost(&h_tsc, sizeof(TsDevConst)));
     MX_CUDA(cudaMalloc(&d_shells, sizeof(float) * gd.N * (size_t)p.ts_num_filter_steps));
     make_shell_map();
+    MX_CUDA(cudaMalloc(&d_ft_tables, sizeof(FreqDevTables)));
+    MX_CUDA(cudaMalloc(&d_ft, sizeof(FreqDevResult)));
+    MX_CUDA(cudaMallocHost(&h_ft, sizeof(FreqDevResult)));
+    std::unique_ptr<FreqDevTables> ft(new FreqDevTables());
+    fill_freq_dev_tables(ht, ft.get());
+    MX_CUDA(cudaMemcpy(d_ft_tables, ft.get(), sizeof(FreqDevTables), cudaMemcpyHostToDevice));
   }
   // forward transform: padded real input -> half spectrum (out of place)
   int n[3] = { gd.D, gd.D, gd.D };
@@ -1025,9 +1039,38 @@ static void compute_shells(mx_ctx* c, const ShellPlan& sp, float* sfr, float* sf
   }
 }
 
+// Frequency-integral tables for the X-ray thresholds of `sets` on stream fs,
+// once the sums of f_coll and x_e (d_sums[0..1]) are there, copied to the
+// pinned h_ft.
+static void launch_tables(mx_ctx* c, const ShellPlan& sp, int snapshot, const std::vector<double>& E0, cudaStream_t fs)
+{
+  FreqArgs a = make_freq_args(c->p, c->d, c->zz, c->stored_fcoll, snapshot, sp);
+  a.tables = c->d_ft_tables;
+  a.sums = c->d_sums;
+  a.total = (double)c->gd.N;
+  a.n_sets = (int)E0.size();
+  for (int i = 0; i < a.n_sets; i++)
+    a.E0[i] = E0[i];
+  a.out = c->d_ft;
+  Prof pr(c, "freq_tables", 0.0, fs);
+  launch_freq_tables(a, fs);
+  MX_CUDA(cudaMemcpyAsync(c->h_ft, c->d_ft, sizeof(FreqDevResult), cudaMemcpyDeviceToHost, fs));
+}
+
+// The tables of set i from h_ft (or from host threads, where an adaptive
+// integral outgrew the device's interval list).  `p` holds the set's E0.
+static void take_tables(mx_ctx* c, const mx_params& p, const ShellPlan& sp, int snapshot, int i, double x_e_ave,
+                        FreqTables* ft)
+{
+  if (c->h_ft->fail)
+    build_freq_integrals(p, c->d, c->ht, c->zz, c->stored_fcoll, snapshot, sp, x_e_ave, c->nthreads, ft);
+  else
+    ft->tab.assign(c->h_ft->tab[i], c->h_ft->tab[i] + (size_t)FREQ_TAB * sp.S);
+}
+
 // ComputeTs's host work inside a captured step: a host node of the graph
-// reads the collapse fraction and <x_e> (copied to pinned slots by the node
-// before it), builds the frequency-integral tables and fills the evolve
+// reads the collapse fraction and <x_e> and the frequency-integral tables
+// (copied to pinned memory by the nodes before it) and fills the evolve
 // kernels' constants into the pinned h_tsc, which the next node uploads.
 struct TsHostWork
 {
@@ -1047,8 +1090,8 @@ static void CUDART_CB ts_tables_host(void* arg)
     const double collapse_fraction = w->cf[0] / w->total, x_e_ave = w->cf[1] / w->total;
     c->stored_fcoll[w->snapshot] = collapse_fraction;
     FreqTables ft;
-    build_freq_tables(c->p, c->d, c->ht, c->zz, c->stored_fcoll, w->snapshot, w->sp, x_e_ave, w->sp.weight_after,
-                      c->nthreads, &ft);
+    build_freq_scalars(c->p, c->ht, c->zz, w->snapshot, w->sp, w->sp.weight_after, &ft);
+    take_tables(c, c->p, w->sp, w->snapshot, 0, x_e_ave, &ft);
     TsDevConst* t = c->h_tsc;
     std::memset(t, 0, sizeof(TsDevConst));
     fill_common_ts(c, t, w->zp);
@@ -1132,39 +1175,26 @@ static void run_ComputeTs(mx_ctx* c, int snapshot, const mx_grids* g, mx_globals
     ca.R3 = std::pow(R0, 3.0);
     ca.pixel_volume = pixel_volume;
     ca.partials = c->d_partials;
-    if (early_shells) {
-      // the shells first on s; the sums on the side stream after the grids
-      // they read, copied to the host, where the tables wait for them
-      cudaStream_t as = c->aux_stream;
+    // the tables of the X-ray frequency integrals need these sums and nothing
+    // else of the GPU's work: they are built on the side stream while the
+    // shells are smoothed on s.  With early_shells (host grids) the sums wait
+    // there too, for the grids that they read.
+    cudaStream_t as = c->aux_stream, cs = early_shells ? as : s;
+    if (early_shells)
       MX_CUDA(cudaStreamWaitEvent(as, up->first, 0));
-      {
-        Prof pr(c, "k_cf_xe", 3.0 * 4.0 * (double)gd.N, as);
-        launch_cf_xe(ca, gd, as);
-      }
-      launch_finalize(c->d_partials, 2, c->d_sums, as);
-      MX_CUDA(cudaMemcpyAsync(c->h_sums, c->d_sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, as));
-      MX_CUDA(cudaEventRecord(c->ev_cf, as));
-      compute_shells(c, sp, g->sfr, g->sfr_histories, s, up);
-      MX_CUDA(cudaEventSynchronize(c->ev_cf));
-      collapse_fraction = c->h_sums[0] / total;
-      x_e_ave = c->h_sums[1] / total;
-      c->stored_fcoll[snapshot] = collapse_fraction;
-      FreqTables ft;
-      build_freq_tables(p, c->d, c->ht, c->zz, c->stored_fcoll, snapshot, sp, x_e_ave, sp.weight_after, c->nthreads,
-                        &ft);
-      fill_ts_constants(c, t, sp, ft, zp, prev_z, collapse_fraction, pixel_volume);
-      // the evolve kernel rewrites x_e_box_prev, which the side stream read
-      MX_CUDA(cudaStreamWaitEvent(s, c->ev_cf, 0));
-      MX_CUDA(cudaMemcpyAsync(c->d_tsc, t, sizeof(TsDevConst), cudaMemcpyHostToDevice, s));
-    } else {
     {
-      Prof pr(c, "k_cf_xe", 3.0 * 4.0 * (double)gd.N, s);
-      launch_cf_xe(ca, gd, s);
+      Prof pr(c, "k_cf_xe", 3.0 * 4.0 * (double)gd.N, cs);
+      launch_cf_xe(ca, gd, cs);
     }
-    launch_finalize(c->d_partials, 2, c->d_sums, s);
+    launch_finalize(c->d_partials, 2, c->d_sums, cs);
+    if (!early_shells) {
+      MX_CUDA(cudaEventRecord(c->ev_a, s));
+      MX_CUDA(cudaStreamWaitEvent(as, c->ev_a, 0));
+    }
+    const std::vector<double> E0 = { p.nu_xray_gal_threshold };
     if (c->capturing) {
-      // a captured step: the tables are built by a host node on a side
-      // branch of the graph while the shells are smoothed on s
+      // a captured step: the constants are filled by a host node on the side
+      // branch of the graph
       hw = std::make_shared<TsHostWork>();
       hw->c = c;
       hw->snapshot = snapshot;
@@ -1173,45 +1203,30 @@ static void run_ComputeTs(mx_ctx* c, int snapshot, const mx_grids* g, mx_globals
       hw->prev_z = prev_z;
       hw->pixel_volume = pixel_volume;
       hw->total = total;
-      cudaStream_t hs = c->copy_stream;
-      MX_CUDA(cudaEventRecord(c->ev_a, s));
-      MX_CUDA(cudaStreamWaitEvent(hs, c->ev_a, 0));
-      hw->cf = readback(c, (const double*)c->d_sums, 2, hs);
-      MX_CUDA(cudaLaunchHostFunc(hs, ts_tables_host, hw.get()));
-      MX_CUDA(cudaMemcpyAsync(c->d_tsc, c->h_tsc, sizeof(TsDevConst), cudaMemcpyHostToDevice, hs));
-      MX_CUDA(cudaEventRecord(c->ev_b, hs));
+      hw->cf = readback(c, (const double*)c->d_sums, 2, as);
+      launch_tables(c, sp, snapshot, E0, as);
+      MX_CUDA(cudaLaunchHostFunc(as, ts_tables_host, hw.get()));
+      MX_CUDA(cudaMemcpyAsync(c->d_tsc, c->h_tsc, sizeof(TsDevConst), cudaMemcpyHostToDevice, as));
+      MX_CUDA(cudaEventRecord(c->ev_b, as));
       c->graph_keep.push_back(hw);
       compute_shells(c, sp, g->sfr, g->sfr_histories, s, up);
       MX_CUDA(cudaStreamWaitEvent(s, c->ev_b, 0));
     } else {
-      MX_CUDA(cudaMemcpyAsync(c->h_sums, c->d_sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
-      MX_CUDA(cudaStreamSynchronize(s));
+      MX_CUDA(cudaMemcpyAsync(c->h_sums, c->d_sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, as));
+      launch_tables(c, sp, snapshot, E0, as);
+      MX_CUDA(cudaEventRecord(c->ev_cf, as));
+      compute_shells(c, sp, g->sfr, g->sfr_histories, s, up);
+      FreqTables ft;
+      build_freq_scalars(p, c->ht, c->zz, snapshot, sp, sp.weight_after, &ft);
+      MX_CUDA(cudaEventSynchronize(c->ev_cf));
       collapse_fraction = c->h_sums[0] / total;
       x_e_ave = c->h_sums[1] / total;
       c->stored_fcoll[snapshot] = collapse_fraction;
-
-      // X-ray frequency tables on host threads while the shells are smoothed
-      FreqTables ft;
-      std::vector<double> zz = c->zz;
-      std::future<void> tables = std::async(std::launch::async, [&]() {
-        build_freq_tables(p, c->d, c->ht, zz, c->stored_fcoll, snapshot, sp, x_e_ave, sp.weight_after, c->nthreads,
-                          &ft);
-      });
-
-      // shells (ComputeTs.c:276-503): apply the SFR-history operations, forward
-      // transform when the grid changed, then filter + inverse transform in
-      // batches of shells sharing a spectrum.
-      try {
-        compute_shells(c, sp, g->sfr, g->sfr_histories, s, up);
-      } catch (...) {
-        tables.wait();
-        throw;
-      }
-      tables.get();
-
+      take_tables(c, p, sp, snapshot, 0, x_e_ave, &ft);
       fill_ts_constants(c, t, sp, ft, zp, prev_z, collapse_fraction, pixel_volume);
+      // the evolve kernel rewrites x_e_box_prev, which the sums read
+      MX_CUDA(cudaStreamWaitEvent(s, c->ev_cf, 0));
       MX_CUDA(cudaMemcpyAsync(c->d_tsc, t, sizeof(TsDevConst), cudaMemcpyHostToDevice, s));
-    }
     }
     EvolveArgs ea;
     ea.shells = c->d_shells;
@@ -1618,36 +1633,33 @@ static void run_adjoint(mx_ctx* c, int snapshot, const mx_grids* g, const float*
   ca.partials = c->d_partials;
   launch_cf_xe(ca, gd, s);
   launch_finalize(c->d_partials, 2, c->d_sums, s);
-  MX_CUDA(cudaMemcpyAsync(c->h_sums, c->d_sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
-  MX_CUDA(cudaStreamSynchronize(s));
-  const double collapse_fraction = c->h_sums[0] / total;
-  const double x_e_ave = c->h_sums[1] / total;
-  c->stored_fcoll[snapshot] = collapse_fraction;
-  // frequency tables at E0 and E0 (1 +- h) for d/dE0, on host threads while
-  // the shells are recomputed
+  // frequency tables at E0 and E0 (1 +- h) for d/dE0, on the side stream
+  // while the shells are recomputed
   const double h = 1e-3;
   FreqTables ft, ftp, ftm;
   mx_params pp = p, pm = p;
   pp.nu_xray_gal_threshold = p.nu_xray_gal_threshold * (1 + h);
   pm.nu_xray_gal_threshold = p.nu_xray_gal_threshold * (1 - h);
-  const int nt = std::max(1, c->nthreads / 3);
-  auto build = [&](const mx_params& q, FreqTables* out) {
-    return std::async(std::launch::async, [&, out]() {
-      build_freq_tables(q, c->d, c->ht, c->zz, c->stored_fcoll, snapshot, sp, x_e_ave, sp.weight_after, nt, out);
-    });
-  };
-  std::future<void> tables[3] = { build(p, &ft), build(pp, &ftp), build(pm, &ftm) };
-  try {
-    // shells of the forward, from a copy of the SFR grid
-    MX_CUDA(cudaMemcpyAsync(c->d_adj_sfr, g->sfr, sizeof(float) * gd.P, cudaMemcpyDeviceToDevice, s));
-    compute_shells(c, sp, c->d_adj_sfr, g->sfr_histories, s);
-  } catch (...) {
-    for (auto& f : tables)
-      f.wait();
-    throw;
-  }
-  for (auto& f : tables)
-    f.get();
+  cudaStream_t as = c->aux_stream;
+  MX_CUDA(cudaEventRecord(c->ev_a, s));
+  MX_CUDA(cudaStreamWaitEvent(as, c->ev_a, 0));
+  MX_CUDA(cudaMemcpyAsync(c->h_sums, c->d_sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, as));
+  launch_tables(c, sp, snapshot, { p.nu_xray_gal_threshold, pp.nu_xray_gal_threshold, pm.nu_xray_gal_threshold }, as);
+  MX_CUDA(cudaEventRecord(c->ev_cf, as));
+  // shells of the forward, from a copy of the SFR grid
+  MX_CUDA(cudaMemcpyAsync(c->d_adj_sfr, g->sfr, sizeof(float) * gd.P, cudaMemcpyDeviceToDevice, s));
+  compute_shells(c, sp, c->d_adj_sfr, g->sfr_histories, s);
+  build_freq_scalars(p, c->ht, c->zz, snapshot, sp, sp.weight_after, &ft);
+  build_freq_scalars(pp, c->ht, c->zz, snapshot, sp, sp.weight_after, &ftp);
+  build_freq_scalars(pm, c->ht, c->zz, snapshot, sp, sp.weight_after, &ftm);
+  MX_CUDA(cudaEventSynchronize(c->ev_cf));
+  const double collapse_fraction = c->h_sums[0] / total;
+  const double x_e_ave = c->h_sums[1] / total;
+  c->stored_fcoll[snapshot] = collapse_fraction;
+  take_tables(c, p, sp, snapshot, 0, x_e_ave, &ft);
+  take_tables(c, pp, sp, snapshot, 1, x_e_ave, &ftp);
+  take_tables(c, pm, sp, snapshot, 2, x_e_ave, &ftm);
+  MX_CUDA(cudaStreamWaitEvent(s, c->ev_cf, 0));
   fill_ts_constants(c, t, sp, ft, zp, prev_z, collapse_fraction, pixel_volume);
   MX_CUDA(cudaMemcpyAsync(c->d_tsc, t, sizeof(TsDevConst), cudaMemcpyHostToDevice, s));
   {
@@ -2603,7 +2615,10 @@ static int create_ctx(const mx_params* params, const char* tables_dir, size_t wo
     }
     MX_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     MX_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
-    MX_CUDA(cudaStreamCreateWithFlags(&c->aux_stream, cudaStreamNonBlocking));
+    // the side stream's few small blocks go ahead of the shells' thousands
+    int least = 0, greatest = 0;
+    MX_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    MX_CUDA(cudaStreamCreateWithPriority(&c->aux_stream, cudaStreamNonBlocking, greatest));
     MX_CUDA(cudaEventCreateWithFlags(&c->ev_cf, cudaEventDisableTiming));
     MX_CUDA(cudaEventCreateWithFlags(&c->ev_a, cudaEventDisableTiming));
     MX_CUDA(cudaEventCreateWithFlags(&c->ev_b, cudaEventDisableTiming));
