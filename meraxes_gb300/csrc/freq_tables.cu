@@ -18,7 +18,11 @@
 // integrals are the same numbers: the first of them is computed for all.
 //
 // On 16 host threads the tables took 8.4 ms per snapshot, longer than the
-// shells' transforms of any grid below 512^3.
+// shells' transforms of any grid below 512^3.  Here (40 shells, one E0)
+// k_tau_lower takes 171 us, 20 steps one after another, and k_freq_integrals
+// 354 us, bound by the bisections of the longest integral (30 and more rounds)
+// at the FP64 rate and latency; with the cross sections' formulas instead of
+// their polynomials they took 360 and 986 us.
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -62,25 +66,48 @@ struct Panel
   double result, abserr, resabs, resasc;
 };
 
-// Sum of NV values over the 64 threads of a panel (two warps); every thread
-// of the block calls it.  `sh` holds 2 x NV doubles per panel.
-template <int NV>
-__device__ __forceinline__ void panel_sum(double (&v)[NV], double* sh)
+// The sums of one panel: Kronrod, Gauss, Kronrod of |f|, and Kronrod of
+// |f - mean|, two warps' parts each.
+struct PanelSums
 {
+  double part[2][4], asc[2];
+};
+
+// Sums of v[0..3] over a warp, sum i in the lanes with (lane & 3) == i: the
+// first two exchanges halve the values that a lane carries, so that the four
+// sums take six additions (at 16 cycles each per warp) instead of twenty.
+__device__ __forceinline__ double warp_sum4(const double (&v)[4])
+{
+  const int lane = threadIdx.x & 31;
+  const bool hi = lane & 2, odd = lane & 1;
+  double a = hi ? v[2] : v[0], b = hi ? v[3] : v[1];
+  a += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 2);
+  b += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 2);
+  double s = odd ? b : a;
+  s += __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
 #pragma unroll
-  for (int q = 0; q < NV; q++)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  for (int o = 4; o < 32; o <<= 1)
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// The panel's sums from the integrand values f of its 64 threads (0 in the
+// last three), in p; the block calls it for all its panels together.  The
+// sums may be read after the next block barrier.
+__device__ __forceinline__ void panel_sums(double f, const Rule& w, PanelSums& p)
+{
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 1;
+  const double s = warp_sum4({ w.wk * f, w.wg * f, w.wk * fabs(f), 0.0 });
+  if (lane < 4)
+    p.part[warp][lane] = s;
   __syncthreads();
-  if ((threadIdx.x & 31) == 0)
+  const double mean = (p.part[0][0] + p.part[1][0]) * 0.5;
+  double c = w.wk * fabs(f - mean);
 #pragma unroll
-    for (int q = 0; q < NV; q++)
-      sh[((threadIdx.x >> 5) & 1) * NV + q] = v[q];
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < NV; q++)
-    v[q] = sh[q] + sh[NV + q];
+  for (int o = 1; o < 32; o <<= 1)
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  if (lane == 0)
+    p.asc[warp] = c;
 }
 
 __device__ double rescale_err(double err, double res_abs, double res_asc)
@@ -99,19 +126,15 @@ __device__ double rescale_err(double err, double res_abs, double res_asc)
   return err;
 }
 
-// The panel's sums from the 61 threads' integrand values f (0 in the others).
-__device__ Panel panel_of(double f, const Rule& w, double a, double b, double* sh)
+__device__ Panel panel_of(const PanelSums& s, double a, double b)
 {
   const double half = 0.5 * (b - a), ahalf = fabs(half);
-  double v[3] = { w.wk * f, w.wg * f, w.wk * fabs(f) };
-  panel_sum<3>(v, sh);
-  double u[1] = { w.wk * fabs(f - v[0] * 0.5) };
-  panel_sum<1>(u, sh);
+  const double rk = s.part[0][0] + s.part[1][0], rg = s.part[0][1] + s.part[1][1];
   Panel p;
-  p.result = v[0] * half;
-  p.resabs = v[2] * ahalf;
-  p.resasc = u[0] * ahalf;
-  p.abserr = rescale_err((v[0] - v[1]) * half, p.resabs, p.resasc);
+  p.result = rk * half;
+  p.resabs = (s.part[0][2] + s.part[1][2]) * ahalf;
+  p.resasc = (s.asc[0] + s.asc[1]) * ahalf;
+  p.abserr = rescale_err((rk - rg) * half, p.resabs, p.resasc);
   return p;
 }
 
@@ -123,8 +146,8 @@ struct Qag
   int order[FREQ_INTERVALS];
   int size, nrmax, i, rt1, rt2, etype, more;
   double area, errsum, tol, epsrel, result;
-  double red[16];    // panel_sum scratch
-  Panel second;      // the upper half's panel
+  PanelSums sums[2];
+  Panel panel[2];
 
   __device__ void sort_errors()
   {
@@ -231,7 +254,8 @@ struct Qag
 };
 
 // ---------------------------------------------------------- cross sections
-// XRayHeatingFunctions.c:823-900; eps = sqrt(nu / nu0 - 1)
+// The formulas (XRayHeatingFunctions.c:823-900; eps = sqrt(nu / nu0 - 1)), for
+// frequencies near and below a threshold.
 __device__ double xs_hydrogenic(double nu, double nu0, double sigma)
 {
   if (nu < nu0)
@@ -242,10 +266,10 @@ __device__ double xs_hydrogenic(double nu, double nu0, double sigma)
   const double eps = sqrt(nu / nu0 - 1), ieps = 1.0 / eps;
   return sigma * (q2 * q2) * exp(4 - (4 * atan(eps) * ieps)) / (1 - exp(-2 * k::PI * ieps));
 }
-__device__ __forceinline__ double xs_HI(double nu) { return xs_hydrogenic(nu, k::NU_HI, k::SIGMA_HI); }
-__device__ __forceinline__ double xs_HeII(double nu) { return xs_hydrogenic(nu, k::NU_HEII, 6.3e-18 / 4); }
-__device__ double xs_HeI(double nu)
+__device__ __noinline__ double xs_formula(int q, double nu)
 {
+  if (q != 1)
+    return q == 0 ? xs_hydrogenic(nu, k::NU_HI, k::SIGMA_HI) : xs_hydrogenic(nu, k::NU_HEII, 6.3e-18 / 4);
   if (nu < k::NU_HEI)
     return 0;
   const double x = nu * (1.0 / k::NU_OVER_EV / 13.61) - 0.4434;
@@ -253,6 +277,48 @@ __device__ double xs_HeI(double nu)
   // y^(0.5 * 3.188 - 5.5) (1 + sqrt(y / 1.469))^-3.188
   return 9.492e-16 * ((x - 1) * (x - 1) + 2.039 * 2.039) *
          exp((0.5 * 3.188 - 5.5) * log(y) - 3.188 * log(1.0 + sqrt(y * (1.0 / 1.469))));
+}
+
+// Interval and local coordinate of nu in the polynomial tables.  The tables
+// agree with the formulas to 4e-16 of the value, at 9 multiply-adds instead
+// of roots, exponentials, logarithms and an arctangent (several hundred
+// operations at the FP64 rate).
+struct XsAt
+{
+  int i;
+  double t;
+};
+__device__ __forceinline__ XsAt xs_at(double nu)
+{
+  const double x = nu * (1.0 / k::NU_HI);
+  const int hi = __double2hiint(x);
+  const int sub = (hi >> 16) & (XS_SUB - 1);  // leading mantissa bits
+  XsAt p;
+  p.i = ((hi >> 20) - 1023) * XS_SUB + sub;  // x > 0: the sign bit is clear
+  const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
+  p.t = (m - (1.0 + (sub + 0.5) / XS_SUB)) * (2.0 * XS_SUB);
+  return p;
+}
+// first interval at or above 1.5 thresholds: x = 1.5, 2.7122 (2.75), 6
+__device__ __forceinline__ bool xs_in_table(int q, int i)
+{
+  return i >= (q == 0 ? XS_SUB / 2 : (q == 1 ? XS_SUB + 3 * XS_SUB / 8 : 2 * XS_SUB + XS_SUB / 2)) && i < XS_INTERVALS;
+}
+__device__ __forceinline__ double xs_poly(const double (&tab)[XS_INTERVALS][XS_N], const XsAt& p)
+{
+  const double2* c = reinterpret_cast<const double2*>(tab[p.i]);
+  double2 v[XS_N / 2];
+#pragma unroll
+  for (int j = 0; j < XS_N / 2; j++)
+    v[j] = __ldg(c + j);
+  double s = v[XS_N / 2 - 1].y;
+#pragma unroll
+  for (int j = XS_N / 2 - 1; j >= 0; j--) {
+    s = fma(s, p.t, v[j].x);
+    if (j > 0)
+      s = fma(s, p.t, v[j - 1].y);
+  }
+  return s;
 }
 
 // ---------------------------------------------------------- optical depth
@@ -292,7 +358,7 @@ __global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant
   const double zpp = a.zpp[r], zp = a.zp;
   const double z0 = 0.5 * (zpp + zp) + 0.5 * (zp - zpp) * w.x;
   const double factor0 = j < 61 ? tau_factor(a, z0, fcoll1, x_e) : 0.0;
-  const double sH = a.f_h * (1 - x_e), sHe = a.f_he * (1 - x_e), sHe2 = a.f_he * x_e;
+  const double share[3] = { a.f_h * (1 - x_e), a.f_he * (1 - x_e), a.f_he * x_e };
   // tau_X(nu): the integral from zpp to zp
   auto tau = [&](double nu) {
     const double nu0 = nu / (1 + zp);
@@ -300,25 +366,29 @@ __global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant
       if (j >= 61)
         return 0.0;
       const double nuhat = nu0 * (1 + zhat);
-      return factor * (sH * xs_HI(nuhat) + sHe * xs_HeI(nuhat) + sHe2 * xs_HeII(nuhat));
+      const XsAt p = xs_at(nuhat);
+      double sig = 0;
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+        sig += share[q] * (xs_in_table(q, p.i) ? xs_poly(a.tables->xs[q], p) : xs_formula(q, nuhat));
+      return factor * sig;
     };
-    const Panel p = panel_of(value(z0, factor0), w, zpp, zp, q.red);
+    panel_sums(value(z0, factor0), w, q.sums[0]);
     __syncthreads();
     if (j == 0)
-      q.begin(p, zpp, zp, 0.005);
+      q.begin(panel_of(q.sums[0], zpp, zp), zpp, zp, 0.005);
     __syncthreads();
     while (q.more) {
       const double lo = q.a[q.i], hi = q.b[q.i], mid = 0.5 * (lo + hi);
-      Panel half[2];
 #pragma unroll 1
       for (int h = 0; h < 2; h++) {
         const double pa = h ? mid : lo, pb = h ? hi : mid;
         const double z = 0.5 * (pa + pb) + 0.5 * (pb - pa) * w.x;
-        half[h] = panel_of(value(z, tau_factor(a, z, fcoll1, x_e)), w, pa, pb, q.red);
+        panel_sums(value(z, tau_factor(a, z, fcoll1, x_e)), w, q.sums[h]);
       }
       __syncthreads();
       if (j == 0)
-        q.step(half[0], half[1], &a.out->fail);
+        q.step(panel_of(q.sums[0], lo, mid), panel_of(q.sums[1], mid, hi), &a.out->fail);
       __syncthreads();
     }
     return q.result;
@@ -408,12 +478,11 @@ struct EnergyBin
   int n;  // -1: below the table
   float dE, width;
 };
-__device__ EnergyBin energy_bin(const FreqDevTables& t, double E)
+__device__ __forceinline__ EnergyBin energy_bin(const FreqDevTables& t, float En)
 {
   EnergyBin b;
-  float En = (float)E;
-  if (En > 0.999 * t.energy[k::NENERGY - 1]) {
-    En = (float)(t.energy[k::NENERGY - 1] * 0.999);
+  if (En > t.energy_cap) {
+    En = t.energy_top;
   } else if (En < t.energy[0]) {
     b.n = -1;
     return b;
@@ -450,27 +519,31 @@ __device__ float interp(const FreqDevTables& t, const float (*tab)[k::NENERGY], 
   return v + lo;
 }
 
-__device__ double integrand(const FreqArgs& a, double nu, int flag, int xi, double E0nu)
+__device__ __forceinline__ double integrand(const FreqArgs& a, double nu, int flag, int xi, double spec)
 {
   const FreqDevTables& t = *a.tables;
   const double xe = t.xhii[xi];
   const double nus[3] = { k::NU_HI, k::NU_HEI, k::NU_HEII };
-  const double xs[3] = { a.f_h * (1 - xe) * xs_HI(nu), a.f_he * (1 - xe) * xs_HeI(nu), a.f_he * xe * xs_HeII(nu) };
+  const double share[3] = { a.f_h * (1 - xe), a.f_he * (1 - xe), a.f_he * xe };
+  const XsAt p = xs_at(nu);
+  const double eV = nu * (1.0 / k::NU_OVER_EV);
   double s = 0;
-#pragma unroll 1
+#pragma unroll
   for (int q = 0; q < 3; q++) {
-    const EnergyBin b = energy_bin(t, (nu - nus[q]) * (1.0 / k::NU_OVER_EV));
-    double c;
+    const EnergyBin b = energy_bin(t, (float)(eV - nus[q] / k::NU_OVER_EV));
+    double c = share[q];
     if (flag == 0)
-      c = (double)interp(t, t.fheat, 1.0f, b, xi) * k::PLANCK * (nu - nus[q]);
+      c *= (double)interp(t, t.fheat, 1.0f, b, xi) * (nu - nus[q]);
     else if (flag == 1)
-      c = (double)(interp(t, t.nion[0], 0.0f, b, xi) + interp(t, t.nion[1], 0.0f, b, xi) +
-                   interp(t, t.nion[2], 0.0f, b, xi) + 1);
+      c *= (double)(interp(t, t.nion[0], 0.0f, b, xi) + interp(t, t.nion[1], 0.0f, b, xi) +
+                    interp(t, t.nion[2], 0.0f, b, xi) + 1);
     else
-      c = (double)interp(t, t.nlya, 0.0f, b, xi);
-    s += c * xs[q];
+      c *= (double)interp(t, t.nlya, 0.0f, b, xi);
+    const double xs = xs_in_table(q, p.i) ? xs_poly(t.xs_spec[q], p)
+                                          : xs_formula(q, nu) * exp((-a.alpha - 1) * log(nu * (1.0 / k::NU_HI)));
+    s = fma(c, xs, s);
   }
-  return s * exp((-a.alpha - 1) * log(nu / E0nu));
+  return s * spec;
 }
 
 __global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_constant__ FreqArgs a)
@@ -493,25 +566,28 @@ __global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_con
   const double lower = at_E0 ? E0nu : a.out->nu1[r];
   const int j = threadIdx.x & 63, h = threadIdx.x >> 6;
   const Rule w = rule_of(j);
-  auto panel = [&](double pa, double pb) {
-    const double f = j < 61 ? integrand(a, 0.5 * (pa + pb) + 0.5 * (pb - pa) * w.x, flag, xi, E0nu) : 0.0;
-    return panel_of(f, w, pa, pb, q.red + 8 * h);
-  };
-  {
-    const Panel p = panel(lower, a.numax);
+  // the factors that do not depend on nu or the species
+  const double spec = a.spec[set] * (flag == 0 ? k::PLANCK : 1.0);
+  auto sums = [&](double pa, double pb) {
+    const double f = j < 61 ? integrand(a, 0.5 * (pa + pb) + 0.5 * (pb - pa) * w.x, flag, xi, spec) : 0.0;
+    panel_sums(f, w, q.sums[h]);
     __syncthreads();
-    if (threadIdx.x == 0)
-      q.begin(p, lower, a.numax, 0.01);
-  }
+  };
+  sums(lower, a.numax);
+  if (threadIdx.x == 0)
+    q.begin(panel_of(q.sums[0], lower, a.numax), lower, a.numax, 0.01);
   __syncthreads();
   while (q.more) {
     const double lo = q.a[q.i], hi = q.b[q.i], mid = 0.5 * (lo + hi);
-    const Panel p = panel(h ? mid : lo, h ? hi : mid);
-    if (threadIdx.x == 64)
-      q.second = p;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      q.step(p, q.second, &a.out->fail);
+    sums(h ? mid : lo, h ? hi : mid);
+    if (threadIdx.x < 2) {
+      // the two panels' error estimates side by side, then the bookkeeping
+      const int u = threadIdx.x;
+      q.panel[u] = panel_of(q.sums[u], u ? mid : lo, u ? hi : mid);
+      __syncwarp(3u);
+      if (u == 0)
+        q.step(q.panel[0], q.panel[1], &a.out->fail);
+    }
     __syncthreads();
   }
   if (threadIdx.x < a.S) {
@@ -525,8 +601,45 @@ __global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_con
 }
 }  // namespace
 
-void fill_freq_dev_tables(const HeatTables& ht, FreqDevTables* t)
+// Interpolation at the Chebyshev nodes of each interval, as powers of the local
+// coordinate.
+static void fill_xs(double alpha, FreqDevTables* t)
 {
+  double (*xs[3])(double) = { xs_HI, xs_HeI, xs_HeII };
+  double node[XS_N], cheb[XS_N][XS_N] = {};  // cheb[j]: powers of T_j
+  for (int n = 0; n < XS_N; n++)
+    node[n] = std::cos(k::PI * (n + 0.5) / XS_N);
+  cheb[0][0] = cheb[1][1] = 1.0;
+  for (int j = 2; j < XS_N; j++)
+    for (int m = 0; m < XS_N; m++)
+      cheb[j][m] = (m ? 2.0 * cheb[j - 1][m - 1] : 0.0) - cheb[j - 2][m];
+  for (int i = 0; i < XS_INTERVALS; i++)
+    for (int q = 0; q < 3; q++) {
+      double v[2][XS_N];
+      for (int n = 0; n < XS_N; n++) {
+        const double x = std::ldexp(1.0 + (i % XS_SUB + 0.5 + 0.5 * node[n]) / XS_SUB, i / XS_SUB);
+        v[0][n] = xs[q](x * k::NU_HI);
+        v[1][n] = v[0][n] * std::pow(x, -alpha - 1);
+      }
+      double (*out[2])[XS_N] = { &t->xs[q][i], &t->xs_spec[q][i] };
+      for (int w = 0; w < 2; w++) {
+        for (int m = 0; m < XS_N; m++)
+          (*out[w])[m] = 0.0;
+        for (int j = 0; j < XS_N; j++) {
+          double c = 0.0;
+          for (int n = 0; n < XS_N; n++)
+            c += v[w][n] * std::cos(k::PI * j * (n + 0.5) / XS_N);
+          c *= (j ? 2.0 : 1.0) / XS_N;
+          for (int m = 0; m <= j; m++)
+            (*out[w])[m] += c * cheb[j][m];
+        }
+      }
+    }
+}
+
+void fill_freq_dev_tables(const HeatTables& ht, double alpha, FreqDevTables* t)
+{
+  fill_xs(alpha, t);
   std::memcpy(t->energy, ht.energy, sizeof(t->energy));
   std::memcpy(t->xhii, ht.xhii, sizeof(t->xhii));
   std::memcpy(t->fheat, ht.fheat, sizeof(t->fheat));
@@ -534,6 +647,11 @@ void fill_freq_dev_tables(const HeatTables& ht, FreqDevTables* t)
   std::memcpy(t->nion[0], ht.nion_hi, sizeof(t->nion[0]));
   std::memcpy(t->nion[1], ht.nion_hei, sizeof(t->nion[1]));
   std::memcpy(t->nion[2], ht.nion_heii, sizeof(t->nion[2]));
+  // the last energy's 0.999 as interp_tab compares (in double) and takes it:
+  // the largest float not above it, and its float
+  const double cap = 0.999 * ht.energy[k::NENERGY - 1];
+  t->energy_top = (float)(ht.energy[k::NENERGY - 1] * 0.999);
+  t->energy_cap = (double)(float)cap > cap ? std::nextafter((float)cap, 0.0f) : (float)cap;
   // loc_energy does not decrease with the energy: bisect the float at which
   // it reaches n
   const float top = ht.energy[k::NENERGY - 1];
@@ -559,11 +677,10 @@ FreqArgs make_freq_args(const mx_params& p, const Derived& d, const std::vector<
 {
   FreqArgs a{};
   a.S = sp.S;
-  a.n_sets = 1;
+
   a.zp = zz[snapshot];
   for (int r = 0; r < sp.S; r++)
     a.zpp[r] = shell_redshift(sp, a.zp, r);
-  a.E0[0] = p.nu_xray_gal_threshold;
   a.alpha = p.spec_index_xray_gal;
   a.numax = p.nu_xray_max * k::NU_OVER_EV;
   a.hubble = hubble(p, (float)a.zp);

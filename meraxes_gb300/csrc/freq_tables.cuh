@@ -11,16 +11,25 @@ namespace mx {
 constexpr int FREQ_SETS = 3;  // X-ray thresholds E0 of one call (the adjoint needs three)
 constexpr int FREQ_TAB = 3 * k::NXHII;  // rows of a set: tab[(flag * 14 + x) * S + r]
 
-// The secondary-electron tables and the bin edges of their energy index.
+// Cross sections as polynomials: a sixteenth of an octave in nu / NU_HI per
+// interval, XS_N coefficients in its local coordinate (-1 ... 1), from 1.5
+// times the species' threshold (below, the formulas) to 2^17 NU_HI.
+constexpr int XS_SUB = 16, XS_OCTAVES = 17, XS_INTERVALS = XS_SUB * XS_OCTAVES, XS_N = 10;
+
+// The secondary-electron tables, the bin edges of their energy index, and the
+// cross sections of HI, HeI and HeII (xs), and times (nu / NU_HI)^(-alpha - 1)
+// (xs_spec).
 struct FreqDevTables
 {
+  double xs[3][XS_INTERVALS][XS_N], xs_spec[3][XS_INTERVALS][XS_N];
   float energy[k::NENERGY];
+  float energy_cap, energy_top;  // energies above cap are looked up at top
   float edge[k::NENERGY + 1];  // smallest energy whose index (loc_energy) is n
   float xhii[k::NXHII];
   float fheat[k::NXHII][k::NENERGY], nlya[k::NXHII][k::NENERGY];
   float nion[3][k::NXHII][k::NENERGY];
 };
-void fill_freq_dev_tables(const HeatTables& ht, FreqDevTables* t);
+void fill_freq_dev_tables(const HeatTables& ht, double alpha, FreqDevTables* t);
 
 // What the kernels write: the frequency of unit optical depth of each shell,
 // the tables (S entries per row), and whether an integral needed more
@@ -39,7 +48,8 @@ struct FreqArgs
   double total;                 // cells
   int S, n_sets;
   double zp, zpp[MAX_SHELLS];
-  double E0[FREQ_SETS];  // NuXrayGalThreshold [eV]
+  double E0[FREQ_SETS];    // NuXrayGalThreshold [eV]
+  double spec[FREQ_SETS];  // (NU_HI / E0)^(-alpha - 1)
   double alpha, numax, hubble;
   double om, ol, hubble_h, n_b0, f_h, f_he, eff;
   // collapse fraction over redshift (interpolate_fcoll): linear from fcoll0 at

@@ -873,7 +873,6 @@ ShellPlan plan_shells(const mx_params& p, const std::vector<double>& zz, int sna
 }
 
 // ====================================================== frequency tables
-namespace {
 double xs_HI(double nu)
 {
   if (nu < k::NU_HI)
@@ -904,8 +903,6 @@ double xs_HeI(double nu)
   return 9.492e-16 * ((x - 1) * (x - 1) + 2.039 * 2.039) * std::pow(y, (0.5 * 3.188 - 5.5)) *
          std::pow(1.0 + std::sqrt(y / 1.469), -3.188);
 }
-
-}  // namespace
 
 int loc_energy(float En)
 {

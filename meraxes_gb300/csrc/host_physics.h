@@ -198,5 +198,10 @@ void build_freq_scalars(const mx_params& p,
                         FreqTables* out);
 // Energy-table bin of a photoelectron energy (XRayHeatingFunctions.c:914-940).
 int loc_energy(float En);
+// Photoionisation cross sections of HI, HeI and HeII (XRayHeatingFunctions.c:
+// 823-900).
+double xs_HI(double nu);
+double xs_HeI(double nu);
+double xs_HeII(double nu);
 
 }  // namespace mx

@@ -410,7 +410,7 @@ void mx_ctx::alloc_scratch()
     MX_CUDA(cudaMalloc(&d_ft, sizeof(FreqDevResult)));
     MX_CUDA(cudaMallocHost(&h_ft, sizeof(FreqDevResult)));
     std::unique_ptr<FreqDevTables> ft(new FreqDevTables());
-    fill_freq_dev_tables(ht, ft.get());
+    fill_freq_dev_tables(ht, p.spec_index_xray_gal, ft.get());
     MX_CUDA(cudaMemcpy(d_ft_tables, ft.get(), sizeof(FreqDevTables), cudaMemcpyHostToDevice));
   }
   // forward transform: padded real input -> half spectrum (out of place)
@@ -1049,8 +1049,10 @@ static void launch_tables(mx_ctx* c, const ShellPlan& sp, int snapshot, const st
   a.sums = c->d_sums;
   a.total = (double)c->gd.N;
   a.n_sets = (int)E0.size();
-  for (int i = 0; i < a.n_sets; i++)
+  for (int i = 0; i < a.n_sets; i++) {
     a.E0[i] = E0[i];
+    a.spec[i] = std::pow(k::NU_HI / (E0[i] * k::NU_OVER_EV), -a.alpha - 1);
+  }
   a.out = c->d_ft;
   Prof pr(c, "freq_tables", 0.0, fs);
   launch_freq_tables(a, fs);
