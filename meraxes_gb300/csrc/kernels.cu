@@ -384,21 +384,28 @@ void launch_fhb_reduce(const FhbReduceArgs& a, const GridDims& gd, cudaStream_t 
   g_launches++;
 }
 
-__global__ void k_finalize(const double* __restrict__ partials, int nvals, int nblocks, double* __restrict__ out)
+// A warp per value: lane l adds the partials of blocks l, l + 32, ... in order,
+// then the lanes are added in a fixed tree.  One thread per value, a chain of
+// RED_BLOCKS dependent FP64 additions, took 47 us.
+__global__ void __launch_bounds__(RED_THREADS) k_finalize(const double* __restrict__ partials, int nvals, int nblocks,
+                                                          double* __restrict__ out)
 {
-  // one thread per value, fixed summation order over blocks
-  const int v = threadIdx.x;
-  if (v < nvals) {
+  const int lane = threadIdx.x & 31;
+  for (int v = threadIdx.x >> 5; v < nvals; v += RED_THREADS / 32) {
     double s = 0.0;
-    for (int b = 0; b < nblocks; b++)
+#pragma unroll 4
+    for (int b = lane; b < nblocks; b += 32)
       s += partials[(long long)b * nvals + v];
-    out[v] = s;
+    for (int o = 16; o > 0; o >>= 1)
+      s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0)
+      out[v] = s;
   }
 }
 
 void launch_finalize(const double* partials, int nvals, double* out, cudaStream_t s, int nblocks)
 {
-  k_finalize<<<1, 32, 0, s>>>(partials, nvals, nblocks, out);
+  k_finalize<<<1, RED_THREADS, 0, s>>>(partials, nvals, nblocks, out);
   g_launches++;
 }
 
@@ -408,9 +415,24 @@ __global__ void k_fill(float* p, long long n, float v)
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     p[i] = v;
 }
-void launch_fill(float* p, long long n, float v, cudaStream_t s)
+// The state that find_HII_bubbles starts from (find_HII_bubbles.c:102-116), one
+// launch for the three grids; n2 = cells / 2 (grid sizes are even, device grids
+// 8-byte aligned).  J_21 may be NULL.
+__global__ void k_fhb_init(float2* __restrict__ xH, float2* __restrict__ r_bubble, float2* __restrict__ J21,
+                           long long n2)
 {
-  k_fill<<<blocks_for(n, 256), 256, 0, s>>>(p, n, v);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2; i += (long long)gridDim.x * blockDim.x) {
+    xH[i] = make_float2(1.0f, 1.0f);
+    r_bubble[i] = make_float2(0.0f, 0.0f);
+    if (J21)
+      J21[i] = make_float2(0.0f, 0.0f);
+  }
+}
+void launch_fhb_init(float* xH, float* r_bubble, float* J21, const GridDims& gd, cudaStream_t s)
+{
+  k_fhb_init<<<blocks_for(gd.N / 2, 256), 256, 0, s>>>(reinterpret_cast<float2*>(xH),
+                                                        reinterpret_cast<float2*>(r_bubble),
+                                                        reinterpret_cast<float2*>(J21), gd.N / 2);
   g_launches++;
 }
 __global__ void k_fill_real_in_padded(float* p, int D, int H, long long N, float v)

@@ -142,7 +142,7 @@ void launch_fhb_reduce(const FhbReduceArgs& a, const GridDims& gd, cudaStream_t 
 void launch_finalize(const double* partials, int nvals, double* out, cudaStream_t s, int nblocks = RED_BLOCKS);
 
 // ------------------------------------------------------------ grid helpers
-void launch_fill(float* p, long long n, float v, cudaStream_t s);
+void launch_fhb_init(float* xH, float* r_bubble, float* J21, const GridDims& gd, cudaStream_t s);
 void launch_fill_real_in_padded(float* p, const GridDims& gd, float v, cudaStream_t s);
 
 // ---------------------------------------------------------------- ComputeTs

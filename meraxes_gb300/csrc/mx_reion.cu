@@ -520,14 +520,9 @@ static void run_find_HII_bubbles(mx_ctx* c, int snapshot, const mx_grids* g, mx_
 
   // initial state (find_HII_bubbles.c:102-116)
   const double B4N = 4.0 * (double)gd.N, B8C = 8.0 * (double)gd.C;
-  if (uvb) {
-    Prof pr(c, "k_fill", B4N, s);
-    launch_fill(g->J_21, gd.N, 0.0f, s);
-  }
   {
-    Prof pr(c, "k_fill", 2 * B4N, s);
-    launch_fill(g->xH, gd.N, 1.0f, s);
-    launch_fill(g->r_bubble, gd.N, 0.0f, s);
+    Prof pr(c, "k_fhb_init", (uvb ? 3 : 2) * B4N, s);
+    launch_fhb_init(g->xH, g->r_bubble, uvb ? g->J_21 : nullptr, gd, s);
   }
 
   // forward transforms of the G fields (find_HII_bubbles.c:118-163)

@@ -42,16 +42,23 @@ __global__ void k_ps_sum(const float* __restrict__ dT, long long N, double* part
   }
 }
 
-// sums[v] = sum over blocks of partials[b * nvals + v], fixed order
-__global__ void k_ps_finalize(const double* __restrict__ partials, int nblocks, int nvals, double* __restrict__ sums)
+// sums[v] = sum over blocks of partials[b * nvals + v], fixed order, a warp per
+// value (see k_finalize, kernels.cu)
+constexpr int FIN_WARPS = 4;
+__global__ void __launch_bounds__(32 * FIN_WARPS) k_ps_finalize(const double* __restrict__ partials, int nblocks,
+                                                                int nvals, double* __restrict__ sums)
 {
-  const int v = threadIdx.x;
-  if (v < nvals) {
-    double s = 0.0;
-    for (int b = 0; b < nblocks; b++)
-      s += partials[(long long)b * nvals + v];
+  const int lane = threadIdx.x & 31, v = blockIdx.x * FIN_WARPS + (threadIdx.x >> 5);
+  if (v >= nvals)
+    return;
+  double s = 0.0;
+#pragma unroll 4
+  for (int b = lane; b < nblocks; b += 32)
+    s += partials[(long long)b * nvals + v];
+  for (int o = 16; o > 0; o >>= 1)
+    s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0)
     sums[v] = s;
-  }
 }
 
 // ComputePowerSpectrum.c:94-110
@@ -201,7 +208,7 @@ __global__ void k_padded_to_real(const float* __restrict__ in, float scale, int 
 void launch_ps_mean(const float* dT, long long N, double* partials, double* sum, cudaStream_t s)
 {
   k_ps_sum<<<RED_BLOCKS, RED_THREADS, 0, s>>>(dT, N, partials);
-  k_ps_finalize<<<1, 32, 0, s>>>(partials, RED_BLOCKS, 1, sum);
+  k_ps_finalize<<<1, 32 * FIN_WARPS, 0, s>>>(partials, RED_BLOCKS, 1, sum);
   ps_launches += 2;
 }
 
@@ -215,7 +222,7 @@ void launch_ps_field(const float* dT, const double* sum, float volume, const Gri
 void launch_ps_bin(const PsArgs& a, double* sums, cudaStream_t s)
 {
   k_ps_bin<<<RED_BLOCKS, RED_THREADS, 0, s>>>(a);
-  k_ps_finalize<<<1, 3 * PS_MAX_BINS, 0, s>>>(a.partials, RED_BLOCKS, 3 * a.nb, sums);
+  k_ps_finalize<<<(3 * a.nb + FIN_WARPS - 1) / FIN_WARPS, 32 * FIN_WARPS, 0, s>>>(a.partials, RED_BLOCKS, 3 * a.nb, sums);
   ps_launches += 2;
 }
 
