@@ -77,9 +77,9 @@ __host__ __device__ constexpr int brev(int i, int bits)
 
 // tw[j] = exp(+2 pi i j / D) for j < D
 template <int D>
-__device__ void fill_twiddles(float2* tw)
+__device__ void fill_twiddles(float2* tw, int tid, int nthreads)
 {
-  for (int j = threadIdx.x; j < D; j += blockDim.x) {
+  for (int j = tid; j < D; j += nthreads) {
     float s, c;
     sincospif(2.0f * (float)j / (float)D, &s, &c);
     tw[j] = make_float2(c, s);
@@ -342,6 +342,33 @@ struct TilePlan
   static __device__ __forceinline__ int at(int line, int t) { return line * TXC + t; }
 };
 
+// A tile is transformed by NTHR threads.  Tiles of 128 threads run two to a
+// block of 256 (TILE_GROUPS), each with its own shared memory and its own named
+// barrier; larger tiles have the block to themselves.
+template <int NTHR>
+__host__ __device__ constexpr int tile_groups()
+{
+  return NTHR == 128 ? 2 : 1;
+}
+template <int NTHR>
+__device__ __forceinline__ int tile_tid()
+{
+  return tile_groups<NTHR>() == 2 ? (int)(threadIdx.x & (NTHR - 1)) : (int)threadIdx.x;
+}
+template <int NTHR>
+__device__ __forceinline__ int tile_group()
+{
+  return tile_groups<NTHR>() == 2 ? (int)(threadIdx.x / NTHR) : 0;
+}
+template <int NTHR>
+__device__ __forceinline__ void tile_sync()
+{
+  if constexpr (tile_groups<NTHR>() == 2)
+    asm volatile("barrier.sync %0, %1;" ::"r"(1 + tile_group<NTHR>()), "n"(NTHR) : "memory");
+  else
+    __syncthreads();
+}
+
 // Inverse DFT of the tile's columns in three steps, each a member of
 // TileSteps; the caller puts a barrier between them and after the last one
 // before it reuses buf.  tile_dft() runs all three.
@@ -351,6 +378,19 @@ struct TilePlan
 // so every shared and global access of a half-warp is one 128-byte line.
 // Slot s takes the work items s, s + S, s + 2S, ... of each step; the loops
 // over them are unrolled, so their index arithmetic is constant offsets.
+// shared memory of one tile (float2): twiddles and tile, and the x-pass's
+// filter weights (16-byte multiples)
+template <int D>
+struct YSmem
+{
+  static constexpr int FLOAT2 = D + TilePlan<D>::BUF;
+};
+template <int D>
+struct XSmem
+{
+  static constexpr int FLOAT2 = YSmem<D>::FLOAT2 + ((D / 2 + 1) * TXC + 1) / 2;
+};
+
 template <int D, int NTHR>
 struct TileSteps
 {
@@ -367,7 +407,7 @@ struct TileSteps
   template <class F>
   static __device__ __forceinline__ void for_each_input(F f)
   {
-    const int s = threadIdx.x / TXC;
+    const int s = tile_tid<NTHR>() / TXC;
 #pragma unroll
     for (int j = 0; j < JA; j++) {
       const int np = s + S * j;
@@ -384,7 +424,7 @@ struct TileSteps
   template <class Load>
   static __device__ __forceinline__ void a(float2* buf, const float2* tw, Load load)
   {
-    const int t = threadIdx.x % TXC, s = threadIdx.x / TXC;
+    const int t = tile_tid<NTHR>() % TXC, s = tile_tid<NTHR>() / TXC;
     float2* col = buf + t;
 #pragma unroll
     for (int j = 0; j < JA; j++) {
@@ -406,7 +446,7 @@ struct TileSteps
   // step B: items (n3, k1) with n3 = s % R3 fixed
   static __device__ __forceinline__ void b(float2* buf, const float2* tw)
   {
-    const int t = threadIdx.x % TXC, s = threadIdx.x / TXC;
+    const int t = tile_tid<NTHR>() % TXC, s = tile_tid<NTHR>() / TXC;
     float2* col = buf + t;
     const int n3 = s % R3;
 #pragma unroll
@@ -432,7 +472,7 @@ struct TileSteps
   template <class Store>
   static __device__ __forceinline__ void c(const float2* buf, Store store)
   {
-    const int t = threadIdx.x % TXC, s = threadIdx.x / TXC;
+    const int t = tile_tid<NTHR>() % TXC, s = tile_tid<NTHR>() / TXC;
     const float2* col = buf + t;
     const int k2 = s % R2;
 #pragma unroll
@@ -458,9 +498,9 @@ __device__ __forceinline__ void tile_dft(float2* buf, const float2* tw, Load loa
 {
   using T = TileSteps<D, NTHR>;
   T::a(buf, tw, load);
-  __syncthreads();
+  tile_sync<NTHR>();
   T::b(buf, tw);
-  __syncthreads();
+  tile_sync<NTHR>();
   T::c(buf, store);
 }
 
@@ -479,25 +519,42 @@ __device__ __forceinline__ void tile_dft(float2* buf, const float2* tw, Load loa
 // sincosf) measured slower: the table read before the block's barrier is a
 // DRAM wait that the weights' arithmetic is not (a 28-radius one-field batch
 // at 512^3 took 8.75 ms with tables, 5.90 ms without).
-// XTHREADS threads per block: 256 or 512 (the context's autotuner picks).
+// XTHREADS threads per tile: 128 (64^3 and 128^3), 256 or 512 (the context's
+// autotuner picks).  A tile of a small grid has few points: 128 threads hold
+// D / 8 of them each, all in flight at once, and more tiles fit on an SM whose
+// barriers and loads are independent of each other (us for 41 radii of 5
+// fields with 128, 256, 512 threads: 64^3 125, 126, 184; 128^3 726, 836, 1047;
+// 256^3 6202, 5456, 5923).
+template <int D>
+constexpr bool X_TILE_128 = D == 64 || D == 128;
 template <int D, int XTHREADS>
-__global__ void __launch_bounds__(XTHREADS, XTHREADS == 256 && D < 512 ? 3 : 2) k_fft_x_filter(const __grid_constant__ XPassArgs a)
+constexpr int x_min_blocks()
+{
+  return XTHREADS == 128 ? 4 : (XTHREADS == 256 && D < 512 ? 3 : 2);
+}
+template <int D, int XTHREADS>
+__global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_blocks<D, XTHREADS>())
+  k_fft_x_filter(const __grid_constant__ XPassArgs a)
 {
   using P = TilePlan<D>;
   constexpr int H = D / 2 + 1;
   extern __shared__ float2 smem[];
-  float2* tw = smem;
-  float2* buf = smem + D;
+  const int tid = tile_tid<XTHREADS>();
+  float2* tw = smem + tile_group<XTHREADS>() * XSmem<D>::FLOAT2;
+  float2* buf = tw + D;
   float* wsm = reinterpret_cast<float*>(buf + P::BUF);
-  fill_twiddles<D>(tw);
-  const int r = blockIdx.x % a.n;
-  const int tile = blockIdx.x / a.n;
+  const unsigned item = blockIdx.x * tile_groups<XTHREADS>() + tile_group<XTHREADS>();
+  if (item >= (unsigned)(H * P::NT) * a.n)
+    return;
+  fill_twiddles<D>(tw, tid, XTHREADS);
+  const int r = item % a.n;
+  const int tile = item / a.n;
   const int kyp = tile / P::NT;  // |ky|: the block transforms rows ky = kyp and D - kyp
   const int kz0 = (tile % P::NT) * TXC;
   // the weights depend on ky only through kyv^2, the same for both rows
   const float kyv = kcomp(kyp, D, a.delta_k);
   // this thread's column: kz = kz0 + t, the same in every step
-  const int t0 = threadIdx.x % TXC;
+  const int t0 = tid % TXC;
   const bool live = kz0 + t0 < H;
   // the unfiltered points of step A, read into registers before the step
   using T = TileSteps<D, XTHREADS>;
@@ -512,7 +569,7 @@ __global__ void __launch_bounds__(XTHREADS, XTHREADS == 256 && D < 512 ? 3 : 2) 
   // kx) <= D/2, then the first field's points (read after the weights, whose
   // sincosf would otherwise push them out of registers; the reads are in
   // flight across the barrier)
-  for (int i = threadIdx.x; i < H * TXC; i += XTHREADS) {
+  for (int i = tid; i < H * TXC; i += XTHREADS) {
     const int kx = i / TXC, t = i % TXC;
     wsm[i] = a.apply[r] ? x_weight(kx, kyv, kz0 + t, D, a.delta_k, a.filter_type, a.R[r], a.sharpk_max, a.scale)
                         : a.scale;
@@ -523,16 +580,16 @@ __global__ void __launch_bounds__(XTHREADS, XTHREADS == 256 && D < 512 ? 3 : 2) 
     const int ky = h == 0 ? kyp : D - kyp;
     read_points(ky, 0);
     if (h == 0)
-      __syncthreads();
+      tile_sync<XTHREADS>();
     // steps B and C of field g after its step A
     auto finish = [&](int g) {
-      __syncthreads();
+      tile_sync<XTHREADS>();
       T::b(buf, tw);
-      __syncthreads();
+      tile_sync<XTHREADS>();
       float2* __restrict__ dst =
         a.out + (long long)(r * a.G + g) * a.C + (long long)ky * Pitch<D>::HP + kz0 + t0;
       T::c(buf, [&](int x, int, float2 v) { dst[(long long)x * (D * Pitch<D>::HP)] = v; });
-      __syncthreads();
+      tile_sync<XTHREADS>();
     };
     auto step_a = [&]() {
       T::a(buf, tw, [&](int kx, int, int i) {
@@ -575,7 +632,7 @@ __global__ void __launch_bounds__(YTHREADS, YTHREADS == 256 ? 3 : 2) k_fft_y(flo
   using T = TileSteps<D, YTHREADS>;
   float2 pts[T::NPTS];
   T::for_each_input([&](int ky, int i) { pts[i] = col[ky * HP]; });
-  fill_twiddles<D>(tw);
+  fill_twiddles<D>(tw, threadIdx.x, YTHREADS);
   __syncthreads();
   T::a(buf, tw, [&](int, int, int i) { return pts[i]; });
   __syncthreads();
@@ -1197,7 +1254,7 @@ __global__ void __launch_bounds__(T) k_fft_z_r2c(const __grid_constant__ FwdArgs
     if (i < FWD_ROWS * H)
       v[j] = __ldg(src + i);
   }
-  fill_twiddles<L>(tw);
+  fill_twiddles<L>(tw, threadIdx.x, T);
   for (int k = threadIdx.x; k < H; k += T) {
     float sn, cs;
     sincospif(2.0f * (float)k / (float)D, &sn, &cs);
@@ -1256,7 +1313,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_fwd_cols(float2* da
   using TS = TileSteps<D, T>;
   float2 pts[TS::NPTS];
   TS::for_each_input([&](int n, int i) { pts[i] = col[n * LINE]; });
-  fill_twiddles<D>(tw);
+  fill_twiddles<D>(tw, threadIdx.x, T);
   __syncthreads();
   TS::a(buf, tw, [&](int, int, int i) { return make_float2(pts[i].x, -pts[i].y); });
   __syncthreads();
@@ -1298,7 +1355,7 @@ template <int D>
 __device__ __forceinline__ void zg_tables(float2* s2)
 {
   using P = ZGPlan<D>;
-  fill_twiddles<P::L>(s2 + P::OFF_TW);
+  fill_twiddles<P::L>(s2 + P::OFF_TW, threadIdx.x, TILE_THREADS_3);
   for (int k = threadIdx.x; k < P::L; k += TILE_THREADS_3) {
     float sn, cs;
     sincospif(2.0f * (float)k / (float)D, &sn, &cs);
@@ -1537,24 +1594,28 @@ int fft_pitch(int D) { return (D / 2 + 1 + TXC - 1) / TXC * TXC; }
 template <int D>
 constexpr size_t smem_y()
 {
-  return sizeof(float2) * (D + (size_t)TilePlan<D>::BUF);
+  return sizeof(float2) * (size_t)YSmem<D>::FLOAT2;
 }
-template <int D>
+template <int D, int T>
 constexpr size_t smem_x()
 {
-  return smem_y<D>() + sizeof(float) * (size_t)(D / 2 + 1) * TXC;
+  return sizeof(float2) * (size_t)XSmem<D>::FLOAT2 * tile_groups<T>();
 }
-
 template <int D, int T>
 static void launch_x_t(const XPassArgs& a, cudaStream_t s)
 {
-  cudaFuncSetAttribute(k_fft_x_filter<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_x<D>());
-  const long long blocks = (long long)(D / 2 + 1) * TilePlan<D>::NT * a.n;
-  k_fft_x_filter<D, T><<<(unsigned)blocks, T, smem_x<D>(), s>>>(a);
+  const size_t bytes = smem_x<D, T>();
+  cudaFuncSetAttribute(k_fft_x_filter<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const long long tiles = (long long)(D / 2 + 1) * TilePlan<D>::NT * a.n;
+  const long long blocks = (tiles + tile_groups<T>() - 1) / tile_groups<T>();
+  k_fft_x_filter<D, T><<<(unsigned)blocks, T * tile_groups<T>(), bytes, s>>>(a);
 }
 template <int D>
 static void launch_x(const XPassArgs& a, int threads, cudaStream_t s)
 {
+  if constexpr (X_TILE_128<D>)
+    if (threads == 128)
+      return launch_x_t<D, 128>(a, s);
   if (threads == 256)
     launch_x_t<D, 256>(a, s);
   else
@@ -1667,6 +1728,11 @@ bool launch_fft_y(int D, float2* data, long long C, int n_spectra, int threads, 
   }
   fft_launches++;
   return true;
+}
+
+bool fft_x_threads_ok(int D, int threads)
+{
+  return threads == 256 || threads == 512 || (threads == 128 && (D == 64 || D == 128));
 }
 
 int fft_z_rows_per_group(int D) { return fft3d_factor3(D) ? ZG_ROWS : 2048 / D; }

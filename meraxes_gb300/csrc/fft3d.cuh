@@ -70,7 +70,9 @@ int fft_pitch(int D);
 // the filter of the x-pass
 void launch_filter_accumulate(int D, float2* acc, const float2* U, float R, int filter_type, float delta_k,
                               float scale, bool first, cudaStream_t s);
-// threads per block of the x- and y-pass: 256 or 512
+// threads per tile of the passes of a power-of-two grid: 256 or 512, and for
+// the x-pass at 64^3 and 128^3 also 128 (two tiles to a block of 256)
+bool fft_x_threads_ok(int D, int threads);
 bool launch_fft_x_filter(int D, const XPassArgs& a, int threads, cudaStream_t s);
 bool launch_fft_y(int D, float2* data, long long C, int n_spectra, int threads, cudaStream_t s);
 // three launches: z (real rows -> half spectrum), y, x; threads of the y and

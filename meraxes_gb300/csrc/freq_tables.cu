@@ -606,9 +606,12 @@ __global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_con
 static void fill_xs(double alpha, FreqDevTables* t)
 {
   double (*xs[3])(double) = { xs_HI, xs_HeI, xs_HeII };
-  double node[XS_N], cheb[XS_N][XS_N] = {};  // cheb[j]: powers of T_j
-  for (int n = 0; n < XS_N; n++)
+  double node[XS_N], dct[XS_N][XS_N], cheb[XS_N][XS_N] = {};  // cheb[j]: powers of T_j
+  for (int n = 0; n < XS_N; n++) {
     node[n] = std::cos(k::PI * (n + 0.5) / XS_N);
+    for (int j = 0; j < XS_N; j++)
+      dct[j][n] = std::cos(k::PI * j * (n + 0.5) / XS_N) * (j ? 2.0 : 1.0) / XS_N;
+  }
   cheb[0][0] = cheb[1][1] = 1.0;
   for (int j = 2; j < XS_N; j++)
     for (int m = 0; m < XS_N; m++)
@@ -628,8 +631,7 @@ static void fill_xs(double alpha, FreqDevTables* t)
         for (int j = 0; j < XS_N; j++) {
           double c = 0.0;
           for (int n = 0; n < XS_N; n++)
-            c += v[w][n] * std::cos(k::PI * j * (n + 0.5) / XS_N);
-          c *= (j ? 2.0 : 1.0) / XS_N;
+            c += v[w][n] * dct[j][n];
           for (int m = 0; m <= j; m++)
             (*out[w])[m] += c * cheb[j][m];
         }

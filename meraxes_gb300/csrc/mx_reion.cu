@@ -92,7 +92,7 @@ struct mx_ctx
   // inverse transforms: fused three-pass kernels for power-of-two grids
   // (fft3d.cu), cuFFT otherwise or when MX_TRANSFORM=cufft
   bool fused_fft = false;
-  // threads per block of the fused x- and y-pass, chosen by tune_fft()
+  // threads per tile of the fused x- and y-pass, chosen by tune_fft()
   int x_threads = 512, y_threads = 256;
   // register budget of the threshold z-pass: 2 or 3 resident blocks per SM
   int z_blocks = 2;
@@ -2389,15 +2389,16 @@ int mx_create_limited(const mx_params* params, const char* tables_dir, size_t ma
   return create_ctx(params, tables_dir, max_work_bytes, out);
 }
 
-// Block-size autotuner of the fused x- and y-pass.  Both passes are
-// available with 256 and 512 threads per block and give identical results
+// Block-size autotuner of the fused x- and y-pass.  Both passes are compiled
+// for tiles of 256 and 512 threads (the x-pass of small grids for 128, two tiles
+// to a block, too) and give identical results
 // (the thread count changes only which thread runs which column transform,
-// not the arithmetic).  Which one is faster depends on the grid size: at
-// small grids the larger block hides more latency, at 512^3 the smaller one
-// keeps more blocks resident.  The context times both on its own scratch at
-// creation (a zero spectrum, up to four radii, best of three launches) and
-// keeps the faster.  MX_XPASS_THREADS / MX_YPASS_THREADS (256 or 512) fix a
-// choice; MX_AUTOTUNE=0 keeps the defaults (x 512, y 256).
+// not the arithmetic).  Which one is faster depends on the grid size: a tile
+// of a small grid has few points, at 512^3 the larger block keeps more loads in
+// flight.  The context times them on its own scratch at creation (zero spectra
+// of its fields, up to 16 radii or 1 GB, best of five launches) and keeps the
+// fastest.  MX_XPASS_THREADS / MX_YPASS_THREADS fix a choice; MX_AUTOTUNE=0
+// keeps the defaults (x 512, y 256).
 // Register budget of the threshold z-pass (power-of-two grids): 2 resident
 // blocks per SM (128 registers) or 3 (80, with a few spills).  Timed at
 // context creation on scratch: up to 4 radii of zero spectra of the
@@ -2493,7 +2494,11 @@ static void tune_fft(mx_ctx* c)
     c->x_threads = c->y_threads = 384;
     return;
   }
-  const int fx = env_threads("MX_XPASS_THREADS"), fy = env_threads("MX_YPASS_THREADS");
+  int fx = env_threads("MX_XPASS_THREADS");
+  if (const char* v = std::getenv("MX_XPASS_THREADS"))
+    if (std::atoi(v) == 128 && fft_x_threads_ok(c->gd.D, 128))
+      fx = 128;
+  const int fy = env_threads("MX_YPASS_THREADS");
   if (fx)
     c->x_threads = fx;
   if (fy)
@@ -2503,12 +2508,15 @@ static void tune_fft(mx_ctx* c)
     return;
   const GridDims& gd = c->gd;
   cudaStream_t s = c->stream;
-  MX_CUDA(cudaMemsetAsync(c->d_unf, 0, sizeof(float2) * c->unf_C, s));
-  const int n = (int)std::min<long long>(std::min<long long>(c->work_fields, 4), MAX_RADII);
+  const int G = n_fields(c->p);
+  MX_CUDA(cudaMemsetAsync(c->d_unf, 0, sizeof(float2) * c->unf_C * G, s));
+  const long long spectrum_bytes = (long long)sizeof(float2) * c->work_C;
+  const int n =
+    (int)std::max<long long>(1, std::min<long long>({ c->work_fields / G, (1LL << 30) / (spectrum_bytes * G), 16 }));
   XPassArgs xa;
   for (int f = 0; f < MAX_FIELDS; f++)
-    xa.in[f] = f == 0 ? c->d_unf : nullptr;
-  xa.G = 1;
+    xa.in[f] = f < G ? c->d_unf + (long long)f * c->unf_C : nullptr;
+  xa.G = G;
   xa.n = n;
   xa.out = c->d_work;
   xa.C = c->work_C;
@@ -2525,7 +2533,7 @@ static void tune_fft(mx_ctx* c)
   auto best_ms = [&](auto&& launch) {
     launch();  // warm-up
     float best = 1e30f;
-    for (int i = 0; i < 3; i++) {
+    for (int i = 0; i < 5; i++) {
       cudaEventRecord(e0, s);
       launch();
       cudaEventRecord(e1, s);
@@ -2536,22 +2544,27 @@ static void tune_fft(mx_ctx* c)
     }
     return best;
   };
-  const int cand[2] = { 256, 512 };
-  float tx[2] = { 0, 0 }, ty[2] = { 0, 0 };
-  for (int i = 0; i < 2; i++) {
-    if (!fx)
-      tx[i] = best_ms([&] { launch_fft_x_filter(gd.D, xa, cand[i], s); });
-    if (!fy)
-      ty[i] = best_ms([&] { launch_fft_y(gd.D, c->d_work, c->work_C, n, cand[i], s); });
+  float tx = 1e30f, ty = 1e30f;
+  for (const int t : { 128, 256, 512 }) {
+    if (!fx && fft_x_threads_ok(gd.D, t)) {
+      const float ms = best_ms([&] { launch_fft_x_filter(gd.D, xa, t, s); });
+      if (ms < tx) {
+        tx = ms;
+        c->x_threads = t;
+      }
+    }
+    if (!fy && t >= 256) {
+      const float ms = best_ms([&] { launch_fft_y(gd.D, c->d_work, c->work_C, n * G, t, s); });
+      if (ms < ty) {
+        ty = ms;
+        c->y_threads = t;
+      }
+    }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   MX_CUDA(cudaGetLastError());
   MX_CUDA(cudaStreamSynchronize(s));
-  if (!fx)
-    c->x_threads = tx[0] < tx[1] ? 256 : 512;
-  if (!fy)
-    c->y_threads = ty[0] < ty[1] ? 256 : 512;
 }
 
 static int create_ctx(const mx_params* params, const char* tables_dir, size_t work_cap_bytes, mx_ctx** out)
@@ -2699,7 +2712,8 @@ int mx_fft_block_sizes(const mx_ctx* ctx, int32_t* x_threads, int32_t* y_threads
 {
   if (!ctx || !x_threads || !y_threads)
     return MX_EINVAL;
-  *x_threads = ctx->fused_fft ? ctx->x_threads : 0;
+  // x-pass tiles of 128 threads run two to a block
+  *x_threads = ctx->fused_fft ? std::max(256, ctx->x_threads) : 0;
   *y_threads = ctx->fused_fft ? ctx->y_threads : 0;
   return MX_OK;
 }
