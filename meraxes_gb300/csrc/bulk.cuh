@@ -1,5 +1,6 @@
 // Bulk asynchronous copies global -> shared memory (cp.async.bulk) with
-// completion on an mbarrier, and bounded waits on the barrier.
+// completion on an mbarrier, and bounded waits on the barrier; 16-byte
+// asynchronous copies (cp.async).
 #pragma once
 
 #include <cstdint>
@@ -42,6 +43,19 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned b
     "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
     "l"(src), "r"(bytes), "r"(smem_addr(bar))
     : "memory");
+}
+
+// 16-byte asynchronous copies global -> shared by the calling thread, in groups;
+// both addresses 16-byte aligned.  wait<N>: all but the last N groups are done.
+__device__ __forceinline__ void copy16_async(void* dst, const void* src)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait()
+{
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // Opaque copy of a CUtensorMap (128 bytes, 64-byte aligned), so that kernel
@@ -139,11 +153,15 @@ __device__ __forceinline__ bool mbar_wait_polls(uint64_t* bar, unsigned parity, 
   return false;
 }
 
+// Whether consumers wait the full limit: read once per kernel, so that a wait
+// does not start with a load of the limit.
+__device__ __forceinline__ bool full_waits() { return consumer_wait_polls >= WAIT_LIMIT_ITERS; }
+
 // A consumer's wait for phase `parity` of the barrier; false when it gives
 // up (consumer_wait_polls polls, or about WAIT_LIMIT_NS).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity)
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, bool full)
 {
-  return mbar_wait_polls(bar, parity, consumer_wait_polls);
+  return full ? mbar_wait_polls(bar, parity, WAIT_LIMIT_ITERS) : mbar_wait_polls(bar, parity, consumer_wait_polls);
 }
 
 // The wait of a block that gave up, for its own copies still in flight

@@ -467,6 +467,40 @@ struct TileSteps
     }
   }
 
+  static constexpr int JC = (R1 * R2 + S - 1) / S;  // step-C items per thread
+  static constexpr int NOUT = JC * R3;              // output points per thread
+
+  // output point of this thread's register i (0 ... NOUT - 1), or -1
+  static __device__ __forceinline__ int out_point(int i)
+  {
+    const int s = tile_tid<NTHR>() / TXC, j = i / R3, k3 = i % R3;
+    const int k1 = s / R2 + (S / R2) * j;
+    return (R1 * R2) % S == 0 || k1 < R1 ? k1 + R1 * (s % R2 + R2 * k3) : -1;
+  }
+  // step C into registers: out[i] is output point out_point(i) of column
+  // tid % TXC
+  static __device__ __forceinline__ void c_regs(const float2* buf, float2 (&out)[NOUT])
+  {
+    const int t = tile_tid<NTHR>() % TXC, s = tile_tid<NTHR>() / TXC;
+    const float2* col = buf + t;
+    const int k2 = s % R2;
+#pragma unroll
+    for (int j = 0; j < JC; j++) {
+      const int k1 = s / R2 + (S / R2) * j;
+      if ((R1 * R2) % S == 0 || k1 < R1) {
+        const float2* line = col + (k1 * M + R3 * k2) * TXC;
+        float2 v[R3];
+#pragma unroll
+        for (int n3 = 0; n3 < R3; n3++)
+          v[n3] = line[n3 * TXC];
+        dft_any<R3>(v);
+#pragma unroll
+        for (int k3 = 0; k3 < R3; k3++)
+          out[j * R3 + k3] = v[k3];
+      }
+    }
+  }
+
   // step C: items (k2, k1) with k2 = s % R2 fixed; output k = k1 + R1 (k2 + R2 k3)
   // goes to store(k, t, v)
   template <class Store>
@@ -814,9 +848,11 @@ struct ZTw
   float2 kb, kr;  // w_D^k for the 4 points: kb * kr^i
   float2 fb, fs;  // four-step w_{D/2}^{n2 k1} for slot e: fb * fs^e
   float2 la[3], lb[3];  // lane twiddles w, w^2, w^3 of steps A and B
+  bool full;            // the pipeline waits' limit (bulk.cuh)
   __device__ __forceinline__ void init()
   {
     constexpr int P1 = ZS<D>::P1, P2 = ZS<D>::P2, L1 = P1 / 4, L2 = P2 / 4, DH = D / 2;
+    full = full_waits();
     const int l = threadIdx.x % L1, n2 = (threadIdx.x / L1) % P2;
     kb = unit(n2 + P2 * l, D);
     kr = unit(P2 * L1, D);
@@ -870,7 +906,7 @@ __device__ __forceinline__ bool z_c2r(char* smem, int it, int n_items, const flo
   const float2* st = reinterpret_cast<const float2*>(smem + P::OFF_STAGE) + (size_t)(it % ZSTAGES) * P::STAGE;
   float2* buf = reinterpret_cast<float2*>(smem + P::OFF_BUF) + (size_t)(it & 1) * P::BUF;
   float2* xs = reinterpret_cast<float2*>(smem + P::OFF_XS) + (threadIdx.x / 32) * P::XS_WARP;
-  const bool arrived = mbar_wait(&bars[it % ZSTAGES], (unsigned)(it / ZSTAGES) & 1u);
+  const bool arrived = mbar_wait(&bars[it % ZSTAGES], (unsigned)(it / ZSTAGES) & 1u, w.full);
   {
     // step A: row t, column n2, lane-part l of the P1-point DFT over n1
     const int l = threadIdx.x % L1, n2 = (threadIdx.x / L1) % P2, t = threadIdx.x / (L1 * P2);
@@ -924,10 +960,10 @@ __device__ __forceinline__ bool z_c2r(char* smem, int it, int n_items, const flo
 // arrive.
 template <int D>
 __device__ __forceinline__ bool z_skip(char* smem, int it, int n_items, const float2* spectra, long long C,
-                                       long long row0, int G)
+                                       long long row0, int G, bool full)
 {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-  const bool arrived = mbar_wait(&bars[it % ZSTAGES], (unsigned)(it / ZSTAGES) & 1u);
+  const bool arrived = mbar_wait(&bars[it % ZSTAGES], (unsigned)(it / ZSTAGES) & 1u, full);
   if (__syncthreads_or(!arrived))
     return false;
   if (threadIdx.x == 0 && it + ZSTAGES < n_items)
@@ -1132,7 +1168,7 @@ __global__ void __launch_bounds__(FFT_THREADS, MINB) k_fft_z_threshold(ZThreshol
       // field 2 of this radius: transformed if a cell of the block needs it
       const bool any = __syncthreads_or((first_ion | first_z) != 0);
       const bool ok = any ? z_c2r<D, true>(smem, it, n_items, a.spectra, a.C, row0, w, f[2], G)
-                          : z_skip<D>(smem, it, n_items, a.spectra, a.C, row0, G);
+                          : z_skip<D>(smem, it, n_items, a.spectra, a.C, row0, G, w.full);
       if (!ok) {
         z_abort<D>(smem, it, n_items, a.err);
         return;
@@ -1418,75 +1454,174 @@ __device__ __forceinline__ bool zg_test(float dx, float stv, float nr, float xe,
   return threshold_fp64(dx, stv, nr, xe, RECOMB, SPIN, rp.M_mean, rp.R_cubed, pixel_volume, eff, xpart);
 }
 
-// z-pass fused with the per-cell test for grids with a factor 3: every field
-// of a radius is transformed into shared memory, then each thread tests its
-// cells (cell c = threadIdx.x + j * TILE_THREADS_3 of the block's 16 rows).
-// Same state, bookkeeping and stores as k_fft_z_threshold.
-template <int D, bool SPIN, bool RECOMB>
-__global__ void __launch_bounds__(TILE_THREADS_3) k_fft_z_threshold_gen(const __grid_constant__ ZThresholdArgs a)
+// z-pass fused with the per-cell test for grids with a factor 3.  A block owns
+// 16 rows and ZTGen<D>::T threads, as many as the tile engine's steps keep busy.
+// The rows of each (radius, field) spectrum arrive through a ring of ZT_STAGES
+// stages filled by 16-byte asynchronous copies (cp.async; the bulk copies of
+// k_fft_z_threshold would need one per row, whose fixed cost bounds the ring),
+// the transform's outputs stay in registers (a thread gets the same points of
+// every field, so the fields of a cell meet there), and weighted_sfr is
+// transformed only for a block with a first crossing, as in k_fft_z_threshold.
+// Same tests, bookkeeping and stores.
+//
+// Bound by latency between the three barriers of a transform: 4.1 ms for the 41
+// radii of 5 fields at 192^3, 0.55 ms at 96^3, registers for two blocks per SM
+// (three, with spills, took 0.77 ms at 96^3; a ring of per-row bulk copies 4.8
+// and 0.75 ms).  A block of 384 threads (half of them idle in step A) that read
+// each spectrum's rows after the last one's transform and kept every field's
+// real rows in shared memory (90 KB per block) took 12.7 and 1.93 ms.
+constexpr int ZT_STAGES = 3;
+template <int D>
+struct ZTGen
 {
-  using P = ZGPlan<D>;
+  static constexpr int L = D / 2, H = D / 2 + 1, HP = Pitch<D>::HP;
+  static constexpr int T = 192;               // threads: 12 slots of 16 rows
+  static constexpr int RP = H + 1;            // float2 row pitch of a stage: 16-byte rows
+  static constexpr int STAGE = ZG_ROWS * RP;  // float2
+  static constexpr int CHUNKS = RP / 2;       // 16-byte copies per row
+  static constexpr int OFF_TW = 0, OFF_POST = OFF_TW + L, OFF_TILE = OFF_POST + L;
+  static constexpr int OFF_STAGE = (OFF_TILE + L * TXC + 15) / 16 * 16;
+  static constexpr size_t BYTES = sizeof(float2) * (size_t)(OFF_STAGE + ZT_STAGES * STAGE);
+  static_assert((RP * sizeof(float2)) % 16 == 0 && (OFF_STAGE * sizeof(float2)) % 16 == 0, "copy alignment");
+};
+
+template <int D, bool SPIN, bool RECOMB>
+__global__ void __launch_bounds__(ZTGen<D>::T, 2)
+  k_fft_z_threshold_gen(const __grid_constant__ ZThresholdArgs a)
+{
+  using P = ZTGen<D>;
+  using TS = TileSteps<P::L, P::T>;
+  constexpr int L = P::L, H = P::H, HP = P::HP, RP = P::RP, NOUT = TS::NOUT;
   constexpr int G = 3 + (SPIN ? 1 : 0) + (RECOMB ? 1 : 0);
   constexpr int IXE = 3, INR = SPIN ? 4 : 3;
-  constexpr int CELLS = ZG_ROWS * D, CPT = (CELLS + TILE_THREADS_3 - 1) / TILE_THREADS_3;
-  extern __shared__ __align__(16) unsigned char zgsm[];
+  extern __shared__ __align__(128) unsigned char zgsm[];
   float2* s2 = reinterpret_cast<float2*>(zgsm);
-  float* real = reinterpret_cast<float*>(zgsm + sizeof(float2) * P::END2);
-  zg_tables<D>(s2);
+  const float2 *tw = s2 + P::OFF_TW, *post = s2 + P::OFF_POST;
+  float2* tile = s2 + P::OFF_TILE;
   const long long row0 = ((long long)blockIdx.x + a.group0) * ZG_ROWS;
-  unsigned st[CPT];
+  const int n_items = a.n_f * G;
+  // the 16 rows of item `it` into stage it % ZT_STAGES; one group of copies
+  // per item, also past the last one
+  auto issue = [&](int it) {
+    if (it < n_items) {
+      const float2* src = a.spectra + (long long)z_item_spectrum(it, G) * a.C + row0 * HP;
+      float2* dst = s2 + P::OFF_STAGE + (it % ZT_STAGES) * P::STAGE;
 #pragma unroll
-  for (int j = 0; j < CPT; j++) {
-    const int c = threadIdx.x + j * TILE_THREADS_3;
-    st[j] = 0;
-    if (c < CELLS) {
-      const long long ir = row0 * D + c;
-      const float x0 = a.xH[ir], z0 = a.z_at_ion[ir];
-      st[j] = (x0 > REL_TOL_F ? ST_XHIGH : 0u) | (x0 < REL_TOL_F ? ST_XLOW : 0u) | (z0 < 0 ? ST_ZUNSET : 0u);
+      for (int c = threadIdx.x; c < ZG_ROWS * P::CHUNKS; c += P::T) {
+        const int row = c / P::CHUNKS, col = 2 * (c - row * P::CHUNKS);
+        copy16_async(dst + row * RP + col, src + row * HP + col);
+      }
+    }
+    copy_async_commit();
+  };
+  fill_twiddles<L>(s2 + P::OFF_TW, threadIdx.x, P::T);
+  for (int k = threadIdx.x; k < L; k += P::T) {
+    float sn, cs;
+    sincospif(2.0f * (float)k / (float)D, &sn, &cs);
+    s2[P::OFF_POST + k] = make_float2(cs, sn);
+  }
+  for (int it = 0; it < ZT_STAGES; it++)
+    issue(it);
+  // C2R of item `it`: out[i] = (x[2m], x[2m + 1]) of row tid % 16, m =
+  // out_point(i).  Without `use` the item is only consumed.
+  auto c2r = [&](int it, float2 (&out)[NOUT], bool use) {
+    copy_async_wait<ZT_STAGES - 1>();
+    // everyone's copies have landed, and everyone has read the last item's tile
+    __syncthreads();
+    if (use) {
+      const float2* rows = s2 + P::OFF_STAGE + (it % ZT_STAGES) * P::STAGE;
+      TS::a(tile, tw, [&](int k, int t, int) {
+        float2 A = rows[t * RP + k];
+        float2 B = rows[t * RP + (L - k)];
+        if (k == 0) {
+          A.y = 0.0f;
+          B.y = 0.0f;
+        }
+        B.y = -B.y;
+        const float2 E = cadd(A, B);
+        const float2 O = cmul(csub(A, B), post[k]);
+        return make_float2(E.x - O.y, E.y + O.x);
+      });
+      __syncthreads();
+      issue(it + ZT_STAGES);
+      TS::b(tile, tw);
+      __syncthreads();
+      TS::c_regs(tile, out);
+    } else {
+      issue(it + ZT_STAGES);
+    }
+  };
+  // this thread's cells: row t, z = 2 m + {0, 1}; the state of a pair in the
+  // halves of a register (ST_* bits, radius index from bit ST_RB_SHIFT on)
+  const int t = threadIdx.x % TXC;
+  const long long cell0 = (row0 + t) * D;
+  unsigned st[NOUT];
+#pragma unroll
+  for (int i = 0; i < NOUT; i++) {
+    const int m = TS::out_point(i);
+    st[i] = 0;
+    if (m >= 0) {
+      const float2 x0 = *reinterpret_cast<const float2*>(a.xH + cell0 + 2 * m);
+      const float2 z0 = *reinterpret_cast<const float2*>(a.z_at_ion + cell0 + 2 * m);
+      st[i] = ((x0.x > REL_TOL_F ? ST_XHIGH : 0u) | (x0.x < REL_TOL_F ? ST_XLOW : 0u) | (z0.x < 0 ? ST_ZUNSET : 0u)) |
+              ((x0.y > REL_TOL_F ? ST_XHIGH : 0u) | (x0.y < REL_TOL_F ? ST_XLOW : 0u) | (z0.y < 0 ? ST_ZUNSET : 0u)) << 16;
     }
   }
+  const bool need_ws = a.uvb || RECOMB;
+  int it = 0;
   for (int r = 0; r < a.n_r; r++) {
     const RadiusParams rp = a.rp[r];
     const bool direct = rp.last != 0;
+    float2 f[G][NOUT];
     if (!direct) {
+#pragma unroll
+      for (int j = 0; j < G - 1; j++)
+        c2r(it++, f[j < 2 ? j : j + 1], true);
+    } else {
+#pragma unroll
       for (int g = 0; g < G; g++)
-        zg_c2r<D>(a.spectra + (long long)(r * G + g) * a.C, row0, s2, real + g * P::REAL);
+#pragma unroll
+        for (int i = 0; i < NOUT; i++) {
+          const int m = TS::out_point(i);
+          if (m >= 0)
+            f[g][i] = *reinterpret_cast<const float2*>(a.direct[g] + (row0 + t) * 2LL * H + 2 * m);
+        }
     }
+    // bit c of first_ion / first_z: cell c's J_21 and Gamma12 resp.
+    // J_21_at_ionization are written below
+    unsigned first_ion = 0, first_z = 0;
 #pragma unroll
-    for (int j = 0; j < CPT; j++) {
-      const int c = threadIdx.x + j * TILE_THREADS_3;
-      if (c >= CELLS)
+    for (int c = 0; c < 2 * NOUT; c++) {
+      const int i = c >> 1, half = (c & 1) * 16;
+      const int m = TS::out_point(i);
+      if (m < 0)
         continue;
-      const int t = c / D, z = c - t * D;
-      const long long ir = row0 * D + c;
-      float f[G];
-#pragma unroll
-      for (int g = 0; g < G; g++)
-        f[g] = direct ? a.direct[g][(row0 + t) * 2LL * P::H + z] : real[g * P::REAL + t * P::RD + z];
-      const float dx = fmaxf(f[0], -1 + REL_TOL_F);
-      float stv = fmaxf(f[1], 0.0f);
+      const bool hi = c & 1;
+      const float dx = fmaxf(hi ? f[0][i].y : f[0][i].x, -1 + REL_TOL_F);
+      float stv = fmaxf(hi ? f[1][i].y : f[1][i].x, 0.0f);
       if (stv < ABS_TOL_F)
         stv = 0;
       float nr = 0.0f, xe = 0.0f;
       if constexpr (RECOMB) {
-        nr = fmaxf(f[INR], 0.0f);
+        nr = fmaxf(hi ? f[INR][i].y : f[INR][i].x, 0.0f);
         if (nr < ABS_TOL_F)
           nr = 0;
       }
       if constexpr (SPIN) {
-        xe = fmaxf(f[IXE], 0.0f);
+        xe = fmaxf(hi ? f[IXE][i].y : f[IXE][i].x, 0.0f);
         if (xe < ABS_TOL_F)
           xe = 0;
         xe = fminf(xe, 0.999f);
       }
       float xpart;
       const bool ionised = zg_test<SPIN, RECOMB>(dx, stv, nr, xe, rp, a.pixel_volume, a.eff, &xpart);
-      unsigned s = st[j];
+      const long long ir = cell0 + 2 * m + (hi ? 1 : 0);
+      unsigned s = st[i] >> half & 0xffffu;
       const bool xr_high = !(s & ST_ION) && (s & ST_XHIGH);
       bool xr_low = (s & ST_ION) || (s & ST_XLOW);
-      bool first_ion = false, first_z = false;
       if (ionised) {
-        first_ion = xr_high;
+        if (xr_high)
+          first_ion |= 1u << c;
         s = (s & ((1u << ST_RB_SHIFT) - 1)) | ST_ION | ((unsigned)r << ST_RB_SHIFT);
         xr_low = true;
       } else if (rp.last && xr_high) {
@@ -1496,33 +1631,46 @@ __global__ void __launch_bounds__(TILE_THREADS_3) k_fft_z_threshold_gen(const __
       }
       if (xr_low && (s & ST_ZUNSET)) {
         a.z_at_ion[ir] = (float)a.redshift;
-        first_z = true;
+        first_z |= 1u << c;
         s &= ~ST_ZUNSET;
       }
-      st[j] = s;
-      if ((a.uvb || RECOMB) && (first_ion || (a.uvb && first_z))) {
-        float ws = fmaxf(f[2], 0.0f);
-        if (ws < ABS_TOL_F)
-          ws = 0;
-        const float J21_aux = a.uvb ? ws * rp.kj : 0.0f;
-        if (first_ion) {
-          if (a.uvb)
-            a.J21[ir] = J21_aux;
-          if (RECOMB)
-            a.Gamma12[ir] = ws * rp.kg;
-        }
-        if (a.uvb && first_z)
-          a.J21_at_ion[ir] = J21_aux * a.gamma_halo_bias;
+      st[i] = (st[i] & ~(0xffffu << half)) | s << half;
+    }
+    if (!need_ws)
+      first_ion = first_z = 0;
+    if (!a.uvb)
+      first_z = 0;
+    if (!direct) {
+      const bool any = __syncthreads_or((first_ion | first_z) != 0);
+      c2r(it++, f[2], any);
+    }
+#pragma unroll
+    for (int c = 0; c < 2 * NOUT; c++) {
+      if (!((first_ion | first_z) >> c & 1u))
+        continue;
+      const int i = c >> 1;
+      const long long ir = cell0 + 2 * TS::out_point(i) + (c & 1);
+      float ws = fmaxf((c & 1) ? f[2][i].y : f[2][i].x, 0.0f);
+      if (ws < ABS_TOL_F)
+        ws = 0;
+      const float J21_aux = a.uvb ? ws * rp.kj : 0.0f;
+      if (first_ion >> c & 1u) {
+        if (a.uvb)
+          a.J21[ir] = J21_aux;
+        if (RECOMB)
+          a.Gamma12[ir] = ws * rp.kg;
       }
+      if (first_z >> c & 1u)
+        a.J21_at_ion[ir] = J21_aux * a.gamma_halo_bias;
     }
   }
 #pragma unroll
-  for (int j = 0; j < CPT; j++) {
-    const int c = threadIdx.x + j * TILE_THREADS_3;
-    if (c < CELLS && (st[j] & ST_ION)) {
-      const long long ir = row0 * D + c;
+  for (int c = 0; c < 2 * NOUT; c++) {
+    const unsigned s = st[c >> 1] >> (c & 1) * 16 & 0xffffu;
+    if (s & ST_ION) {
+      const long long ir = cell0 + 2 * TS::out_point(c >> 1) + (c & 1);
       a.xH[ir] = 0.0f;
-      a.r_bubble[ir] = (float)a.rp[st[j] >> ST_RB_SHIFT].R;
+      a.r_bubble[ir] = (float)a.rp[s >> ST_RB_SHIFT].R;
     }
   }
 }
@@ -1787,11 +1935,11 @@ int fft_z_row_groups(int D) { return D * D / fft_z_rows_per_group(D); }
 template <int D, bool SPIN, bool RECOMB>
 static void launch_ztg_cfg(const ZThresholdArgs& a, cudaStream_t s)
 {
-  const size_t bytes = ZGPlan<D>::bytes(3 + (SPIN ? 1 : 0) + (RECOMB ? 1 : 0));
+  const size_t bytes = ZTGen<D>::BYTES;
   cudaFuncSetAttribute(k_fft_z_threshold_gen<D, SPIN, RECOMB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)bytes);
   const int groups = a.n_groups > 0 ? a.n_groups : D * D / ZG_ROWS;
-  k_fft_z_threshold_gen<D, SPIN, RECOMB><<<groups, TILE_THREADS_3, bytes, s>>>(a);
+  k_fft_z_threshold_gen<D, SPIN, RECOMB><<<groups, ZTGen<D>::T, bytes, s>>>(a);
 }
 template <int D>
 static void launch_ztg(const ZThresholdArgs& a, cudaStream_t s)

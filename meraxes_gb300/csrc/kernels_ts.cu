@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
   const long long ntiles = (N + EV_TILE - 1) / EV_TILE;
   const int my_tiles = blockIdx.x < ntiles ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
   const bool light = !c.no_light;
+  const bool full = bulk::full_waits();
   if (threadIdx.x == 0 && light) {
     for (int b = 0; b < STAGES; b++)
       bulk::mbar_init(&bars[b], 1);
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
     const float w = __fdividef(xcall - c.xhii[lo], c.xhii[hi] - c.xhii[lo]);
     float heat = 0.f, ion = 0.f, lya = 0.f, star = 0.f;
     if (light) {
-      const bool arrived = bulk::mbar_wait(&bars[k % STAGES], (unsigned)(k / STAGES) & 1u);
+      const bool arrived = bulk::mbar_wait(&bars[k % STAGES], (unsigned)(k / STAGES) & 1u, full);
       if (__syncthreads_or(!arrived)) {
         if (threadIdx.x == 0) {
           atomicOr(a.err, bulk::ERR_PIPELINE_TIMEOUT);
@@ -612,6 +613,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_evolve_adjoint(AdjointArgs a, i
   const long long ntiles = (N + EV_TILE - 1) / EV_TILE;
   const int my_tiles = blockIdx.x < ntiles ? (int)((ntiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
   const bool light = !c.no_light;
+  const bool full = bulk::full_waits();
   if (threadIdx.x == 0 && light) {
     bulk::mbar_init(&bars[0], 1);
     bulk::mbar_init(&bars[1], 1);
@@ -667,7 +669,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_evolve_adjoint(AdjointArgs a, i
     float heat = 0.f, ion = 0.f, lya = 0.f, star = 0.f, dheat = 0.f, dion = 0.f, dlya = 0.f;
     const float* st = nullptr;
     if (light) {
-      const bool arrived = bulk::mbar_wait(&bars[k & 1], (unsigned)(k >> 1) & 1u);
+      const bool arrived = bulk::mbar_wait(&bars[k & 1], (unsigned)(k >> 1) & 1u, full);
       if (__syncthreads_or(!arrived)) {
         if (threadIdx.x == 0) {
           atomicOr(a.err, bulk::ERR_PIPELINE_TIMEOUT);
