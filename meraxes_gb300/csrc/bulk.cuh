@@ -135,8 +135,10 @@ __device__ __forceinline__ bool mbar_test_now(uint64_t* bar, unsigned parity)
 __device__ __forceinline__ bool mbar_wait_polls(uint64_t* bar, unsigned parity, long long polls)
 {
   if (polls < WAIT_LIMIT_ITERS) {
-    // a lowered limit (a test of the give-up path): polls that do not wait
-    for (long long it = 0; it < polls; it++)
+    // a lowered limit (a test of the give-up path): polls that do not wait; the
+    // last one gives up whether the copy has landed by then or not, so that a
+    // limit of 1 does not depend on timing
+    for (long long it = 1; it < polls; it++)
       if (mbar_test_now(bar, parity))
         return true;
     return false;

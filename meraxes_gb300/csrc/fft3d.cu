@@ -538,6 +538,20 @@ __device__ __forceinline__ void tile_dft(float2* buf, const float2* tw, Load loa
   T::c(buf, store);
 }
 
+// The radius of item i in the prefix sums start[0 ... n].
+__device__ __forceinline__ int band_radius(const unsigned* start, int n, unsigned i)
+{
+  int lo = 0, hi = n;
+  while (hi > lo + 1) {
+    const int mid = (lo + hi) >> 1;
+    if (start[mid] <= i)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
 // ------------------------------------------------------------------ x-pass
 // Grid: one block per (|ky| <= D/2, tile of TXC kz columns, radius), the
 // radius fastest, so that the blocks of all radii of a tile run together and
@@ -548,6 +562,12 @@ __device__ __forceinline__ void tile_dft(float2* buf, const float2* tw, Load loa
 // HP, the forward transform's layout; columns past H are not read), scales by 1/N, multiplies by W(|k| R), inverse-DFTs along x and stores
 // to out[(r*G + g) * C + (x*D + ky)*HP + kz], all HP columns (those past H
 // are zero in, zero out).
+//
+// Band-limited batches (the default k-space top-hat of the ComputeTs shells)
+// leave out the tiles that hold only zeros: the 40 shells' radii grow by a fifth
+// each from one cell up, so that all but the first few keep a small corner of
+// the spectrum (x- and y-pass of the 40 shells at 512^3: 15 -> 3 ms; ComputeTs at
+// 256^3 6.2 -> 4.5 ms).
 //
 // Per-radius weight tables built once per context (read instead of the
 // sincosf) measured slower: the table read before the block's barrier is a
@@ -566,7 +586,9 @@ constexpr int x_min_blocks()
 {
   return XTHREADS == 128 ? 4 : (XTHREADS == 256 && D < 512 ? 3 : 2);
 }
-template <int D, int XTHREADS>
+// BANDED: only the tiles with a mode inside the radius's band (Bands), radius
+// by radius; their lines outside it are not read.
+template <int D, int XTHREADS, bool BANDED>
 __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_blocks<D, XTHREADS>())
   k_fft_x_filter(const __grid_constant__ XPassArgs a)
 {
@@ -578,13 +600,33 @@ __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_bloc
   float2* buf = tw + D;
   float* wsm = reinterpret_cast<float*>(buf + P::BUF);
   const unsigned item = blockIdx.x * tile_groups<XTHREADS>() + tile_group<XTHREADS>();
-  if (item >= (unsigned)(H * P::NT) * a.n)
-    return;
+  int r, kyp, kz0;  // |ky|: the block transforms rows ky = kyp and D - kyp
+  int pitch = Pitch<D>::HP;
+  float kx2_max = 0.0f;
+  if constexpr (BANDED) {
+    if (item >= a.bands.xstart[a.n])
+      return;
+    r = band_radius(a.bands.xstart, a.n, item);
+    const unsigned local = item - a.bands.xstart[r];
+    const int nt = a.bands.nt[r];
+    kyp = local / nt;
+    kz0 = (local % nt) * TXC;
+    // the same test as the y-pass's, which reads what is written here
+    const float m2 = a.bands.m2[r];
+    if ((float)(kyp * kyp + kz0 * kz0) > m2)
+      return;
+    kx2_max = m2 - (float)(kyp * kyp + kz0 * kz0);
+    if (a.bands.compact)
+      pitch = nt * TXC;
+  } else {
+    if (item >= (unsigned)(H * P::NT) * a.n)
+      return;
+    r = item % a.n;
+    const int tile = item / a.n;
+    kyp = tile / P::NT;
+    kz0 = (tile % P::NT) * TXC;
+  }
   fill_twiddles<D>(tw, tid, XTHREADS);
-  const int r = item % a.n;
-  const int tile = item / a.n;
-  const int kyp = tile / P::NT;  // |ky|: the block transforms rows ky = kyp and D - kyp
-  const int kz0 = (tile % P::NT) * TXC;
   // the weights depend on ky only through kyv^2, the same for both rows
   const float kyv = kcomp(kyp, D, a.delta_k);
   // this thread's column: kz = kz0 + t, the same in every step
@@ -596,7 +638,12 @@ __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_bloc
   auto read_points = [&](int ky, int g) {
     const float2* __restrict__ src = a.in[g] + (long long)ky * Pitch<D>::HP + kz0 + t0;
     T::for_each_input([&](int kx, int i) {
-      pts[i] = live ? src[(long long)kx * (D * Pitch<D>::HP)] : make_float2(0.f, 0.f);
+      bool read = live;
+      if constexpr (BANDED) {
+        const int ka = kx <= D / 2 ? kx : D - kx;
+        read = read && (float)(ka * ka) <= kx2_max;
+      }
+      pts[i] = read ? src[(long long)kx * (D * Pitch<D>::HP)] : make_float2(0.f, 0.f);
     });
   };
   // filter weights of the tile, wsm[|kx| * TXC + t] for |kx| = min(kx, D -
@@ -621,8 +668,11 @@ __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_bloc
       T::b(buf, tw);
       tile_sync<XTHREADS>();
       float2* __restrict__ dst =
-        a.out + (long long)(r * a.G + g) * a.C + (long long)ky * Pitch<D>::HP + kz0 + t0;
-      T::c(buf, [&](int x, int, float2 v) { dst[(long long)x * (D * Pitch<D>::HP)] = v; });
+        a.out + (long long)(r * a.G + g) * a.C + (long long)ky * pitch + kz0 + t0;
+      if constexpr (BANDED)
+        T::c(buf, [&](int x, int, float2 v) { dst[(long long)x * D * pitch] = v; });
+      else
+        T::c(buf, [&](int x, int, float2 v) { dst[(long long)x * (D * Pitch<D>::HP)] = v; });
       tile_sync<XTHREADS>();
     };
     auto step_a = [&]() {
@@ -646,33 +696,77 @@ __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_bloc
 
 // ------------------------------------------------------------------ y-pass
 // Grid: (spectrum, x, tile of TXC kz columns).  In-place inverse DFT along y
-// over all HP columns of the pitch.
-template <int D, int YTHREADS>
-__global__ void __launch_bounds__(YTHREADS, YTHREADS == 256 ? 3 : 2) k_fft_y(float2* data, long long C, int n_spectra)
+// over all HP columns of the pitch; BANDED: over the tiles inside the radius's
+// band, reading only the lines inside it (the x-pass wrote no others).
+struct YPassArgs
+{
+  float2* data;
+  long long C;
+  int n_spectra;
+  Bands bands;
+};
+template <int D, int YTHREADS, bool BANDED>
+__global__ void __launch_bounds__(YTHREADS, YTHREADS == 256 ? 3 : 2) k_fft_y(const __grid_constant__ YPassArgs a)
 {
   using P = TilePlan<D>;
   constexpr int HP = Pitch<D>::HP;
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* buf = smem + D;
-  const long long blk = blockIdx.x;
-  const int tile = (int)(blk % P::NT);
-  const int x = (int)((blk / P::NT) % D);
-  const long long s = blk / ((long long)P::NT * D);
-  const int kz0 = tile * TXC;
-  float2* col = data + s * C + (long long)x * D * HP + kz0 + threadIdx.x % TXC;
-  // the points of step A are read first, so that the reads are in flight
-  // while the twiddle table is filled
   using T = TileSteps<D, YTHREADS>;
   float2 pts[T::NPTS];
-  T::for_each_input([&](int ky, int i) { pts[i] = col[ky * HP]; });
+  int pitch = HP;
+  float2* col;
+  if constexpr (BANDED) {
+    const int G = a.n_spectra / a.bands.n;
+    int r, g, x, tile;
+    if (a.bands.compact) {
+      r = band_radius(a.bands.ystart, a.bands.n, blockIdx.x);
+      const unsigned local = blockIdx.x - a.bands.ystart[r];
+      const int nt = a.bands.nt[r];
+      tile = local % nt;
+      x = local / nt % D;
+      g = local / nt / D;
+      pitch = nt * TXC;
+    } else {
+      tile = blockIdx.x % P::NT;
+      x = blockIdx.x / P::NT % D;
+      const int sp = blockIdx.x / P::NT / D;
+      r = sp / G;
+      g = sp - r * G;
+    }
+    const int kz0 = tile * TXC;
+    col = a.data + (long long)(r * G + g) * a.C + (long long)x * D * pitch + kz0 + threadIdx.x % TXC;
+    const float m2 = a.bands.m2[r];
+    if ((float)(kz0 * kz0) > m2) {
+      for (int y = threadIdx.x / TXC; y < D; y += YTHREADS / TXC)
+        col[y * pitch] = make_float2(0.f, 0.f);
+      return;
+    }
+    T::for_each_input([&](int ky, int i) {
+      const int ka = ky <= D / 2 ? ky : D - ky;
+      pts[i] = (float)(ka * ka + kz0 * kz0) <= m2 ? col[ky * pitch] : make_float2(0.f, 0.f);
+    });
+  } else {
+    const long long blk = blockIdx.x;
+    const int tile = (int)(blk % P::NT);
+    const int x = (int)((blk / P::NT) % D);
+    const long long s = blk / ((long long)P::NT * D);
+    col = a.data + s * a.C + (long long)x * D * HP + tile * TXC + threadIdx.x % TXC;
+    // the points of step A are read first, so that the reads are in flight
+    // while the twiddle table is filled
+    T::for_each_input([&](int ky, int i) { pts[i] = col[ky * HP]; });
+  }
   fill_twiddles<D>(tw, threadIdx.x, YTHREADS);
   __syncthreads();
   T::a(buf, tw, [&](int, int, int i) { return pts[i]; });
   __syncthreads();
   T::b(buf, tw);
   __syncthreads();
-  T::c(buf, [&](int y, int, float2 v) { col[y * HP] = v; });
+  if constexpr (BANDED)
+    T::c(buf, [&](int y, int, float2 v) { col[y * pitch] = v; });
+  else
+    T::c(buf, [&](int y, int, float2 v) { col[y * HP] = v; });
 }
 
 // ------------------------------------------------------------------ z-pass
@@ -882,13 +976,13 @@ __device__ __forceinline__ int z_item_spectrum(int it, int G)
 // Producer side of the ring: thread 0 issues item `it` into stage it % ZSTAGES.
 template <int D>
 __device__ __forceinline__ void z_issue(char* smem, const float2* spectra, long long C, long long row0, int it,
-                                        int G = 1)
+                                        int G = 1, int pitch = ZPlan<D>::HP)
 {
   using P = ZPlan<D>;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   float2* st = reinterpret_cast<float2*>(smem + P::OFF_STAGE) + (size_t)(it % ZSTAGES) * P::STAGE;
-  bulk_load(st, spectra + (long long)z_item_spectrum(it, G) * C + row0 * P::HP, (unsigned)(sizeof(float2) * P::STAGE),
-            &bars[it % ZSTAGES]);
+  bulk_load(st, spectra + (long long)z_item_spectrum(it, G) * C + row0 * pitch,
+            (unsigned)(sizeof(float2) * P::TZ) * pitch, &bars[it % ZSTAGES]);
 }
 
 // C2R along z of the TZ staged rows of item `it`.  On return z[e] holds
@@ -896,9 +990,12 @@ __device__ __forceinline__ void z_issue(char* smem, const float2* spectra, long 
 // m = k1 + P1 * lane_out(L2, e, l), k1 = (threadIdx.x / L2) % P1,
 // l = threadIdx.x % L2.  Returns false (for every thread) if the copy did not
 // arrive.  One block barrier per call: the transpose buffer alternates.
-template <int D, bool XS>
+// BANDED: the rows hold their first nt[it] tiles of columns only, the others
+// are zero.
+template <int D, bool XS, bool BANDED = false>
 __device__ __forceinline__ bool z_c2r(char* smem, int it, int n_items, const float2* spectra, long long C,
-                                      long long row0, const ZTw<D>& w, float2 (&z)[4], int G = 1)
+                                      long long row0, const ZTw<D>& w, float2 (&z)[4], int G = 1,
+                                      const unsigned short* nt = nullptr)
 {
   using P = ZPlan<D>;
   constexpr int H = P::H, DH = P::DH, P1 = P::P1, P2 = P::P2, L1 = P::L1, L2 = P::L2;
@@ -910,14 +1007,21 @@ __device__ __forceinline__ bool z_c2r(char* smem, int it, int n_items, const flo
   {
     // step A: row t, column n2, lane-part l of the P1-point DFT over n1
     const int l = threadIdx.x % L1, n2 = (threadIdx.x / L1) % P2, t = threadIdx.x / (L1 * P2);
-    const float2* row = st + t * P::HP;
+    const int pitch = BANDED ? nt[it] * TXC : P::HP;
+    const float2* row = st + t * pitch;
     float2 v[4];
     float2 tk = w.kb;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const int k = n2 + P2 * (l + L1 * i);
-      float2 A = row[k];
-      float2 B = row[DH - k];
+      float2 A, B;
+      if constexpr (BANDED) {
+        A = k < pitch ? row[k] : make_float2(0.f, 0.f);
+        B = DH - k < pitch ? row[DH - k] : make_float2(0.f, 0.f);
+      } else {
+        A = row[k];
+        B = row[DH - k];
+      }
       if (i == 0 && k == 0) {
         A.y = 0.0f;  // imaginary parts of kz = 0 and kz = D/2 are ignored
         B.y = 0.0f;
@@ -942,7 +1046,7 @@ __device__ __forceinline__ bool z_c2r(char* smem, int it, int n_items, const flo
   if (__syncthreads_or(!arrived))
     return false;
   if (threadIdx.x == 0 && it + ZSTAGES < n_items)
-    z_issue<D>(smem, spectra, C, row0, it + ZSTAGES, G);
+    z_issue<D>(smem, spectra, C, row0, it + ZSTAGES, G, BANDED ? nt[it + ZSTAGES] * TXC : P::HP);
   {
     // step B: row t, k1, lane-part l of the P2-point DFT over n2
     const int l = threadIdx.x % L2, k1 = (threadIdx.x / L2) % P1, t = threadIdx.x / (L2 * P1);
@@ -974,7 +1078,7 @@ __device__ __forceinline__ bool z_skip(char* smem, int it, int n_items, const fl
 // Ring setup: barriers, the first ZSTAGES copies.
 template <int D>
 __device__ __forceinline__ void z_setup(char* smem, const float2* spectra, long long C, long long row0, int n_items,
-                                        int G = 1)
+                                        int G = 1, const unsigned short* nt = nullptr)
 {
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   if (threadIdx.x == 0) {
@@ -985,7 +1089,7 @@ __device__ __forceinline__ void z_setup(char* smem, const float2* spectra, long 
   __syncthreads();
   if (threadIdx.x == 0)
     for (int it = 0; it < ZSTAGES && it < n_items; it++)
-      z_issue<D>(smem, spectra, C, row0, it, G);
+      z_issue<D>(smem, spectra, C, row0, it, G, nt ? nt[it] * TXC : ZPlan<D>::HP);
 }
 
 // After a timed-out wait: record the error and wait (bounded) for the copies
@@ -1208,26 +1312,35 @@ __global__ void __launch_bounds__(FFT_THREADS, MINB) k_fft_z_threshold(ZThreshol
 
 // z-pass storing clamped real values (ComputeTs shells, ComputeTs.c:476-500):
 // shells[(r0 + r) * N + cell] = max(value, 0) for every spectrum of the batch.
-template <int D>
-__global__ void __launch_bounds__(FFT_THREADS, 2) k_fft_z_store(const float2* spectra, long long C, int n, int r0,
-                                                                   float* shells, long long N, unsigned* err)
+struct ZStoreArgs
+{
+  const float2* spectra;
+  long long C;
+  int n, r0;
+  float* shells;
+  long long N;
+  unsigned* err;
+  unsigned short nt[MAX_BANDED];  // tiles per row of each spectrum (BANDED)
+};
+template <int D, bool BANDED>
+__global__ void __launch_bounds__(FFT_THREADS, 2) k_fft_z_store(const __grid_constant__ ZStoreArgs a)
 {
   using P = ZPlan<D>;
   extern __shared__ __align__(128) unsigned char zsmem[];
   char* smem = reinterpret_cast<char*>(zsmem);
   const long long row0 = (long long)blockIdx.x * P::TZ;
-  z_setup<D>(smem, spectra, C, row0, n);
+  z_setup<D>(smem, a.spectra, a.C, row0, a.n, 1, BANDED ? a.nt : nullptr);
   ZTw<D> w;
   w.init();
   const int l = threadIdx.x % P::L2, k1 = (threadIdx.x / P::L2) % P::P1, t = threadIdx.x / (P::L2 * P::P1);
   const long long base = (row0 + t) * D;
-  for (int r = 0; r < n; r++) {
+  for (int r = 0; r < a.n; r++) {
     float2 z[4];
-    if (!z_c2r<D, false>(smem, r, n, spectra, C, row0, w, z)) {
-      z_abort<D>(smem, r, n, err);
+    if (!z_c2r<D, false, BANDED>(smem, r, a.n, a.spectra, a.C, row0, w, z, 1, a.nt)) {
+      z_abort<D>(smem, r, a.n, a.err);
       return;
     }
-    float* dst = shells + (long long)(r0 + r) * N + base;
+    float* dst = a.shells + (long long)(a.r0 + r) * a.N + base;
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       const int zc = 2 * (k1 + P::P1 * lane_out(P::L2, e, l));
@@ -1313,8 +1426,9 @@ __global__ void __launch_bounds__(T) k_fft_z_r2c(const __grid_constant__ FwdArgs
     [&](int k, int t, float2 v) { rows[t * H + k] = make_float2(v.x, -v.y); });
   __syncthreads();
   float2* __restrict__ dst = a.out + (long long)g * a.C + r0 * HP;
-  for (int i = threadIdx.x; i < FWD_ROWS * HP; i += T) {
-    const int t = i / HP, k = i - t * HP;
+  const int W = a.nt * TXC;  // columns that are read
+  for (int i = threadIdx.x; i < FWD_ROWS * W; i += T) {
+    const int t = i / W, k = i - t * W;
     float2 X = make_float2(0.f, 0.f);
     if (k < H) {
       const float2 zk = rows[t * H + (k < L ? k : 0)];
@@ -1324,15 +1438,15 @@ __global__ void __launch_bounds__(T) k_fft_z_r2c(const __grid_constant__ FwdArgs
       const float2 C = cmul(B, post[k]);                       // w_D^-k B
       X = make_float2(0.5f * (A.x + C.y), 0.5f * (A.y - C.x)); // (A - i C) / 2
     }
-    dst[i] = X;
+    dst[t * HP + k] = X;
   }
 }
 
-// Forward DFT along y (AXIS 1) or x (AXIS 0) of n spectra [D][D][HP], in
-// place, tiles of 16 kz columns; the inverse y-pass's engine with conjugated
-// input and output.
+// Forward DFT along y (AXIS 1) or x (AXIS 0) of spectra [D][D][HP], in place,
+// the first nt tiles of 16 kz columns of n_outer rows (all x, or the |ky| that
+// are read); the inverse y-pass's engine with conjugated input and output.
 template <int D, int T, int AXIS>
-__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_fwd_cols(float2* data, long long C, int n_spectra)
+__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_fwd_cols(float2* data, long long C, int nt, int n_outer)
 {
   using P = TilePlan<D>;
   constexpr int HP = Pitch<D>::HP;
@@ -1341,10 +1455,11 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_fwd_cols(float2* da
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* buf = smem + D;
-  const long long blk = blockIdx.x;
-  const int tile = (int)(blk % P::NT);
-  const int o = (int)((blk / P::NT) % D);
-  const long long s = blk / ((long long)P::NT * D);
+  const unsigned tile = blockIdx.x % nt, rest = blockIdx.x / nt;
+  int o = rest % n_outer;
+  const long long s = rest / n_outer;
+  if (AXIS == 0 && o > n_outer / 2)
+    o += D - n_outer;  // |ky| <= n_outer / 2
   float2* col = data + s * C + (long long)o * OUTER + tile * TXC + threadIdx.x % TXC;
   using TS = TileSteps<D, T>;
   float2 pts[TS::NPTS];
@@ -1401,25 +1516,26 @@ __device__ __forceinline__ void zg_tables(float2* s2)
 
 // C2R along z of the 16 rows starting at row0 of one spectrum into real
 // (16 rows of RD floats).  Starts and ends with a block barrier.
+// The rows hold their first `pitch` columns only, the others are zero.
 template <int D>
-__device__ void zg_c2r(const float2* __restrict__ spectrum, long long row0, float2* s2, float* real)
+__device__ void zg_c2r(const float2* __restrict__ spectrum, long long row0, float2* s2, float* real, int pitch)
 {
   using P = ZGPlan<D>;
-  constexpr int L = P::L, HP = P::HP, RP = P::RP, RD = P::RD;
+  constexpr int L = P::L, RP = P::RP, RD = P::RD;
   float2* rows = s2 + P::OFF_ROWS;
   const float2* post = s2 + P::OFF_POST;
-  const float2* __restrict__ src = spectrum + row0 * HP;
+  const float2* __restrict__ src = spectrum + row0 * pitch;
   __syncthreads();  // the previous consumer of rows / real is done
-  for (int i = threadIdx.x; i < ZG_ROWS * HP; i += TILE_THREADS_3) {
-    const int t = i / HP;
-    rows[t * RP + (i - t * HP)] = __ldg(src + i);
+  for (int i = threadIdx.x; i < ZG_ROWS * pitch; i += TILE_THREADS_3) {
+    const int t = i / pitch;
+    rows[t * RP + (i - t * pitch)] = __ldg(src + i);
   }
   __syncthreads();
   tile_dft<L, TILE_THREADS_3>(
     s2 + P::OFF_TILE, s2 + P::OFF_TW,
     [&](int k, int t, int) {
-      float2 A = rows[t * RP + k];
-      float2 B = rows[t * RP + (L - k)];
+      float2 A = k < pitch ? rows[t * RP + k] : make_float2(0.f, 0.f);
+      float2 B = L - k < pitch ? rows[t * RP + (L - k)] : make_float2(0.f, 0.f);
       if (k == 0) {
         A.y = 0.0f;
         B.y = 0.0f;
@@ -1678,8 +1794,7 @@ __global__ void __launch_bounds__(ZTGen<D>::T, 2)
 // Clamped store of ComputeTs shells for grids with a factor 3 (as
 // k_fft_z_store): shells[(r0 + r) * N + cell] = max(value, 0).
 template <int D>
-__global__ void __launch_bounds__(TILE_THREADS_3) k_fft_z_store_gen(const float2* spectra, long long C, int n, int r0,
-                                                                     float* shells, long long N)
+__global__ void __launch_bounds__(TILE_THREADS_3) k_fft_z_store_gen(const __grid_constant__ ZStoreArgs a)
 {
   using P = ZGPlan<D>;
   constexpr int CELLS = ZG_ROWS * D;
@@ -1688,9 +1803,9 @@ __global__ void __launch_bounds__(TILE_THREADS_3) k_fft_z_store_gen(const float2
   float* real = reinterpret_cast<float*>(zgsm + sizeof(float2) * P::END2);
   zg_tables<D>(s2);
   const long long row0 = (long long)blockIdx.x * ZG_ROWS;
-  for (int r = 0; r < n; r++) {
-    zg_c2r<D>(spectra + (long long)r * C, row0, s2, real);
-    float* dst = shells + (long long)(r0 + r) * N + row0 * D;
+  for (int r = 0; r < a.n; r++) {
+    zg_c2r<D>(a.spectra + (long long)r * a.C, row0, s2, real, a.nt[r] * TXC);
+    float* dst = a.shells + (long long)(a.r0 + r) * a.N + row0 * D;
     for (int c = threadIdx.x; c < CELLS; c += TILE_THREADS_3) {
       const int t = c / D;
       dst[c] = fmaxf(real[t * P::RD + (c - t * D)], 0.0f);
@@ -1749,14 +1864,19 @@ constexpr size_t smem_x()
 {
   return sizeof(float2) * (size_t)XSmem<D>::FLOAT2 * tile_groups<T>();
 }
+template <int D, int T, bool BANDED>
+static void launch_x_b(const XPassArgs& a, cudaStream_t s)
+{
+  const size_t bytes = smem_x<D, T>();
+  cudaFuncSetAttribute(k_fft_x_filter<D, T, BANDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const long long tiles = BANDED ? (long long)a.bands.xstart[a.n] : (long long)(D / 2 + 1) * TilePlan<D>::NT * a.n;
+  const long long blocks = (tiles + tile_groups<T>() - 1) / tile_groups<T>();
+  k_fft_x_filter<D, T, BANDED><<<(unsigned)blocks, T * tile_groups<T>(), bytes, s>>>(a);
+}
 template <int D, int T>
 static void launch_x_t(const XPassArgs& a, cudaStream_t s)
 {
-  const size_t bytes = smem_x<D, T>();
-  cudaFuncSetAttribute(k_fft_x_filter<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  const long long tiles = (long long)(D / 2 + 1) * TilePlan<D>::NT * a.n;
-  const long long blocks = (tiles + tile_groups<T>() - 1) / tile_groups<T>();
-  k_fft_x_filter<D, T><<<(unsigned)blocks, T * tile_groups<T>(), bytes, s>>>(a);
+  a.bands.n ? launch_x_b<D, T, true>(a, s) : launch_x_b<D, T, false>(a, s);
 }
 template <int D>
 static void launch_x(const XPassArgs& a, int threads, cudaStream_t s)
@@ -1769,20 +1889,26 @@ static void launch_x(const XPassArgs& a, int threads, cudaStream_t s)
   else
     launch_x_t<D, 512>(a, s);
 }
-template <int D, int T>
-static void launch_y_t(float2* data, long long C, int n_spectra, cudaStream_t s)
+template <int D, int T, bool BANDED>
+static void launch_y_b(const YPassArgs& a, cudaStream_t s)
 {
-  const long long blocks = (long long)n_spectra * D * TilePlan<D>::NT;
-  cudaFuncSetAttribute(k_fft_y<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_y<D>());
-  k_fft_y<D, T><<<(unsigned)blocks, T, smem_y<D>(), s>>>(data, C, n_spectra);
+  const long long blocks = BANDED && a.bands.compact ? (long long)a.bands.ystart[a.bands.n]
+                                                     : (long long)a.n_spectra * D * TilePlan<D>::NT;
+  cudaFuncSetAttribute(k_fft_y<D, T, BANDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_y<D>());
+  k_fft_y<D, T, BANDED><<<(unsigned)blocks, T, smem_y<D>(), s>>>(a);
+}
+template <int D, int T>
+static void launch_y_t(const YPassArgs& a, cudaStream_t s)
+{
+  a.bands.n ? launch_y_b<D, T, true>(a, s) : launch_y_b<D, T, false>(a, s);
 }
 template <int D>
-static void launch_y(float2* data, long long C, int n_spectra, int threads, cudaStream_t s)
+static void launch_y(const YPassArgs& a, int threads, cudaStream_t s)
 {
   if (threads == 512)
-    launch_y_t<D, 512>(data, C, n_spectra, s);
+    launch_y_t<D, 512>(a, s);
   else
-    launch_y_t<D, 256>(data, C, n_spectra, s);
+    launch_y_t<D, 256>(a, s);
 }
 template <int D, bool SPIN, bool RECOMB, int MINB>
 static void launch_zt_minb(const ZThresholdArgs& a, cudaStream_t s)
@@ -1810,12 +1936,12 @@ static void launch_zt(const ZThresholdArgs& a, cudaStream_t s)
     a.recomb ? launch_zt_cfg<D, false, true>(a, s) : launch_zt_cfg<D, false, false>(a, s);
 }
 template <int D>
-static void launch_zs(const float2* spectra, long long C, int n, int r0, float* shells, long long N, unsigned* err,
-                      cudaStream_t s)
+static void launch_zs(const ZStoreArgs& a, bool banded, cudaStream_t s)
 {
   const size_t bytes = ZPlan<D>::BYTES_NO_XS;
-  cudaFuncSetAttribute(k_fft_z_store<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  k_fft_z_store<D><<<D * D / ZPlan<D>::TZ, FFT_THREADS, bytes, s>>>(spectra, C, n, r0, shells, N, err);
+  auto kernel = banded ? k_fft_z_store<D, true> : k_fft_z_store<D, false>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  kernel<<<D * D / ZPlan<D>::TZ, FFT_THREADS, bytes, s>>>(a);
 }
 
 // Largest float kR with (float)((double)kR * 0.413566994) <= 1, the last mode
@@ -1829,6 +1955,42 @@ static float sharpk_threshold()
   while ((float)((double)std::nextafter(x, INFINITY) * c) <= 1.0f)
     x = std::nextafter(x, INFINITY);
   return x;
+}
+
+Bands filter_bands(int D, int filter_type, const float* R, int n, int G, float delta_k, bool compact)
+{
+  static const float kmax = sharpk_threshold();
+  Bands b;
+  // the Gaussian exp(-(0.643 kR)^2 / 2) is below the smallest float from kR =
+  // 22.5 on
+  const double cut = filter_type == 1 ? (double)kmax : 23.0;
+  if (filter_type == 0 || n > MAX_BANDED || n < 1)
+    return b;
+  const int NT = fft_pitch(D) / TXC;
+  bool less = false;
+  unsigned x = 0, y = 0;
+  for (int r = 0; r < n; r++) {
+    // the filter takes |k| R in float: a margin of 1e-5 covers its roundings
+    const double m = cut / ((double)R[r] * (double)delta_k) * (1.0 + 1e-5);
+    b.m2[r] = (float)std::min(m * m, 1e9);
+    int nt = 1, ny = 0;
+    while (nt < NT && (float)(nt * TXC * nt * TXC) <= b.m2[r])
+      nt++;
+    while (ny < D / 2 && (float)((ny + 1) * (ny + 1)) <= b.m2[r])
+      ny++;
+    less = less || nt < NT || ny < D / 2;
+    b.nt[r] = (unsigned short)nt;
+    b.xstart[r] = x;
+    b.ystart[r] = y;
+    x += (unsigned)(nt * (ny + 1));
+    y += (unsigned)(nt * D * G);
+  }
+  b.xstart[n] = x;
+  b.ystart[n] = y;
+  b.compact = compact ? 1 : 0;
+  if (less)
+    b.n = n;
+  return b;
 }
 
 void launch_filter_accumulate(int D, float2* acc, const float2* U, float R, int filter_type, float delta_k,
@@ -1860,18 +2022,19 @@ bool launch_fft_x_filter(int D, const XPassArgs& args, int threads, cudaStream_t
   return true;
 }
 
-bool launch_fft_y(int D, float2* data, long long C, int n_spectra, int threads, cudaStream_t s)
+bool launch_fft_y(int D, float2* data, long long C, int n_spectra, const Bands& bands, int threads, cudaStream_t s)
 {
+  const YPassArgs a{ data, C, n_spectra, bands };
   switch (D) {
-    case 32: launch_y<32>(data, C, n_spectra, threads, s); break;
-    case 64: launch_y<64>(data, C, n_spectra, threads, s); break;
-    case 128: launch_y<128>(data, C, n_spectra, threads, s); break;
-    case 256: launch_y<256>(data, C, n_spectra, threads, s); break;
-    case 512: launch_y<512>(data, C, n_spectra, threads, s); break;
-    case 24: launch_y_t<24, TILE_THREADS_3>(data, C, n_spectra, s); break;
-    case 48: launch_y_t<48, TILE_THREADS_3>(data, C, n_spectra, s); break;
-    case 96: launch_y_t<96, TILE_THREADS_3>(data, C, n_spectra, s); break;
-    case 192: launch_y_t<192, TILE_THREADS_3>(data, C, n_spectra, s); break;
+    case 32: launch_y<32>(a, threads, s); break;
+    case 64: launch_y<64>(a, threads, s); break;
+    case 128: launch_y<128>(a, threads, s); break;
+    case 256: launch_y<256>(a, threads, s); break;
+    case 512: launch_y<512>(a, threads, s); break;
+    case 24: launch_y_t<24, TILE_THREADS_3>(a, s); break;
+    case 48: launch_y_t<48, TILE_THREADS_3>(a, s); break;
+    case 96: launch_y_t<96, TILE_THREADS_3>(a, s); break;
+    case 192: launch_y_t<192, TILE_THREADS_3>(a, s); break;
     default: return false;
   }
   fft_launches++;
@@ -1886,11 +2049,12 @@ bool fft_x_threads_ok(int D, int threads)
 int fft_z_rows_per_group(int D) { return fft3d_factor3(D) ? ZG_ROWS : 2048 / D; }
 
 template <int D, int T, int AXIS>
-static void launch_fwd_cols_t(float2* data, long long C, int n, cudaStream_t s)
+static void launch_fwd_cols_t(const FwdArgs& a, cudaStream_t s)
 {
-  const long long blocks = (long long)n * D * TilePlan<D>::NT;
+  const int n_outer = AXIS == 1 ? D : std::min(D, 2 * a.ny + 1);
+  const long long blocks = (long long)a.G * n_outer * a.nt;
   cudaFuncSetAttribute(k_fft_fwd_cols<D, T, AXIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_y<D>());
-  k_fft_fwd_cols<D, T, AXIS><<<(unsigned)blocks, T, smem_y<D>(), s>>>(data, C, n);
+  k_fft_fwd_cols<D, T, AXIS><<<(unsigned)blocks, T, smem_y<D>(), s>>>(a.out, a.C, a.nt, n_outer);
 }
 template <int D>
 static void launch_fwd(const FwdArgs& a, int threads, cudaStream_t s)
@@ -1900,21 +2064,26 @@ static void launch_fwd(const FwdArgs& a, int threads, cudaStream_t s)
   const long long blocks = (long long)a.G * D * D / FWD_ROWS;
   k_fft_z_r2c<D, gen_threads<D>()><<<(unsigned)blocks, gen_threads<D>(), bytes, s>>>(a);
   if constexpr (!is_pow2<D>()) {
-    launch_fwd_cols_t<D, TILE_THREADS_3, 1>(a.out, a.C, a.G, s);
-    launch_fwd_cols_t<D, TILE_THREADS_3, 0>(a.out, a.C, a.G, s);
+    launch_fwd_cols_t<D, TILE_THREADS_3, 1>(a, s);
+    launch_fwd_cols_t<D, TILE_THREADS_3, 0>(a, s);
   } else if (threads == 512) {
-    launch_fwd_cols_t<D, 512, 1>(a.out, a.C, a.G, s);
-    launch_fwd_cols_t<D, 512, 0>(a.out, a.C, a.G, s);
+    launch_fwd_cols_t<D, 512, 1>(a, s);
+    launch_fwd_cols_t<D, 512, 0>(a, s);
   } else {
-    launch_fwd_cols_t<D, 256, 1>(a.out, a.C, a.G, s);
-    launch_fwd_cols_t<D, 256, 0>(a.out, a.C, a.G, s);
+    launch_fwd_cols_t<D, 256, 1>(a, s);
+    launch_fwd_cols_t<D, 256, 0>(a, s);
   }
 }
 
-bool launch_fft_forward(int D, const FwdArgs& a, int threads, cudaStream_t s)
+bool launch_fft_forward(int D, const FwdArgs& args, int threads, cudaStream_t s)
 {
-  if (a.G < 1 || a.G > MAX_FIELDS)
+  if (args.G < 1 || args.G > MAX_FIELDS)
     return false;
+  FwdArgs a = args;
+  if (a.nt <= 0) {
+    a.nt = fft_pitch(D) / TXC;
+    a.ny = D / 2;
+  }
   switch (D) {
     case 32: launch_fwd<32>(a, threads, s); break;
     case 64: launch_fwd<64>(a, threads, s); break;
@@ -1950,11 +2119,11 @@ static void launch_ztg(const ZThresholdArgs& a, cudaStream_t s)
     a.recomb ? launch_ztg_cfg<D, false, true>(a, s) : launch_ztg_cfg<D, false, false>(a, s);
 }
 template <int D>
-static void launch_zsg(const float2* spectra, long long C, int n, int r0, float* shells, long long N, cudaStream_t s)
+static void launch_zsg(const ZStoreArgs& a, cudaStream_t s)
 {
   const size_t bytes = ZGPlan<D>::bytes(1);
   cudaFuncSetAttribute(k_fft_z_store_gen<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  k_fft_z_store_gen<D><<<D * D / ZG_ROWS, TILE_THREADS_3, bytes, s>>>(spectra, C, n, r0, shells, N);
+  k_fft_z_store_gen<D><<<D * D / ZG_ROWS, TILE_THREADS_3, bytes, s>>>(a);
 }
 
 bool launch_fft_z_threshold(int D, const ZThresholdArgs& a, cudaStream_t s)
@@ -1982,22 +2151,36 @@ bool launch_fft_z_threshold(int D, const ZThresholdArgs& a, cudaStream_t s)
   return true;
 }
 
-bool launch_fft_z_store(int D, const float2* spectra, long long C, int n, int r0, float* shells, long long N,
-                        unsigned* err, cudaStream_t s)
+bool launch_fft_z_store(int D, const float2* spectra, long long C, int n, int r0, const Bands& bands, float* shells,
+                        long long N, unsigned* err, cudaStream_t s)
 {
-  switch (D) {
-    case 32: launch_zs<32>(spectra, C, n, r0, shells, N, err, s); break;
-    case 64: launch_zs<64>(spectra, C, n, r0, shells, N, err, s); break;
-    case 128: launch_zs<128>(spectra, C, n, r0, shells, N, err, s); break;
-    case 256: launch_zs<256>(spectra, C, n, r0, shells, N, err, s); break;
-    case 512: launch_zs<512>(spectra, C, n, r0, shells, N, err, s); break;
-    case 24: launch_zsg<24>(spectra, C, n, r0, shells, N, s); break;
-    case 48: launch_zsg<48>(spectra, C, n, r0, shells, N, s); break;
-    case 96: launch_zsg<96>(spectra, C, n, r0, shells, N, s); break;
-    case 192: launch_zsg<192>(spectra, C, n, r0, shells, N, s); break;
-    default: return false;
+  // without band limits a batch may exceed the list: it goes in parts
+  for (int q = 0; q < n; q += MAX_BANDED) {
+    ZStoreArgs a;
+    a.spectra = spectra + (long long)q * C;
+    a.C = C;
+    a.n = std::min(n - q, MAX_BANDED);
+    a.r0 = r0 + q;
+    a.shells = shells;
+    a.N = N;
+    a.err = err;
+    for (int r = 0; r < a.n; r++)
+      a.nt[r] = bands.n ? bands.nt[q + r] : (unsigned short)(fft_pitch(D) / TXC);
+    const bool banded = bands.n > 0;
+    switch (D) {
+      case 32: launch_zs<32>(a, banded, s); break;
+      case 64: launch_zs<64>(a, banded, s); break;
+      case 128: launch_zs<128>(a, banded, s); break;
+      case 256: launch_zs<256>(a, banded, s); break;
+      case 512: launch_zs<512>(a, banded, s); break;
+      case 24: launch_zsg<24>(a, s); break;
+      case 48: launch_zsg<48>(a, s); break;
+      case 96: launch_zsg<96>(a, s); break;
+      case 192: launch_zsg<192>(a, s); break;
+      default: return false;
+    }
+    fft_launches++;
   }
-  fft_launches++;
   return true;
 }
 

@@ -491,13 +491,19 @@ float* mx_grids::* const SLAB_OUTPUTS[] = { &mx_grids::xH,   &mx_grids::z_at_ion
 static void run_xy(mx_ctx* c, const XPassArgs& xa, cudaStream_t s)
 {
   const double B8C = 8.0 * (double)c->gd.C;
-  const double x_bytes = B8C * xa.G * (1 + xa.n), y_bytes = 2.0 * B8C * xa.G * xa.n;
+  double x_bytes = B8C * xa.G * (1 + xa.n), y_bytes = 2.0 * B8C * xa.G * xa.n;
+  if (xa.bands.n) {
+    // the tiles inside the bands: read and written once (x), read and written (y)
+    const double line = 8.0 * 16.0 * c->gd.D;
+    x_bytes = 2.0 * 2.0 * line * xa.G * xa.bands.xstart[xa.n];
+    y_bytes = xa.bands.compact ? 2.0 * line * xa.bands.ystart[xa.n] : y_bytes;
+  }
   {
     Prof pr(c, "fft_x_filter", x_bytes, s);
     launch_fft_x_filter(c->gd.D, xa, c->x_threads, s);
   }
   Prof pr(c, "fft_y", y_bytes, s);
-  launch_fft_y(c->gd.D, xa.out, xa.C, xa.n * xa.G, c->y_threads, s);
+  launch_fft_y(c->gd.D, xa.out, xa.C, xa.n * xa.G, xa.bands, c->y_threads, s);
 }
 
 static void run_find_HII_bubbles(mx_ctx* c, int snapshot, const mx_grids* g, mx_globals* out, cudaStream_t s,
@@ -622,6 +628,7 @@ static void run_find_HII_bubbles(mx_ctx* c, int snapshot, const mx_grids* g, mx_
         xa.filter_type = p.filter_type;
         xa.delta_k = (float)(2.0 * k::PI / (float)p.box_size);
         xa.scale = (float)(1.0 / (double)gd.N);
+        xa.bands = filter_bands(gd.D, p.filter_type, xa.R, nf, G, xa.delta_k, false);
         run_xy(c, xa, s);
       }
       if (dl && dl->state_in && r0 == 0)
@@ -937,6 +944,7 @@ static void compute_shells(mx_ctx* c, const ShellPlan& sp, float* sfr, float* sf
   const int S = p.ts_num_filter_steps;
   float2* sfr_unf = c->d_unf;
   const long long nhalf = gd.C;
+  const float delta_k = (float)(2.0 * k::PI / (float)p.box_size);
   int r = 0;
   while (r < S) {
     for (const SfrOp& op : sp.ops[r]) {
@@ -970,7 +978,17 @@ static void compute_shells(mx_ctx* c, const ShellPlan& sp, float* sfr, float* sf
       fa.G = 1;
       fa.out = sfr_unf;
       fa.C = c->unf_C;
-      Prof pr(c, "fft_forward", 4.0 * (double)gd.N * (gd.D + 2) / gd.D + 40.0 * (double)c->unf_C, s);
+      // only the modes inside the widest band of the group's shells are read
+      float R_min = (float)sp.R[q_first];
+      for (int q = q_first; q < r_end; q++)
+        R_min = std::min(R_min, (float)sp.R[q]);
+      const Bands widest = filter_bands(gd.D, p.ts_heating_filter_type, &R_min, 1, 1, delta_k, true);
+      if (widest.n) {
+        fa.nt = widest.nt[0];
+        fa.ny = (int)(widest.xstart[1] / widest.nt[0]) - 1;
+      }
+      const double share = fa.nt ? (double)(fa.nt * 16) / fft_pitch(gd.D) : 1.0;
+      Prof pr(c, "fft_forward", 4.0 * (double)gd.N * (gd.D + 2) / gd.D + 40.0 * (double)c->unf_C * share, s);
       launch_fft_forward(gd.D, fa, c->y_threads, s);
     } else if (q_first < r_end) {
       MX_CUFFT(cufftSetStream(c->r2c_plan, s));
@@ -995,12 +1013,15 @@ static void compute_shells(mx_ctx* c, const ShellPlan& sp, float* sfr, float* sf
           xa.apply[q] = 1;
         }
         xa.filter_type = p.ts_heating_filter_type;
-        xa.delta_k = (float)(2.0 * k::PI / (float)p.box_size);
+        xa.delta_k = delta_k;
         xa.scale = (float)(1.0 / (double)gd.N);
+        xa.bands = filter_bands(gd.D, p.ts_heating_filter_type, xa.R, nb, 1, delta_k, true);
         run_xy(c, xa, s);
         {
-          Prof pr(c, "fft_z_store", (8.0 * (double)gd.C + 4.0 * (double)gd.N) * nb, s);
-          launch_fft_z_store(gd.D, c->d_work, c->work_C, nb, q0, c->d_shells, gd.N, c->d_err, s);
+          const double rows =
+            xa.bands.n ? 8.0 * 16.0 * (double)gd.D * xa.bands.ystart[nb] : 8.0 * (double)gd.C * nb;
+          Prof pr(c, "fft_z_store", rows + 4.0 * (double)gd.N * nb, s);
+          launch_fft_z_store(gd.D, c->d_work, c->work_C, nb, q0, xa.bands, c->d_shells, gd.N, c->d_err, s);
         }
         q0 += nb;
         continue;
@@ -2396,7 +2417,7 @@ int mx_create_limited(const mx_params* params, const char* tables_dir, size_t ma
 // not the arithmetic).  Which one is faster depends on the grid size: a tile
 // of a small grid has few points, at 512^3 the larger block keeps more loads in
 // flight.  The context times them on its own scratch at creation (zero spectra
-// of its fields, up to 16 radii or 1 GB, best of five launches) and keeps the
+// of its fields, up to 16 radii or 256 MB, best of three launches) and keeps the
 // fastest.  MX_XPASS_THREADS / MX_YPASS_THREADS fix a choice; MX_AUTOTUNE=0
 // keeps the defaults (x 512, y 256).
 // Register budget of the threshold z-pass (power-of-two grids): 2 resident
@@ -2512,7 +2533,7 @@ static void tune_fft(mx_ctx* c)
   MX_CUDA(cudaMemsetAsync(c->d_unf, 0, sizeof(float2) * c->unf_C * G, s));
   const long long spectrum_bytes = (long long)sizeof(float2) * c->work_C;
   const int n =
-    (int)std::max<long long>(1, std::min<long long>({ c->work_fields / G, (1LL << 30) / (spectrum_bytes * G), 16 }));
+    (int)std::max<long long>(1, std::min<long long>({ c->work_fields / G, (1LL << 28) / (spectrum_bytes * G), 16 }));
   XPassArgs xa;
   for (int f = 0; f < MAX_FIELDS; f++)
     xa.in[f] = f < G ? c->d_unf + (long long)f * c->unf_C : nullptr;
@@ -2533,7 +2554,7 @@ static void tune_fft(mx_ctx* c)
   auto best_ms = [&](auto&& launch) {
     launch();  // warm-up
     float best = 1e30f;
-    for (int i = 0; i < 5; i++) {
+    for (int i = 0; i < 3; i++) {
       cudaEventRecord(e0, s);
       launch();
       cudaEventRecord(e1, s);
@@ -2554,7 +2575,7 @@ static void tune_fft(mx_ctx* c)
       }
     }
     if (!fy && t >= 256) {
-      const float ms = best_ms([&] { launch_fft_y(gd.D, c->d_work, c->work_C, n * G, t, s); });
+      const float ms = best_ms([&] { launch_fft_y(gd.D, c->d_work, c->work_C, n * G, Bands{}, t, s); });
       if (ms < ty) {
         ty = ms;
         c->y_threads = t;
