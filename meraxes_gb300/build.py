@@ -40,7 +40,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     os.makedirs(os.path.join(OUT_DIR, "obj"), exist_ok=True)
     cc = nvcc()
-    common = ["-O3", "-std=c++17", "-lineinfo", "--split-compile=0", "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "include"),
+    common = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "include"),
               "-I", CSRC] + ARCH
 
     def compile_one(src: str) -> str:

@@ -65,6 +65,22 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 }
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// The same in one packed instruction for both parts (each rounded as the scalar
+// operation is); a - b as the fused multiply-add (-1) b + a, whose product is
+// exact.  Fewer issue slots, but register pairs: used where measured faster.
+template <bool PACKED>
+__device__ __forceinline__ float2 padd(float2 a, float2 b)
+{
+  return PACKED ? __fadd2_rn(a, b) : cadd(a, b);
+}
+template <bool PACKED>
+__device__ __forceinline__ float2 psub(float2 a, float2 b)
+{
+  return PACKED ? __ffma2_rn(b, make_float2(-1.0f, -1.0f), a) : csub(a, b);
+}
+// a + i b and a - i b (scalar: the swap of b's parts would cost what packing saves)
+__device__ __forceinline__ float2 cadd_i(float2 a, float2 b) { return make_float2(a.x - b.y, a.y + b.x); }
+__device__ __forceinline__ float2 csub_i(float2 a, float2 b) { return make_float2(a.x + b.y, a.y - b.x); }
 
 __host__ __device__ constexpr int ilog2(int m) { return m <= 1 ? 0 : 1 + ilog2(m / 2); }
 __host__ __device__ constexpr int brev(int i, int bits)
@@ -118,28 +134,48 @@ __device__ __forceinline__ float2 mul_tw(float2 b)
 
 // Butterflies of a radix-2 decimation-in-time DFT, stage HALF, group I,
 // butterfly J, unrolled by template recursion so every twiddle is a constant.
-template <int M, int HALF, int I, int J>
+template <bool PK, int M, int HALF, int I, int J>
 __device__ __forceinline__ void dft_stage(float2 (&v)[M])
 {
   if constexpr (HALF < M) {
     if constexpr (I < M) {
       if constexpr (J < HALF) {
-        const float2 b = mul_tw<J, 2 * HALF>(v[I + J + HALF]);
-        const float2 a = v[I + J];
-        v[I + J] = cadd(a, b);
-        v[I + J + HALF] = csub(a, b);
-        dft_stage<M, HALF, I, J + 1>(v);
+        if constexpr (PK) {
+          constexpr int ROOT8 = 8 * J / (2 * HALF);  // eighth root of unity
+          const float2 b = v[I + J + HALF], a = v[I + J];
+          if constexpr (ROOT8 == 1 || ROOT8 == 3) {
+            // a +- h t with t = b (1 + i) resp. b (i - 1), the multiply-add
+            // that the scalar form contracts to
+            constexpr float h = 0.70710678118654752440f;
+            const float2 t = ROOT8 == 1 ? make_float2(b.x - b.y, b.x + b.y) : make_float2(-(b.x + b.y), b.x - b.y);
+            v[I + J] = __ffma2_rn(t, make_float2(h, h), a);
+            v[I + J + HALF] = __ffma2_rn(t, make_float2(-h, -h), a);
+          } else if constexpr (ROOT8 == 2) {
+            v[I + J] = cadd_i(a, b);
+            v[I + J + HALF] = csub_i(a, b);
+          } else {
+            static_assert(J == 0, "radix 2, 4 or 8");
+            v[I + J] = padd<true>(a, b);
+            v[I + J + HALF] = psub<true>(a, b);
+          }
+        } else {
+          const float2 b = mul_tw<J, 2 * HALF>(v[I + J + HALF]);
+          const float2 a = v[I + J];
+          v[I + J] = cadd(a, b);
+          v[I + J + HALF] = csub(a, b);
+        }
+        dft_stage<PK, M, HALF, I, J + 1>(v);
       } else {
-        dft_stage<M, HALF, I + 2 * HALF, 0>(v);
+        dft_stage<PK, M, HALF, I + 2 * HALF, 0>(v);
       }
     } else {
-      dft_stage<M, 2 * HALF, 0, 0>(v);
+      dft_stage<PK, M, 2 * HALF, 0, 0>(v);
     }
   }
 }
 
 // In-register backward DFT of M points: v[k] <- sum_n v[n] exp(+2 pi i nk/M).
-template <int M>
+template <bool PK, int M>
 __device__ __forceinline__ void dft_bwd(float2 (&v)[M])
 {
   constexpr int LOG = ilog2(M);
@@ -152,7 +188,7 @@ __device__ __forceinline__ void dft_bwd(float2 (&v)[M])
       v[j] = t;
     }
   }
-  dft_stage<M, 1, 0, 0>(v);
+  dft_stage<PK, M, 1, 0, 0>(v);
 }
 
 // Backward DFT of 3 points, v_k <- sum_n v_n w^{nk} with w = exp(2 pi i / 3)
@@ -170,13 +206,13 @@ __device__ __forceinline__ void dft3_bwd(float2 (&v)[3])
 }
 
 // In-register backward DFT of M points, M a power of two or 3.
-template <int M>
+template <bool PK, int M>
 __device__ __forceinline__ void dft_any(float2 (&v)[M])
 {
   if constexpr (M == 3)
     dft3_bwd(v);
   else
-    dft_bwd<M>(v);
+    dft_bwd<PK, M>(v);
 }
 
 // k-space filter of reionization.c:2110-2170:
@@ -350,6 +386,15 @@ __host__ __device__ constexpr int tile_groups()
 {
   return NTHR == 128 ? 2 : 1;
 }
+// The threads of a tile as fill_twiddles takes them.  A constant lets the
+// compiler schedule the table among the loads before it, which is faster for
+// 256 threads (y-pass at 128^3 682 instead of 750 us, 256^3 4.89 instead of 5.10
+// ms) and slower for 512 (512^3 36.1 instead of 34.0 ms).
+template <int NTHR>
+__device__ __forceinline__ int tile_threads()
+{
+  return NTHR == 512 ? (int)blockDim.x : NTHR;
+}
 template <int NTHR>
 __device__ __forceinline__ int tile_tid()
 {
@@ -373,6 +418,10 @@ __device__ __forceinline__ void tile_sync()
 // TileSteps; the caller puts a barrier between them and after the last one
 // before it reuses buf.  tile_dft() runs all three.
 //
+// PK: packed additions.  They pay in the y-pass and the forward passes with 512
+// threads (at 512^3 34.0 -> 32.8 and 3.30 -> 3.17 ms), not with 256 (256^3: 4.89
+// -> 5.22 ms) nor in the x-pass (512^3: 35.5 -> 36.0 ms).
+//
 // Thread roles are fixed: column t = tid % TXC and slot s = tid / TXC of
 // S = NTHR / TXC slots (NTHR threads in the block).  A half-warp is the 16 columns of one slot,
 // so every shared and global access of a half-warp is one 128-byte line.
@@ -391,7 +440,7 @@ struct XSmem
   static constexpr int FLOAT2 = YSmem<D>::FLOAT2 + ((D / 2 + 1) * TXC + 1) / 2;
 };
 
-template <int D, int NTHR>
+template <int D, int NTHR, bool PK = false>
 struct TileSteps
 {
   using P = TilePlan<D>;
@@ -434,7 +483,7 @@ struct TileSteps
 #pragma unroll
         for (int n1 = 0; n1 < R1; n1++)
           v[n1] = load(np + M * n1, t, j * R1 + n1);
-        dft_any<R1>(v);
+        dft_any<PK, R1>(v);
         col[np * TXC] = v[0];
 #pragma unroll
         for (int k1 = 1; k1 < R1; k1++)
@@ -458,7 +507,7 @@ struct TileSteps
 #pragma unroll
         for (int n2 = 0; n2 < R2; n2++)
           v[n2] = line[R3 * n2 * TXC];
-        dft_any<R2>(v);
+        dft_any<PK, R2>(v);
         line[0] = v[0];
 #pragma unroll
         for (int k2 = 1; k2 < R2; k2++)
@@ -493,7 +542,7 @@ struct TileSteps
 #pragma unroll
         for (int n3 = 0; n3 < R3; n3++)
           v[n3] = line[n3 * TXC];
-        dft_any<R3>(v);
+        dft_any<PK, R3>(v);
 #pragma unroll
         for (int k3 = 0; k3 < R3; k3++)
           out[j * R3 + k3] = v[k3];
@@ -518,7 +567,7 @@ struct TileSteps
 #pragma unroll
         for (int n3 = 0; n3 < R3; n3++)
           v[n3] = line[n3 * TXC];
-        dft_any<R3>(v);
+        dft_any<PK, R3>(v);
 #pragma unroll
         for (int k3 = 0; k3 < R3; k3++)
           store(k1 + R1 * (k2 + R2 * k3), t, v[k3]);
@@ -601,8 +650,8 @@ __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_bloc
   float* wsm = reinterpret_cast<float*>(buf + P::BUF);
   const unsigned item = blockIdx.x * tile_groups<XTHREADS>() + tile_group<XTHREADS>();
   int r, kyp, kz0;  // |ky|: the block transforms rows ky = kyp and D - kyp
-  int pitch = Pitch<D>::HP;
-  float kx2_max = 0.0f;
+  int pitch;             // BANDED
+  float kx2_max = 0.0f;  // BANDED
   if constexpr (BANDED) {
     if (item >= a.bands.xstart[a.n])
       return;
@@ -616,17 +665,17 @@ __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_bloc
     if ((float)(kyp * kyp + kz0 * kz0) > m2)
       return;
     kx2_max = m2 - (float)(kyp * kyp + kz0 * kz0);
-    if (a.bands.compact)
-      pitch = nt * TXC;
+    pitch = a.bands.compact ? nt * TXC : Pitch<D>::HP;
+    fill_twiddles<D>(tw, tid, tile_threads<XTHREADS>());
   } else {
-    if (item >= (unsigned)(H * P::NT) * a.n)
+    fill_twiddles<D>(tw, tid, tile_threads<XTHREADS>());
+    if (tile_groups<XTHREADS>() > 1 && item >= (unsigned)(H * P::NT) * a.n)
       return;
     r = item % a.n;
     const int tile = item / a.n;
     kyp = tile / P::NT;
     kz0 = (tile % P::NT) * TXC;
   }
-  fill_twiddles<D>(tw, tid, XTHREADS);
   // the weights depend on ky only through kyv^2, the same for both rows
   const float kyv = kcomp(kyp, D, a.delta_k);
   // this thread's column: kz = kz0 + t, the same in every step
@@ -668,7 +717,7 @@ __global__ void __launch_bounds__(XTHREADS * tile_groups<XTHREADS>(), x_min_bloc
       T::b(buf, tw);
       tile_sync<XTHREADS>();
       float2* __restrict__ dst =
-        a.out + (long long)(r * a.G + g) * a.C + (long long)ky * pitch + kz0 + t0;
+        a.out + (long long)(r * a.G + g) * a.C + (long long)ky * (BANDED ? pitch : Pitch<D>::HP) + kz0 + t0;
       if constexpr (BANDED)
         T::c(buf, [&](int x, int, float2 v) { dst[(long long)x * D * pitch] = v; });
       else
@@ -713,7 +762,7 @@ __global__ void __launch_bounds__(YTHREADS, YTHREADS == 256 ? 3 : 2) k_fft_y(con
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* buf = smem + D;
-  using T = TileSteps<D, YTHREADS>;
+  using T = TileSteps<D, YTHREADS, YTHREADS == 512>;
   float2 pts[T::NPTS];
   int pitch = HP;
   float2* col;
@@ -757,7 +806,7 @@ __global__ void __launch_bounds__(YTHREADS, YTHREADS == 256 ? 3 : 2) k_fft_y(con
     // while the twiddle table is filled
     T::for_each_input([&](int ky, int i) { pts[i] = col[ky * HP]; });
   }
-  fill_twiddles<D>(tw, threadIdx.x, YTHREADS);
+  fill_twiddles<D>(tw, threadIdx.x, tile_threads<YTHREADS>());
   __syncthreads();
   T::a(buf, tw, [&](int, int, int i) { return pts[i]; });
   __syncthreads();
@@ -844,15 +893,15 @@ struct ZPlan
 // index of the output held in slot e by lane-part l of an L-lane DFT
 __device__ __forceinline__ int lane_out(int L, int e, int l) { return L == 4 ? l + 4 * e : e + 4 * l; }
 
+// (packed additions: threshold pass at 512^3 50.9 -> 49.9 ms, 256^3 6.66 -> 6.41)
 __device__ __forceinline__ void dft4_bwd(float2 (&v)[4])
 {
-  const float2 t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-  const float2 t2 = cadd(v[1], v[3]), d = csub(v[1], v[3]);
-  const float2 t3 = make_float2(-d.y, d.x);  // i (v1 - v3)
-  v[0] = cadd(t0, t2);
-  v[1] = cadd(t1, t3);
-  v[2] = csub(t0, t2);
-  v[3] = csub(t1, t3);
+  const float2 t0 = padd<true>(v[0], v[2]), t1 = psub<true>(v[0], v[2]);
+  const float2 t2 = padd<true>(v[1], v[3]), d = psub<true>(v[1], v[3]);
+  v[0] = padd<true>(t0, t2);
+  v[1] = cadd_i(t1, d);
+  v[2] = psub<true>(t0, t2);
+  v[3] = csub_i(t1, d);
 }
 
 __device__ __forceinline__ float2 shfl_xor2(float2 v, int m)
@@ -935,7 +984,8 @@ __device__ __forceinline__ float2 unit(int j, int n)
 
 // Per-thread twiddle factors of the z-pass.  A thread's step-A and step-B
 // roles are fixed for the whole kernel, so its twiddles are a few base values
-// kept in registers; the others follow by complex products.
+// kept in registers; the others follow by complex products (all of them in
+// registers measured no faster, 49.7 against 49.8 ms at 512^3).
 template <int D>
 struct ZTw
 {
@@ -1027,8 +1077,8 @@ __device__ __forceinline__ bool z_c2r(char* smem, int it, int n_items, const flo
         B.y = 0.0f;
       }
       B.y = -B.y;
-      const float2 E = cadd(A, B);
-      const float2 O = cmul(csub(A, B), tk);
+      const float2 E = padd<true>(A, B);
+      const float2 O = cmul(psub<true>(A, B), tk);
       v[i] = make_float2(E.x - O.y, E.y + O.x);
       if (i < 3)
         tk = cmul(tk, w.kr);
@@ -1123,23 +1173,206 @@ __device__ __noinline__ bool threshold_fp64(float dx, float stv, float nr, float
   return f_coll * eff > nf * (1. + rec);
 }
 
-// cell state bits of the threshold z-pass
-constexpr unsigned ST_ION = 1u;      // ionised at some radius of this launch
-constexpr unsigned ST_XHIGH = 2u;    // xH at launch start > REL_TOL
-constexpr unsigned ST_XLOW = 4u;     // xH at launch start < REL_TOL
-constexpr unsigned ST_ZUNSET = 8u;   // z_at_ionization < 0
-constexpr int ST_RB_SHIFT = 8;       // radius index of the last ionising radius
+// v clamped at 0, values below ABS_TOL set to 0 (find_HII_bubbles.c:271-311;
+// also 0 for NaN, as fmaxf gives)
+__device__ __forceinline__ float clamp_tol(float v) { return v >= ABS_TOL_F ? v : 0.0f; }
+
+// State of a thread's 2 NP cells (pairs i = 0 ... NP - 1, cell c = 2 i + {0, 1})
+// in the threshold z-passes: one bit per cell and test, and the index of the
+// last ionising radius of the launch, a byte per cell.  The bookkeeping of a
+// radius is a few operations on the masks instead of a dozen per cell, which
+// were 40% of the pass's instructions.
+template <int NP>
+struct CellState
+{
+  unsigned valid;   // cells of this thread
+  unsigned ion;     // ionised at some radius of this launch
+  unsigned xhigh;   // xH at launch start > REL_TOL
+  unsigned xlow;    // xH at launch start < REL_TOL
+  unsigned zunset;  // z_at_ionization < 0
+  unsigned rb[(2 * NP + 3) / 4];
+
+  __device__ __forceinline__ void clear()
+  {
+    valid = ion = xhigh = xlow = zunset = 0;
+#pragma unroll
+    for (int i = 0; i < (2 * NP + 3) / 4; i++)
+      rb[i] = 0;
+  }
+  // xH and z_at_ionization of pair i at launch start
+  __device__ __forceinline__ void start(int i, float2 x0, float2 z0)
+  {
+    const unsigned lo = 1u << 2 * i, hi = 2u << 2 * i;
+    valid |= lo | hi;
+    xhigh |= (x0.x > REL_TOL_F ? lo : 0u) | (x0.y > REL_TOL_F ? hi : 0u);
+    xlow |= (x0.x < REL_TOL_F ? lo : 0u) | (x0.y < REL_TOL_F ? hi : 0u);
+    zunset |= (z0.x < 0 ? lo : 0u) | (z0.y < 0 ? hi : 0u);
+  }
+  // radius r ionises the cells `now`; returns the cells ionised for the first
+  // time, and in *z those whose z_at_ionization is set
+  __device__ __forceinline__ unsigned ionise(unsigned now, int r, unsigned* z)
+  {
+    const unsigned first = now & xhigh & ~ion;
+    ion |= now;
+#pragma unroll
+    for (int i = 0; i < (2 * NP + 3) / 4; i++) {
+      // four cells' bits to their bytes
+      const unsigned m = (((now >> 4 * i & 0xfu) * 0x00204081u) & 0x01010101u) * 0xffu;
+      rb[i] = (rb[i] & ~m) | (m & (unsigned)r * 0x01010101u);
+    }
+    *z = (ion | xlow) & zunset;
+    zunset &= ~*z;
+    return first;
+  }
+  __device__ __forceinline__ int radius(int c) const { return rb[c >> 2] >> 8 * (c & 3) & 0xff; }
+};
+
+// The cells that a filtered radius ionises (find_HII_bubbles.c:342-428): f
+// holds deltax, stars, -, x_e, N_rec of the thread's pairs.  FP32 (a 2-ulp
+// reciprocal is well inside the margin), and FP64 where the two sides lie
+// within 4e-6 of each other.
+template <bool SPIN, bool RECOMB, int NP, int G>
+__device__ __forceinline__ unsigned ionised_cells(const float2 (&f)[G][NP], unsigned valid, const RadiusParams* rp,
+                                                  double pixel_volume, double eff)
+{
+  constexpr int IXE = 3, INR = SPIN ? 4 : 3;
+  const float kfc = rp->kfc;
+  unsigned now = 0, near = 0;
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+    const float2 one = make_float2(1.0f, 1.0f);
+    const float2 dx = make_float2(fmaxf(f[0][i].x, -1 + REL_TOL_F), fmaxf(f[0][i].y, -1 + REL_TOL_F));
+    const float2 st = make_float2(clamp_tol(f[1][i].x), clamp_tol(f[1][i].y));
+    const float2 dom = __fadd2_rn(one, dx);
+    const float2 inv = make_float2(__fdividef(1.0f, dom.x), __fdividef(1.0f, dom.y));
+    const float2 lhs = __fmul2_rn(__fmul2_rn(st, make_float2(kfc, kfc)), inv);
+    float2 rhs = one;
+    if constexpr (RECOMB) {
+      const float2 nr = make_float2(clamp_tol(f[INR][i].x), clamp_tol(f[INR][i].y));
+      rhs = __ffma2_rn(nr, inv, one);
+    }
+    if constexpr (SPIN) {
+      const float2 xe =
+        make_float2(fminf(clamp_tol(f[IXE][i].x), 0.999f), fminf(clamp_tol(f[IXE][i].y), 0.999f));
+      rhs = __fmul2_rn(__ffma2_rn(xe, make_float2(-1.0f, -1.0f), one), rhs);
+    }
+    const float2 d = psub<true>(lhs, rhs);
+    const float2 band = __fmul2_rn(make_float2(fmaxf(lhs.x, rhs.x), fmaxf(lhs.y, rhs.y)), make_float2(4e-6f, 4e-6f));
+    if (lhs.x > rhs.x)
+      now |= 1u << 2 * i;
+    if (lhs.y > rhs.y)
+      now |= 2u << 2 * i;
+    if (!(fabsf(d.x) > band.x))
+      near |= 1u << 2 * i;
+    if (!(fabsf(d.y) > band.y))
+      near |= 2u << 2 * i;
+  }
+  near &= valid;
+  if (near) {
+    const double M_mean = rp->M_mean, R_cubed = rp->R_cubed;
+#pragma unroll
+    for (int c = 0; c < 2 * NP; c++) {
+      if (!(near >> c & 1u))
+        continue;
+      const int i = c >> 1;
+      auto part = [&](int g) { return (c & 1) ? f[g][i].y : f[g][i].x; };
+      float xpart;
+      const bool in = threshold_fp64(fmaxf(part(0), -1 + REL_TOL_F), clamp_tol(part(1)),
+                                     RECOMB ? clamp_tol(part(INR < G ? INR : 0)) : 0.0f,
+                                     SPIN ? fminf(clamp_tol(part(IXE < G ? IXE : 0)), 0.999f) : 0.0f, RECOMB, SPIN, M_mean,
+                                     R_cubed, pixel_volume, eff, &xpart);
+      now = (now & ~(1u << c)) | (in ? 1u << c : 0u);
+    }
+  }
+  return now & valid;
+}
+
+// The unfiltered last radius r (an identity transform: the fields are read from
+// the padded input grids at ip) for cell c, whose xH may become partial.
+// Returns whether it is ionised; *z as in CellState::ionise.
+template <bool SPIN, bool RECOMB, int NP>
+__device__ __forceinline__ void last_radius_cell(const ZThresholdArgs& a, CellState<NP>& st, int c, int r, long long ip,
+                                                 long long ir)
+{
+  constexpr int IXE = 3, INR = SPIN ? 4 : 3;
+  const RadiusParams& rp = a.rp[r];
+  const float dx = fmaxf(a.direct[0][ip], -1 + REL_TOL_F);
+  const float stv = clamp_tol(a.direct[1][ip]);
+  const float nr = RECOMB ? clamp_tol(a.direct[INR][ip]) : 0.0f;
+  const float xe = SPIN ? fminf(clamp_tol(a.direct[IXE][ip]), 0.999f) : 0.0f;
+  const float inv_dom = __fdividef(1.0f, 1.0f + dx);
+  const float lhs = stv * rp.kfc * inv_dom;
+  const float nf = 1.0f - xe;
+  const float rhs = nf * (1.0f + nr * inv_dom);
+  bool ionised = lhs > rhs;
+  float xpart = nf - lhs;
+  if (!(fabsf(lhs - rhs) > 4e-6f * fmaxf(lhs, rhs)))
+    ionised =
+      threshold_fp64(dx, stv, nr, xe, RECOMB, SPIN, rp.M_mean, rp.R_cubed, a.pixel_volume, a.eff, &xpart);
+  const unsigned bit = 1u << c;
+  const bool running_high = !(st.ion & bit) && (st.xhigh & bit);
+  bool low = (st.ion & bit) || (st.xlow & bit);
+  const bool first = ionised && running_high;
+  if (ionised) {
+    st.ion |= bit;
+    a.xH[ir] = 0.0f;
+    a.r_bubble[ir] = (float)rp.R;
+    low = true;
+  } else if (running_high) {
+    const float xn = fminf(fmaxf(xpart, 0.0f), 1.0f);
+    a.xH[ir] = xn;
+    low = xn < REL_TOL_F;
+  }
+  const bool set_z = low && (st.zunset & bit);
+  if (set_z)
+    a.z_at_ion[ir] = (float)a.redshift;
+  if ((first && (a.uvb || RECOMB)) || (set_z && a.uvb)) {
+    const float ws = clamp_tol(a.direct[2][ip]);
+    const float J21 = a.uvb ? ws * rp.kj : 0.0f;
+    if (first && a.uvb)
+      a.J21[ir] = J21;
+    if (first && RECOMB)
+      a.Gamma12[ir] = ws * rp.kg;
+    if (set_z && a.uvb)
+      a.J21_at_ion[ir] = J21 * a.gamma_halo_bias;
+  }
+}
+
+// The stores of a filtered radius: z_at_ionization of the cells `z`, and for
+// the first crossings the values that weighted_sfr (v) gives.  cell(c) is the
+// REAL index of cell c.
+template <bool RECOMB, int NP, class Cell>
+__device__ __forceinline__ void store_first(const ZThresholdArgs& a, const RadiusParams* rp, unsigned first, unsigned z,
+                                            const float2 (&v)[NP], Cell cell)
+{
+  const float kj = rp->kj, kg = rp->kg;
+#pragma unroll
+  for (int c = 0; c < 2 * NP; c++) {
+    if (!((first | z) >> c & 1u))
+      continue;
+    const long long ir = cell(c);
+    const float ws = clamp_tol((c & 1) ? v[c >> 1].y : v[c >> 1].x);
+    const float J21 = a.uvb ? ws * kj : 0.0f;
+    if (first >> c & 1u) {
+      if (a.uvb)
+        a.J21[ir] = J21;
+      if (RECOMB)
+        a.Gamma12[ir] = ws * kg;
+    }
+    if (z >> c & 1u)
+      a.J21_at_ion[ir] = J21 * a.gamma_halo_bias;
+  }
+}
 }  // namespace
 
 // z-pass fused with the per-cell test of find_HII_bubbles (clamps
 // :271-311, criterion and bookkeeping :342-443) for every radius of the batch.
 // Grid: one block per TZ rows.  A thread transforms, for each field of a
 // radius, the 8 cells it then tests, so the fields of a cell meet in
-// registers.  The cell state is a few bits per cell: whether it is ionised,
-// the xH and z_at_ionization tests at launch start, and the index of the last
-// ionising radius.  J_21, Gamma12, z_at_ionization and J_21_at_ionization
-// change at most once per cell per launch (at the first crossing) and are
-// stored when that happens; xH and r_bubble are stored at the end.
+// registers.  The cell state is a few bits per cell (CellState).  J_21, Gamma12,
+// z_at_ionization and J_21_at_ionization change at most once per cell per
+// launch (at the first crossing) and are stored when that happens; xH and
+// r_bubble are stored at the end.
 //
 // SPIN and RECOMB fix the fields at compile time: deltax, stars,
 // weighted_sfr, then x_e with the spin temperature, then N_rec with
@@ -1151,7 +1384,6 @@ __global__ void __launch_bounds__(FFT_THREADS, MINB) k_fft_z_threshold(ZThreshol
 {
   using P = ZPlan<D>;
   constexpr int G = 3 + (SPIN ? 1 : 0) + (RECOMB ? 1 : 0);
-  constexpr int IXE = 3, INR = SPIN ? 4 : 3;
   extern __shared__ __align__(128) unsigned char zsmem[];
   char* smem = reinterpret_cast<char*>(zsmem);
   const long long row0 = ((long long)blockIdx.x + a.group0) * P::TZ;
@@ -1162,150 +1394,66 @@ __global__ void __launch_bounds__(FFT_THREADS, MINB) k_fft_z_threshold(ZThreshol
   // this thread's cells: row t, z = 2 m_e + {0, 1}
   const int l = threadIdx.x % P::L2, k1 = (threadIdx.x / P::L2) % P::P1, t = threadIdx.x / (P::L2 * P::P1);
   const long long rowc = row0 + t;
-  int zc[4];
+  auto cell = [&](int c) { return rowc * D + 2 * (k1 + P::P1 * lane_out(P::L2, c >> 1, l)) + (c & 1); };
+  CellState<4> st;
+  st.clear();
 #pragma unroll
   for (int e = 0; e < 4; e++)
-    zc[e] = 2 * (k1 + P::P1 * lane_out(P::L2, e, l));
-  unsigned st[8];
-#pragma unroll
-  for (int e = 0; e < 4; e++) {
-    const long long ir = rowc * D + zc[e];
-    const float2 x0 = *reinterpret_cast<const float2*>(a.xH + ir);
-    const float2 z0 = *reinterpret_cast<const float2*>(a.z_at_ion + ir);
-    st[2 * e] = (x0.x > REL_TOL_F ? ST_XHIGH : 0u) | (x0.x < REL_TOL_F ? ST_XLOW : 0u) | (z0.x < 0 ? ST_ZUNSET : 0u);
-    st[2 * e + 1] = (x0.y > REL_TOL_F ? ST_XHIGH : 0u) | (x0.y < REL_TOL_F ? ST_XLOW : 0u) | (z0.y < 0 ? ST_ZUNSET : 0u);
-  }
+    st.start(e, *reinterpret_cast<const float2*>(a.xH + cell(2 * e)),
+             *reinterpret_cast<const float2*>(a.z_at_ion + cell(2 * e)));
   // weighted_sfr (field 2) enters only the J_21 / Gamma12 values of a cell
   // ionised for the first time at this radius and J_21_at_ionization where
   // z_at_ionization is first set; its transform is skipped for a block with
   // no such cell (its ring item is still consumed)
   const bool need_ws = a.uvb || RECOMB;
   int it = 0;
-  for (int r = 0; r < a.n_r; r++) {
-    const RadiusParams rp = a.rp[r];
-    const bool direct = rp.last != 0;
+  for (int r = 0; r < a.n_f; r++) {
     float2 f[G][4];
-    if (!direct) {
 #pragma unroll
-      for (int j = 0; j < G - 1; j++) {
-        const int g = j < 2 ? j : j + 1;
-        if (!z_c2r<D, true>(smem, it, n_items, a.spectra, a.C, row0, w, f[g], G)) {
-          z_abort<D>(smem, it, n_items, a.err);
-          return;
-        }
-        it++;
-      }
-    } else {
-#pragma unroll
-      for (int g = 0; g < G; g++)
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-          f[g][e] = *reinterpret_cast<const float2*>(a.direct[g] + rowc * 2LL * P::H + zc[e]);
-    }
-    // the test and the state update; bit c of first_ion / first_z marks a
-    // cell whose J_21 / Gamma12 resp. J_21_at_ionization is written below
-    unsigned first_ion = 0, first_z = 0;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int e = c >> 1;
-      const bool hi = c & 1;
-      const float v0 = hi ? f[0][e].y : f[0][e].x;
-      const float v1 = hi ? f[1][e].y : f[1][e].x;
-      const float dx = fmaxf(v0, -1 + REL_TOL_F);
-      float stv = fmaxf(v1, 0.0f);
-      if (stv < ABS_TOL_F)
-        stv = 0;
-      float nr = 0.0f, xe = 0.0f;
-      if constexpr (RECOMB) {
-        nr = hi ? f[INR][e].y : f[INR][e].x;
-        nr = fmaxf(nr, 0.0f);
-        if (nr < ABS_TOL_F)
-          nr = 0;
-      }
-      if constexpr (SPIN) {
-        xe = hi ? f[IXE][e].y : f[IXE][e].x;
-        xe = fmaxf(xe, 0.0f);
-        if (xe < ABS_TOL_F)
-          xe = 0;
-        xe = fminf(xe, 0.999f);
-      }
-      // FP32 estimate of the test (a 2-ulp reciprocal is well inside the
-      // 4e-6 margin below which the FP64 comparison decides)
-      const float inv_dom = __fdividef(1.0f, 1.0f + dx);
-      const float lhs_f = stv * rp.kfc * inv_dom;
-      const float nf_f = 1.0f - xe;
-      const float rhs_f = nf_f * (1.0f + nr * inv_dom);
-      bool ionised;
-      float xpart;
-      if (fabsf(lhs_f - rhs_f) > 4e-6f * fmaxf(lhs_f, rhs_f)) {
-        ionised = lhs_f > rhs_f;
-        xpart = nf_f - lhs_f;
-      } else {
-        ionised = threshold_fp64(dx, stv, nr, xe, RECOMB, SPIN, rp.M_mean, rp.R_cubed, a.pixel_volume, a.eff, &xpart);
-      }
-      const long long ir = rowc * D + zc[e] + (hi ? 1 : 0);
-      unsigned s = st[c];
-      const bool xr_high = !(s & ST_ION) && (s & ST_XHIGH);  // running xH > REL_TOL
-      bool xr_low = (s & ST_ION) || (s & ST_XLOW);            // running xH < REL_TOL
-      if (ionised) {
-        if (xr_high)
-          first_ion |= 1u << c;
-        s = (s & ((1u << ST_RB_SHIFT) - 1)) | ST_ION | ((unsigned)r << ST_RB_SHIFT);
-        xr_low = true;
-      } else if (rp.last && xr_high) {
-        const float xn = fminf(fmaxf(xpart, 0.0f), 1.0f);
-        a.xH[ir] = xn;
-        xr_low = xn < REL_TOL_F;
-      }
-      if (xr_low && (s & ST_ZUNSET)) {
-        a.z_at_ion[ir] = (float)a.redshift;
-        first_z |= 1u << c;
-        s &= ~ST_ZUNSET;
-      }
-      st[c] = s;
-    }
-    if (!need_ws)
-      first_ion = first_z = 0;
-    if (!a.uvb)
-      first_z = 0;
-    if (!direct) {
-      // field 2 of this radius: transformed if a cell of the block needs it
-      const bool any = __syncthreads_or((first_ion | first_z) != 0);
-      const bool ok = any ? z_c2r<D, true>(smem, it, n_items, a.spectra, a.C, row0, w, f[2], G)
-                          : z_skip<D>(smem, it, n_items, a.spectra, a.C, row0, G, w.full);
-      if (!ok) {
+    for (int j = 0; j < G - 1; j++) {
+      if (!z_c2r<D, true>(smem, it, n_items, a.spectra, a.C, row0, w, f[j < 2 ? j : j + 1], G)) {
         z_abort<D>(smem, it, n_items, a.err);
         return;
       }
       it++;
     }
+    const RadiusParams* rp = a.rp + r;
+    unsigned z;
+    unsigned first = st.ionise(ionised_cells<SPIN, RECOMB>(f, st.valid, rp, a.pixel_volume, a.eff), r, &z);
+    if (z) {
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      if (!((first_ion | first_z) >> c & 1u))
-        continue;
-      const int e = c >> 1;
-      const bool hi = c & 1;
-      const long long ir = rowc * D + zc[e] + (hi ? 1 : 0);
-      float ws = fmaxf(hi ? f[2][e].y : f[2][e].x, 0.0f);
-      if (ws < ABS_TOL_F)
-        ws = 0;
-      const float J21_aux = a.uvb ? ws * rp.kj : 0.0f;
-      if (first_ion >> c & 1u) {
-        if (a.uvb)
-          a.J21[ir] = J21_aux;
-        if (RECOMB)
-          a.Gamma12[ir] = ws * rp.kg;
-      }
-      if (first_z >> c & 1u)
-        a.J21_at_ion[ir] = J21_aux * a.gamma_halo_bias;
+      for (int c = 0; c < 8; c++)
+        if (z >> c & 1u)
+          a.z_at_ion[cell(c)] = (float)a.redshift;
     }
+    if (!need_ws)
+      first = 0;
+    if (!a.uvb)
+      z = 0;
+    // field 2 of this radius: transformed if a cell of the block needs it
+    const bool any = __syncthreads_or((first | z) != 0);
+    const bool ok = any ? z_c2r<D, true>(smem, it, n_items, a.spectra, a.C, row0, w, f[2], G)
+                        : z_skip<D>(smem, it, n_items, a.spectra, a.C, row0, G, w.full);
+    if (!ok) {
+      z_abort<D>(smem, it, n_items, a.err);
+      return;
+    }
+    it++;
+    if (first | z)
+      store_first<RECOMB>(a, rp, first, z, f[2], cell);
   }
 #pragma unroll
   for (int c = 0; c < 8; c++) {
-    if (st[c] & ST_ION) {
-      const long long ir = rowc * D + zc[c >> 1] + (c & 1);
-      a.xH[ir] = 0.0f;
-      a.r_bubble[ir] = (float)a.rp[st[c] >> ST_RB_SHIFT].R;
+    if (st.ion >> c & 1u) {
+      a.xH[cell(c)] = 0.0f;
+      a.r_bubble[cell(c)] = (float)a.rp[st.radius(c)].R;
+    }
+  }
+  if (a.n_r > a.n_f) {
+#pragma unroll 2
+    for (int c = 0; c < 8; c++) {
+      const long long ir = cell(c);
+      last_radius_cell<SPIN, RECOMB>(a, st, c, a.n_f, rowc * 2LL * P::H + (ir - rowc * D), ir);
     }
   }
 }
@@ -1403,7 +1551,7 @@ __global__ void __launch_bounds__(T) k_fft_z_r2c(const __grid_constant__ FwdArgs
     if (i < FWD_ROWS * H)
       v[j] = __ldg(src + i);
   }
-  fill_twiddles<L>(tw, threadIdx.x, T);
+  fill_twiddles<L>(tw, threadIdx.x, blockDim.x);
   for (int k = threadIdx.x; k < H; k += T) {
     float sn, cs;
     sincospif(2.0f * (float)k / (float)D, &sn, &cs);
@@ -1426,9 +1574,7 @@ __global__ void __launch_bounds__(T) k_fft_z_r2c(const __grid_constant__ FwdArgs
     [&](int k, int t, float2 v) { rows[t * H + k] = make_float2(v.x, -v.y); });
   __syncthreads();
   float2* __restrict__ dst = a.out + (long long)g * a.C + r0 * HP;
-  const int W = a.nt * TXC;  // columns that are read
-  for (int i = threadIdx.x; i < FWD_ROWS * W; i += T) {
-    const int t = i / W, k = i - t * W;
+  auto store = [&](int t, int k) {
     float2 X = make_float2(0.f, 0.f);
     if (k < H) {
       const float2 zk = rows[t * H + (k < L ? k : 0)];
@@ -1439,6 +1585,14 @@ __global__ void __launch_bounds__(T) k_fft_z_r2c(const __grid_constant__ FwdArgs
       X = make_float2(0.5f * (A.x + C.y), 0.5f * (A.y - C.x)); // (A - i C) / 2
     }
     dst[t * HP + k] = X;
+  };
+  if (a.nt == HP / TXC) {
+    for (int i = threadIdx.x; i < FWD_ROWS * HP; i += T)
+      store(i / HP, i % HP);
+  } else {
+    const int W = a.nt * TXC;  // the columns that are read
+    for (int i = threadIdx.x; i < FWD_ROWS * W; i += T)
+      store(i / W, i % W);
   }
 }
 
@@ -1455,16 +1609,25 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_fwd_cols(float2* da
   extern __shared__ float2 smem[];
   float2* tw = smem;
   float2* buf = smem + D;
-  const unsigned tile = blockIdx.x % nt, rest = blockIdx.x / nt;
-  int o = rest % n_outer;
-  const long long s = rest / n_outer;
-  if (AXIS == 0 && o > n_outer / 2)
-    o += D - n_outer;  // |ky| <= n_outer / 2
+  int tile, o;
+  long long s;
+  if (nt == P::NT && n_outer == D) {
+    tile = blockIdx.x % P::NT;
+    o = blockIdx.x / P::NT % D;
+    s = blockIdx.x / (P::NT * D);
+  } else {
+    const int rest = blockIdx.x / nt;
+    tile = blockIdx.x - rest * nt;
+    s = rest / n_outer;
+    o = rest - (int)s * n_outer;
+    if (AXIS == 0 && o > n_outer / 2)
+      o += D - n_outer;  // |ky| <= n_outer / 2
+  }
   float2* col = data + s * C + (long long)o * OUTER + tile * TXC + threadIdx.x % TXC;
-  using TS = TileSteps<D, T>;
+  using TS = TileSteps<D, T, T == 512>;
   float2 pts[TS::NPTS];
   TS::for_each_input([&](int n, int i) { pts[i] = col[n * LINE]; });
-  fill_twiddles<D>(tw, threadIdx.x, T);
+  fill_twiddles<D>(tw, threadIdx.x, tile_threads<T>());
   __syncthreads();
   TS::a(buf, tw, [&](int, int, int i) { return make_float2(pts[i].x, -pts[i].y); });
   __syncthreads();
@@ -1506,7 +1669,7 @@ template <int D>
 __device__ __forceinline__ void zg_tables(float2* s2)
 {
   using P = ZGPlan<D>;
-  fill_twiddles<P::L>(s2 + P::OFF_TW, threadIdx.x, TILE_THREADS_3);
+  fill_twiddles<P::L>(s2 + P::OFF_TW, threadIdx.x, blockDim.x);
   for (int k = threadIdx.x; k < P::L; k += TILE_THREADS_3) {
     float sn, cs;
     sincospif(2.0f * (float)k / (float)D, &sn, &cs);
@@ -1552,24 +1715,6 @@ __device__ void zg_c2r(const float2* __restrict__ spectrum, long long row0, floa
   __syncthreads();
 }
 
-// The per-cell test of find_HII_bubbles (find_HII_bubbles.c:342-428) on the
-// clamped values of one cell: FP32 with the FP64 decision within 4e-6 of
-// threshold, as in k_fft_z_threshold.
-template <bool SPIN, bool RECOMB>
-__device__ __forceinline__ bool zg_test(float dx, float stv, float nr, float xe, const RadiusParams& rp,
-                                        double pixel_volume, double eff, float* xpart)
-{
-  const float inv_dom = __fdividef(1.0f, 1.0f + dx);
-  const float lhs_f = stv * rp.kfc * inv_dom;
-  const float nf_f = 1.0f - xe;
-  const float rhs_f = nf_f * (1.0f + nr * inv_dom);
-  if (fabsf(lhs_f - rhs_f) > 4e-6f * fmaxf(lhs_f, rhs_f)) {
-    *xpart = nf_f - lhs_f;
-    return lhs_f > rhs_f;
-  }
-  return threshold_fp64(dx, stv, nr, xe, RECOMB, SPIN, rp.M_mean, rp.R_cubed, pixel_volume, eff, xpart);
-}
-
 // z-pass fused with the per-cell test for grids with a factor 3.  A block owns
 // 16 rows and ZTGen<D>::T threads, as many as the tile engine's steps keep busy.
 // The rows of each (radius, field) spectrum arrive through a ring of ZT_STAGES
@@ -1609,7 +1754,7 @@ __global__ void __launch_bounds__(ZTGen<D>::T, 2)
   using TS = TileSteps<P::L, P::T>;
   constexpr int L = P::L, H = P::H, HP = P::HP, RP = P::RP, NOUT = TS::NOUT;
   constexpr int G = 3 + (SPIN ? 1 : 0) + (RECOMB ? 1 : 0);
-  constexpr int IXE = 3, INR = SPIN ? 4 : 3;
+  static_assert(2 * NOUT <= 32, "cells per thread");
   extern __shared__ __align__(128) unsigned char zgsm[];
   float2* s2 = reinterpret_cast<float2*>(zgsm);
   const float2 *tw = s2 + P::OFF_TW, *post = s2 + P::OFF_POST;
@@ -1667,126 +1812,56 @@ __global__ void __launch_bounds__(ZTGen<D>::T, 2)
       issue(it + ZT_STAGES);
     }
   };
-  // this thread's cells: row t, z = 2 m + {0, 1}; the state of a pair in the
-  // halves of a register (ST_* bits, radius index from bit ST_RB_SHIFT on)
+  // this thread's cells: row t, z = 2 m + {0, 1}
   const int t = threadIdx.x % TXC;
   const long long cell0 = (row0 + t) * D;
-  unsigned st[NOUT];
+  auto cell = [&](int c) { return cell0 + 2 * TS::out_point(c >> 1) + (c & 1); };
+  CellState<NOUT> st;
+  st.clear();
 #pragma unroll
-  for (int i = 0; i < NOUT; i++) {
-    const int m = TS::out_point(i);
-    st[i] = 0;
-    if (m >= 0) {
-      const float2 x0 = *reinterpret_cast<const float2*>(a.xH + cell0 + 2 * m);
-      const float2 z0 = *reinterpret_cast<const float2*>(a.z_at_ion + cell0 + 2 * m);
-      st[i] = ((x0.x > REL_TOL_F ? ST_XHIGH : 0u) | (x0.x < REL_TOL_F ? ST_XLOW : 0u) | (z0.x < 0 ? ST_ZUNSET : 0u)) |
-              ((x0.y > REL_TOL_F ? ST_XHIGH : 0u) | (x0.y < REL_TOL_F ? ST_XLOW : 0u) | (z0.y < 0 ? ST_ZUNSET : 0u)) << 16;
-    }
-  }
+  for (int i = 0; i < NOUT; i++)
+    if (TS::out_point(i) >= 0)
+      st.start(i, *reinterpret_cast<const float2*>(a.xH + cell(2 * i)),
+               *reinterpret_cast<const float2*>(a.z_at_ion + cell(2 * i)));
   const bool need_ws = a.uvb || RECOMB;
   int it = 0;
-  for (int r = 0; r < a.n_r; r++) {
-    const RadiusParams rp = a.rp[r];
-    const bool direct = rp.last != 0;
+  for (int r = 0; r < a.n_f; r++) {
     float2 f[G][NOUT];
-    if (!direct) {
 #pragma unroll
-      for (int j = 0; j < G - 1; j++)
-        c2r(it++, f[j < 2 ? j : j + 1], true);
-    } else {
+    for (int j = 0; j < G - 1; j++)
+      c2r(it++, f[j < 2 ? j : j + 1], true);
+    const RadiusParams* rp = a.rp + r;
+    unsigned z;
+    unsigned first = st.ionise(ionised_cells<SPIN, RECOMB>(f, st.valid, rp, a.pixel_volume, a.eff), r, &z);
+    if (z) {
 #pragma unroll
-      for (int g = 0; g < G; g++)
-#pragma unroll
-        for (int i = 0; i < NOUT; i++) {
-          const int m = TS::out_point(i);
-          if (m >= 0)
-            f[g][i] = *reinterpret_cast<const float2*>(a.direct[g] + (row0 + t) * 2LL * H + 2 * m);
-        }
-    }
-    // bit c of first_ion / first_z: cell c's J_21 and Gamma12 resp.
-    // J_21_at_ionization are written below
-    unsigned first_ion = 0, first_z = 0;
-#pragma unroll
-    for (int c = 0; c < 2 * NOUT; c++) {
-      const int i = c >> 1, half = (c & 1) * 16;
-      const int m = TS::out_point(i);
-      if (m < 0)
-        continue;
-      const bool hi = c & 1;
-      const float dx = fmaxf(hi ? f[0][i].y : f[0][i].x, -1 + REL_TOL_F);
-      float stv = fmaxf(hi ? f[1][i].y : f[1][i].x, 0.0f);
-      if (stv < ABS_TOL_F)
-        stv = 0;
-      float nr = 0.0f, xe = 0.0f;
-      if constexpr (RECOMB) {
-        nr = fmaxf(hi ? f[INR][i].y : f[INR][i].x, 0.0f);
-        if (nr < ABS_TOL_F)
-          nr = 0;
-      }
-      if constexpr (SPIN) {
-        xe = fmaxf(hi ? f[IXE][i].y : f[IXE][i].x, 0.0f);
-        if (xe < ABS_TOL_F)
-          xe = 0;
-        xe = fminf(xe, 0.999f);
-      }
-      float xpart;
-      const bool ionised = zg_test<SPIN, RECOMB>(dx, stv, nr, xe, rp, a.pixel_volume, a.eff, &xpart);
-      const long long ir = cell0 + 2 * m + (hi ? 1 : 0);
-      unsigned s = st[i] >> half & 0xffffu;
-      const bool xr_high = !(s & ST_ION) && (s & ST_XHIGH);
-      bool xr_low = (s & ST_ION) || (s & ST_XLOW);
-      if (ionised) {
-        if (xr_high)
-          first_ion |= 1u << c;
-        s = (s & ((1u << ST_RB_SHIFT) - 1)) | ST_ION | ((unsigned)r << ST_RB_SHIFT);
-        xr_low = true;
-      } else if (rp.last && xr_high) {
-        const float xn = fminf(fmaxf(xpart, 0.0f), 1.0f);
-        a.xH[ir] = xn;
-        xr_low = xn < REL_TOL_F;
-      }
-      if (xr_low && (s & ST_ZUNSET)) {
-        a.z_at_ion[ir] = (float)a.redshift;
-        first_z |= 1u << c;
-        s &= ~ST_ZUNSET;
-      }
-      st[i] = (st[i] & ~(0xffffu << half)) | s << half;
+      for (int c = 0; c < 2 * NOUT; c++)
+        if (z >> c & 1u)
+          a.z_at_ion[cell(c)] = (float)a.redshift;
     }
     if (!need_ws)
-      first_ion = first_z = 0;
+      first = 0;
     if (!a.uvb)
-      first_z = 0;
-    if (!direct) {
-      const bool any = __syncthreads_or((first_ion | first_z) != 0);
-      c2r(it++, f[2], any);
-    }
-#pragma unroll
-    for (int c = 0; c < 2 * NOUT; c++) {
-      if (!((first_ion | first_z) >> c & 1u))
-        continue;
-      const int i = c >> 1;
-      const long long ir = cell0 + 2 * TS::out_point(i) + (c & 1);
-      float ws = fmaxf((c & 1) ? f[2][i].y : f[2][i].x, 0.0f);
-      if (ws < ABS_TOL_F)
-        ws = 0;
-      const float J21_aux = a.uvb ? ws * rp.kj : 0.0f;
-      if (first_ion >> c & 1u) {
-        if (a.uvb)
-          a.J21[ir] = J21_aux;
-        if (RECOMB)
-          a.Gamma12[ir] = ws * rp.kg;
-      }
-      if (first_z >> c & 1u)
-        a.J21_at_ion[ir] = J21_aux * a.gamma_halo_bias;
-    }
+      z = 0;
+    const bool any = __syncthreads_or((first | z) != 0);
+    c2r(it++, f[2], any);
+    if (first | z)
+      store_first<RECOMB>(a, rp, first, z, f[2], cell);
   }
 #pragma unroll
   for (int c = 0; c < 2 * NOUT; c++) {
-    const unsigned s = st[c >> 1] >> (c & 1) * 16 & 0xffffu;
-    if (s & ST_ION) {
-      const long long ir = cell0 + 2 * TS::out_point(c >> 1) + (c & 1);
-      a.xH[ir] = 0.0f;
-      a.r_bubble[ir] = (float)a.rp[s >> ST_RB_SHIFT].R;
+    if (st.ion >> c & 1u) {
+      a.xH[cell(c)] = 0.0f;
+      a.r_bubble[cell(c)] = (float)a.rp[st.radius(c)].R;
+    }
+  }
+  if (a.n_r > a.n_f) {
+#pragma unroll 2
+    for (int c = 0; c < 2 * NOUT; c++) {
+      if (!(st.valid >> c & 1u))
+        continue;
+      const long long ir = cell(c);
+      last_radius_cell<SPIN, RECOMB>(a, st, c, a.n_f, (row0 + t) * 2LL * H + (ir - cell0), ir);
     }
   }
 }
