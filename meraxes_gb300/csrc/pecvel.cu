@@ -12,8 +12,8 @@
 //                    0.2 H; modes 2-3: optical-depth form
 //                    (1 - exp(-tau / |dv/dx / H + 1|)) 1000 (T_S - T_CMB) / (1+z);
 //   k_rsd_columns    mode 3: the line-of-sight remap along z of the reference's
-//                    50 sub-cells per cell, a thread per cell (FP64 positions
-//                    and sums, order-independent deposits).
+//                    50 sub-cells per cell, a thread per cell (fixed point,
+//                    order-independent deposits).
 #include <algorithm>
 #include <cmath>
 
@@ -78,45 +78,112 @@ __global__ void k_vel_grad_k(float2* spec, int H, long long C, Scale2 inv_n, flo
   }
 }
 
-// 1 - exp(-x).  Optical depths are small: below 1/32 nine terms of the series
-// reach FP64 rounding (x^9 / 9! < 1e-19 of x) without the cancellation.
-__device__ __forceinline__ double one_minus_exp(double x)
+// An unevaluated sum of two floats, |lo| at most half an ulp of hi: about 2^-44
+// of the value, twenty bits beyond the float results of this file, on the FP32
+// pipe (64 times the FP64 rate).
+struct Pair
 {
-  if (!(fabs(x) < 0.03125))
-    return 1. - exp(-x);
-  double s = 1.0 - x * (1.0 / 9);
-  s = 1.0 - x * (1.0 / 8) * s;
-  s = 1.0 - x * (1.0 / 7) * s;
-  s = 1.0 - x * (1.0 / 6) * s;
-  s = 1.0 - x * (1.0 / 5) * s;
-  s = 1.0 - x * (1.0 / 4) * s;
-  s = 1.0 - x * (1.0 / 3) * s;
-  s = 1.0 - x * (1.0 / 2) * s;
-  return x * s;
+  float hi, lo;
+};
+__device__ __forceinline__ Pair fast_two_sum(float a, float b)  // |a| >= |b|
+{
+  const float s = __fadd_rn(a, b);
+  return { s, __fsub_rn(b, __fsub_rn(s, a)) };
+}
+__device__ __forceinline__ Pair two_sum(float a, float b)
+{
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return { s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t)) };
+}
+__device__ __forceinline__ Pair mul(Pair a, Pair b)
+{
+  const float p = __fmul_rn(a.hi, b.hi);
+  const float e = __fmaf_rn(a.hi, b.hi, -p) + (__fmul_rn(a.hi, b.lo) + __fmul_rn(a.lo, b.hi));
+  return fast_two_sum(p, e);
+}
+// a / b for a float a
+__device__ __forceinline__ Pair div(float a, Pair b)
+{
+  const float r = __fdividef(1.0f, b.hi), q = __fmul_rn(a, r);
+  const float rest = __fmaf_rn(-q, b.hi, a) - __fmul_rn(q, b.lo);
+  return fast_two_sum(q, __fmul_rn(rest, r));
 }
 
-// FP64 per cell, like the reference, with the constants' quotients taken once
-// on the host (FP64 issue bounds the kernel; 1.97 ms at 256^3 with a quotient
-// each).
+// x (1 - x/2 + x^2/6 - ...) = 1 - exp(-x) for |x| < 1/8: 1 - x/2 in pairs, the
+// rest (below 2^-8, the last term left out below 2^-36) in float
+constexpr float SMALL_TAU = 0.125f;
+__device__ __forceinline__ Pair one_minus_exp_small(Pair x)
+{
+  float s = 1.0f / 40320.0f;
+  s = fmaf(-s, x.hi, 1.0f / 5040.0f);
+  s = fmaf(-s, x.hi, 1.0f / 720.0f);
+  s = fmaf(-s, x.hi, 1.0f / 120.0f);
+  s = fmaf(-s, x.hi, 1.0f / 24.0f);
+  s = fmaf(-s, x.hi, 1.0f / 6.0f);
+  const Pair p = fast_two_sum(1.0f, -0.5f * x.hi);
+  return mul(x, fast_two_sum(p.hi, p.lo + fmaf(s * x.hi, x.hi, -0.5f * x.lo)));
+}
+
+// The cells of BrightnessTemperature.c:219-320.  The reference works in FP64;
+// here pairs of floats carry the same sums to twenty bits beyond the float
+// result, and cells outside their range (a gradient near -H, optical depths of
+// 1/8 and more, values beyond 1e15, infinities, NaN) take the FP64 form.  In
+// FP64 throughout, its issue rate bound the pass: 1.97 ms at 256^3 with the
+// reference's quotients, 1.31 ms with one.
+__device__ __noinline__ float pecvel_cell_fp64(const PecvelArgs& a, float dT, float grad, float TS)
+{
+  const double g = (double)grad;
+  if (a.mode == 1) {
+    double dvdx = g;
+    if (fabs(dvdx) > a.max_v_deriv)
+      dvdx = dvdx < 0 ? -a.max_v_deriv : a.max_v_deriv;
+    return (float)((double)dT / (dvdx * a.inv_H + 1.0));
+  }
+  const double gc = fabs(g * a.inv_H + 1.0);
+  const double scale = ((double)TS - a.T_rad) * a.mK;
+  if (gc < FRACT_FLOAT_ERR_D)
+    return (float)scale;
+  return (float)((1. - exp(-(double)dT / gc)) * scale);
+}
+
 __global__ void k_pecvel_cells(PecvelArgs a, int D, int H, long long N)
 {
+  // 1/H is 1e17 s and more: powers of two keep the pairs' products in range
+  const Pair invH = { (float)(a.inv_H * 0x1p-60), (float)(a.inv_H * 0x1p-60 - (double)(float)(a.inv_H * 0x1p-60)) };
+  const Pair T_rad = { (float)a.T_rad, (float)(a.T_rad - (double)(float)a.T_rad) };
+  const Pair mK = { (float)a.mK, (float)(a.mK - (double)(float)a.mK) };
+  const float cap = (float)(a.max_v_deriv * 0x1p60);
+  // 1 + dv/dx / H at the caps
+  const double up = 1.0 + a.max_v_deriv * a.inv_H, down = 1.0 - a.max_v_deriv * a.inv_H;
+  const Pair cap_up = { (float)up, (float)(up - (double)(float)up) };
+  const Pair cap_down = { (float)down, (float)(down - (double)(float)down) };
   for (long long ir = blockIdx.x * (long long)blockDim.x + threadIdx.x; ir < N; ir += (long long)gridDim.x * blockDim.x) {
     const long long row = row_of(ir, D);
-    const long long ip = row * 2LL * H + (ir - row * D);
-    const double g = (double)a.grad[ip];
+    const float grad = a.grad[row * 2LL * H + (ir - row * D)], dT = a.delta_T[ir];
+    const float TS = a.mode == 1 ? 0.0f : a.TS[ir];
+    const float g = grad * 0x1p60f;
+    // 1 + dv/dx / H
+    const float q = __fmul_rn(g, invH.hi);
+    const Pair t = two_sum(1.0f, q);
+    const Pair one_g = fast_two_sum(t.hi, t.lo + (__fmaf_rn(g, invH.hi, -q) + __fmul_rn(g, invH.lo)));
+    float out;
+    bool good;
     if (a.mode == 1) {
-      double dvdx = g;
-      if (fabs(dvdx) > a.max_v_deriv)
-        dvdx = dvdx < 0 ? -a.max_v_deriv : a.max_v_deriv;
-      a.delta_T[ir] = (float)((double)a.delta_T[ir] / (dvdx * a.inv_H + 1.0));
+      // capped at +- max_v_deriv; FP64 decides near the cap
+      const Pair r = div(dT, fabsf(g) > cap ? (g < 0.0f ? cap_down : cap_up) : one_g);
+      out = r.hi + r.lo;
+      good = fabsf(fabsf(g) - cap) > 1e-5f * cap && fabsf(dT) < 1e15f && fabsf(dT) > 1e-15f;
     } else {
-      const double gc = fabs(g * a.inv_H + 1.0);
-      const double scale = ((double)a.TS[ir] - a.T_rad) * a.mK;
-      if (gc < FRACT_FLOAT_ERR_D)
-        a.delta_T[ir] = (float)scale;
-      else
-        a.delta_T[ir] = (float)(one_minus_exp((double)a.delta_T[ir] / gc) * scale);
+      const Pair gc = one_g.hi < 0.0f ? Pair{ -one_g.hi, -one_g.lo } : one_g;
+      const Pair x = div(dT, gc);
+      const Pair d = two_sum(TS, -T_rad.hi);
+      const Pair scale = mul(fast_two_sum(d.hi, d.lo - T_rad.lo), mK);
+      const Pair r = mul(one_minus_exp_small(x), scale);
+      out = r.hi + r.lo;
+      good = gc.hi > 1e-4f && gc.hi < 1e6f && fabsf(x.hi) < SMALL_TAU && (fabsf(dT) > 1e-15f || dT == 0.0f) &&
+             fabsf(TS) < 1e15f;
     }
+    a.delta_T[ir] = good ? out : pecvel_cell_fp64(a, dT, grad, TS);
   }
 }
 
@@ -227,71 +294,76 @@ __device__ __noinline__ void rsd_column_sequential(const RsdArgs& a, long long c
 // an arithmetic series: n1 whole sub-cells and n2 - n1 partial ones.  A half
 // needs one such sum per boundary that it crosses (one or two) instead of 25
 // positions with three FP64 quotients each, and every cell is a thread of its
-// own.  Positions, sums and deposits are FP64; n1 and n2 may come from FP32,
-// because the series is continuous where they step (a count off by one within
-// rounding of a step moves 1e-6 of a sub-cell).
+// own.
 //
-// Deposits of different source cells meet in shared memory as 64-bit fixed
-// point (2^-50 of the column's largest source), so that the result does not
-// depend on their order.  D <= 2048 sources of 2^50 stay below 2^63.
+// Everything is fixed point: 100 x position in units of 2^-40 cells (in which
+// the sub-cells' offsets and widths are whole), sub-cells to 2^-(33 - log2 D) and
+// 24-bit sources, relative to the column's largest.  The sums are exact but for
+// the last of these roundings (1e-9 of a source at 256 cells), a column's
+// deposits stay below 2^63, and the result does not depend on their order.  n1
+// and n2 may come from FP32, because the series is continuous where they step (a
+// count off by one within rounding of a step moves 1e-6 of a sub-cell).
 // A column with an infinite source or a displacement of RSD_FAR cells or more
 // (or NaN) takes the sequential routine.
 //
-// Bound by FP64 issue (about 50 operations per cell; 2 lanes per clock and
-// SM).  One thread per column with the sequential loop took 88.1 ms at 256^3.
+// Bound by integer issue and shared-memory atomics.  At 256^3: one thread per
+// column with the sequential loop 88.1 ms; the series in FP64 2.1 ms.
 constexpr int RSD_THREADS = 256;
 constexpr int RSD_CELLS = 1024;   // cells of a block: whole columns, at least one
 constexpr double RSD_FAR = 4096.0;
+constexpr long long RSD_ONE = 1LL << 40, RSD_CELL = 100 * RSD_ONE;
 
-struct RsdSeries
+// floor(x / RSD_CELL)
+__device__ __forceinline__ int rsd_cell_of(long long x)
 {
-  double lo, step;  // lowest lower edge [cells], |B|
-  float inv_step;
-  __device__ __forceinline__ RsdSeries(double lo0, double B)
-  {
-    constexpr int n = RSD_STEPS / 2;
-    lo = B < 0 ? lo0 + B * ((n - 1) * (1.0 / RSD_STEPS)) : lo0;
-    step = fabs(B);
-    inv_step = __fdividef(1.0f, fmaxf((float)step, 1e-20f));
-  }
-  // sub-cells below boundary b
-  __device__ __forceinline__ double below(int b) const
-  {
-    constexpr float n = RSD_STEPS / 2;
-    const double U = ((double)b - lo) * (double)RSD_STEPS;
-    const float u = (float)U;
-    const int n1 = (int)fminf(fmaxf(floorf((u - 1.0f) * inv_step) + 1.0f, 0.0f), n);
-    const int n2 = max(n1, (int)fminf(fmaxf(ceilf(u * inv_step), 0.0f), n));
-    const int m = n2 - n1;
-    return (double)n1 + ((double)m * U - (double)((n1 + n2 - 1) * m / 2) * step);
-  }
-};
+  int c = (int)floorf((float)x * (float)(1.0 / (double)RSD_CELL));
+  while (x < c * RSD_CELL)
+    c--;
+  while (x >= (c + 1) * RSD_CELL)
+    c++;
+  return c;
+}
 
-__device__ __forceinline__ void rsd_half(unsigned long long* acc, int kk, int D, double lo0, double B, double q)
+// The 25 sub-cells of half a cell: lower edge of the first (100 x cells, 2^-40)
+// and B (2^-40); source mantissa, right shift, and bits per sub-cell.
+__device__ __forceinline__ void rsd_half(unsigned long long* acc, int kk, int D, long long lo0, long long B, int mant,
+                                         int shift, int bits)
 {
-  constexpr double n = RSD_STEPS / 2;
-  const RsdSeries s(lo0, B);
-  const int first = (int)floor(s.lo);
-  const int last = (int)ceil(s.lo + s.step * ((n - 1) / RSD_STEPS) + 1.0 / RSD_STEPS) - 1;
-  double done = 0.0;
+  constexpr int n = RSD_STEPS / 2;
+  const long long step = B < 0 ? -B : B;
+  const long long lo = B < 0 ? lo0 + 2 * (n - 1) * B : lo0;
+  const int first = rsd_cell_of(lo), last = rsd_cell_of(lo + 2 * (n - 1) * step + 2 * RSD_ONE - 1);
   int t = kk + first;
   if (t < 0 || t >= D)
     t = wrap(t, D);
-  for (int c = first; c < last; c++) {
-    const double m = s.below(c + 1);
-    atomicAdd(acc + t, (unsigned long long)__double2ll_rn((m - done) * q));
-    done = m;
-    t = t + 1 == D ? 0 : t + 1;
+  auto add = [&](int mass) { atomicAdd(acc + t, (unsigned long long)(((long long)mass * mant) >> shift)); };
+  int done = 0;
+  if (first < last) {
+    const float inv_step = __fdividef(1.0f, fmaxf((float)step * 0x1p-40f, 1e-20f));
+    for (int c = first; c < last; c++) {
+      // sub-cells below the boundary c + 1
+      const long long U = ((c + 1) * RSD_CELL - lo) >> 1;
+      const float u = (float)U * 0x1p-40f;
+      const int n1 = (int)fminf(fmaxf(floorf((u - 1.0f) * inv_step) + 1.0f, 0.0f), (float)n);
+      const int n2 = max(n1, (int)fminf(fmaxf(ceilf(u * inv_step), 0.0f), (float)n));
+      const int m = n2 - n1;
+      const long long below = n1 * RSD_ONE + (m * U - ((n1 + n2 - 1) * m / 2) * step);
+      const int mass = (int)((below + (1LL << (39 - bits))) >> (40 - bits));
+      add(mass - done);
+      done = mass;
+      t = t + 1 == D ? 0 : t + 1;
+    }
   }
-  atomicAdd(acc + t, (unsigned long long)__double2ll_rn((n - done) * q));
+  add((n << bits) - done);
 }
 
-// Block: `cols` whole columns.  Shared memory: displacement [cells] and
-// deposit of each cell.
-__global__ void __launch_bounds__(RSD_THREADS) k_rsd_columns(const __grid_constant__ RsdArgs a, int D, int H, int cols)
+// Block: `cols` whole columns.  Shared memory: displacement (2^-40 cells) and
+// deposit of each cell; `bits` per sub-cell.
+__global__ void __launch_bounds__(RSD_THREADS)
+  k_rsd_columns(const __grid_constant__ RsdArgs a, int D, int H, int cols, int bits)
 {
-  extern __shared__ double rsd_sm[];
-  double* disp = rsd_sm;
+  extern __shared__ long long rsd_sm[];
+  long long* disp = rsd_sm;
   unsigned long long* acc = reinterpret_cast<unsigned long long*>(rsd_sm + cols * D);
   int* top = reinterpret_cast<int*>(acc + cols * D);  // per column: bits of the largest |source|
   int* bad = top + cols;
@@ -309,38 +381,41 @@ __global__ void __launch_bounds__(RSD_THREADS) k_rsd_columns(const __grid_consta
   for (int i = threadIdx.x; i < cells; i += RSD_THREADS) {
     const int c = i / D;
     const double d = (double)__fdiv_rn(a.vel[(col0 + c) * 2LL * H + (i - c * D)], a.H_z) * a.inv_cell;
-    disp[i] = d;
+    const bool near = fabs(d) < RSD_FAR;
+    disp[i] = near ? __double2ll_rn(d * (double)RSD_ONE) : 0;
     acc[i] = 0;
-    const int bits = __float_as_int(fabsf(source(i)));
-    if (bits)
-      atomicMax(top + c, bits);
-    if (!(fabs(d) < RSD_FAR))
+    const int top_bits = __float_as_int(fabsf(source(i)));
+    if (top_bits)
+      atomicMax(top + c, top_bits);
+    if (!near)
       bad[c] = 1;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < cells; i += RSD_THREADS) {
     const int c = i / D, kk = i - c * D;
-    const float dT = source(i);
-    if (dT == 0.0f || bad[c] || top[c] >= 0x7f800000)
+    const int b = __float_as_int(source(i));
+    if (b << 1 == 0 || bad[c] || top[c] >= 0x7f800000)
       continue;
-    // |largest source| * 2^shift in [2^49, 2^50)
-    const int shift = 49 - ((top[c] >> 23) - 127);
-    const double q = (double)dT * __hiloint2double((1023 + shift) << 20, 0) * (1.0 / RSD_STEPS);
-    const double* d = disp + c * D;
-    const double here = d[kk], lo_d = here - d[kk == 0 ? D - 1 : kk - 1], hi_d = d[kk == D - 1 ? 0 : kk + 1] - here;
+    // a source is at least 1e-7: a normal float
+    const int mant = ((b & 0x7fffff) | 0x800000) * (b < 0 ? -1 : 1);
+    const int shift = min((top[c] >> 23) - (b >> 23 & 0xff), 62);
+    const long long* d = disp + c * D;
+    const long long here = d[kk], lo_d = here - d[kk == 0 ? D - 1 : kk - 1], hi_d = d[kk == D - 1 ? 0 : kk + 1] - here;
     // first half: from the lower neighbour's velocity at x = -1/2 to this
     // cell's at 1/2 (sub-cell centres 0.01 ... 0.49); second half: from this
     // cell's at 1/2 to the upper neighbour's at 3/2 (0.51 ... 0.99)
-    rsd_half(acc + c * D, kk, D, here - 0.49 * lo_d, 1.0 + lo_d, q);
-    rsd_half(acc + c * D, kk, D, 0.5 + here + 0.01 * hi_d, 1.0 + hi_d, q);
+    rsd_half(acc + c * D, kk, D, 100 * here - 49 * lo_d, RSD_ONE + lo_d, mant, shift, bits);
+    rsd_half(acc + c * D, kk, D, 50 * RSD_ONE + 100 * here + hi_d, RSD_ONE + hi_d, mant, shift, bits);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < cells; i += RSD_THREADS) {
     const int c = i / D;
     if (bad[c] || top[c] >= 0x7f800000)
       continue;
-    const int shift = 49 - ((top[c] >> 23) - 127);
-    a.delta_T_out[col0 * D + i] = (float)((double)(long long)acc[i] * __hiloint2double((1023 - shift) << 20, 0));
+    // 2^(e - 23 - bits) / 50 per unit, e the exponent of the largest source
+    const int e = (top[c] >> 23) - 127 - 23 - bits;
+    a.delta_T_out[col0 * D + i] =
+      (float)((double)(long long)acc[i] * (__hiloint2double((1023 + e) << 20, 0) * (1.0 / RSD_STEPS)));
   }
   for (int c = threadIdx.x; c < nc; c += RSD_THREADS)
     if (bad[c] || top[c] >= 0x7f800000) {
@@ -385,7 +460,11 @@ void launch_rsd(const RsdArgs& a, const GridDims& gd, cudaStream_t s)
   const long long columns = (long long)gd.D * gd.D;
   const int cols = (int)std::max(1, RSD_CELLS / gd.D);
   const size_t smem = (size_t)cols * (gd.D * (sizeof(double) + sizeof(unsigned long long)) + 2 * sizeof(int));
-  k_rsd_columns<<<(unsigned)((columns + cols - 1) / cols), RSD_THREADS, smem, s>>>(a, gd.D, gd.H, cols);
+  int log2_D = 1;
+  while ((1 << log2_D) < gd.D)
+    log2_D++;
+  k_rsd_columns<<<(unsigned)((columns + cols - 1) / cols), RSD_THREADS, smem, s>>>(a, gd.D, gd.H, cols,
+                                                                                    std::min(25, 33 - log2_D));
   pv_launches++;
 }
 

@@ -91,3 +91,57 @@ def test_remap_matches_subcells(D, cells, far):
         err[1, 2] = 0.0
     assert err.max() < 4e-6
     assert abs(mean - dT3.astype(np.float64).mean()) <= 1e-9 * np.abs(dT3).mean()
+
+
+# Modes 1 and 2 per cell against FP64 on one velocity mode (whose derivative is
+# known), from below to above the cap of 0.2 H and for optical depths from 1e-6
+# to 5 (the pairs of floats up to 1/8, FP64 beyond).  The FP32 transform gives
+# dv/dx to a few 1e-7 of its largest value; divided by 1 + dv/dx / H >= 1/2:
+# 3e-6 relative.  Cells within 1e-5 of the cap may take either side: 1e-5.
+@pytest.mark.parametrize("mode,slope", [(1, 0.1), (1, 0.5), (2, 0.0), (2, 0.5)])
+def test_cells_match_fp64(mode, slope):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import dataclasses
+
+    from meraxes_gb300.api import ReionGridStep
+    from meraxes_gb300.params import workload
+
+    D = 32
+    w = workload("full_256", D)
+    p = dataclasses.replace(w.params, flag_pecvel=mode)
+    z = float(np.float32(w.redshifts[1]))
+    H = 3.2407789e-18 * p.hubble_h * np.sqrt(p.omega_m * (1.0 + z) ** 3 + p.omega_lambda)
+    k = 2.0 * np.pi / p.box_size  # velocity_gradient's k, times h
+    phase = 2.0 * np.pi * np.arange(D) / D
+    rng = np.random.default_rng(5)
+    conv = (1.0 + z) ** 2 * (1e5 / 3.086e24)
+    shape = (D, D, 2 * (D // 2 + 1))
+    vel, deltax = np.zeros(shape, np.float32), np.zeros(shape, np.float32)
+    vel[:, :, :D] = slope * H / (k * p.hubble_h) * np.sin(phase) / conv
+    deltax[:, :, :D] = rng.uniform(-0.9, 3.0, (D, D, D))
+    xH = rng.choice([0.0, 1e-4, 0.3, 1.0], (D, D, D)).astype(np.float32)
+    TS = (10.0 ** rng.uniform(-0.7, 3.0, (D, D, D))).astype(np.float32)
+    g = {"deltax": deltax, "xH": xH, "TS_box": TS, "vel": vel, "delta_T": np.zeros((D, D, D), np.float32)}
+    g = {n: torch.from_numpy(v).cuda() for n, v in g.items()}
+    ReionGridStep(p, w.redshifts).ComputeBrightnessTemperatureBox(1, g)
+    got = g["delta_T"].cpu().numpy().astype(np.float64)
+    h2 = p.hubble_h ** 2
+    factor = 27 * (p.omega_m * p.baryon_frac * h2 / 0.023) * np.sqrt(0.15 / (p.omega_m * h2) * (1 + z) / 10)
+    T_cmb, ts = 2.728 * (1 + z), TS.astype(np.float64)
+    dT = factor * xH.astype(np.float64) * (1 + deltax[:, :, :D].astype(np.float64))
+    grad = slope * np.cos(phase)
+    if mode == 1:
+        want = dT * (1 - T_cmb / ts) / (np.clip(grad, -0.2, 0.2) + 1)
+    else:
+        tau = dT * (1 + z) / (1000 * ts) / np.abs(grad + 1)
+        assert tau.max() > 0.5 and tau[tau > 0].min() < 1e-5
+        want = -np.expm1(-tau) * 1000 * (ts - T_cmb) / (1 + z)
+    # T_S - T_CMB cancels near equality: its float rounding is on T_S
+    scale = np.abs(want) + 1e-7 * np.abs(dT) * T_cmb / np.abs(ts)
+    live = scale > 0
+    assert np.all(got[~live] == 0)
+    err = np.abs(got - want)[live] / scale[live]
+    near = np.abs(ts - T_cmb) < 0.05 * T_cmb
+    assert err[~near[live]].max() < (1e-5 if mode == 1 else 3e-6)
