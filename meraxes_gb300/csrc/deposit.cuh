@@ -27,23 +27,23 @@ struct DepositArgs
   unsigned* keys;        // [n] sorted
   int* idx_in;           // [n]
   int* idx;              // [n] sorted
-  float* buf_stars;      // REAL scratch, zeroed by launch_deposit
-  float* buf_wsfr;
-  float* buf_sfr;
   unsigned* err;         // bit 4: a galaxy below the box
   float* stars;          // PADDED outputs
   float* weighted_sfr;
   float* sfr;
-  float* sfr_hist0;      // newest history slice, or NULL
+  float* sfr_hist0;      // SFR history, newest slice first, or NULL
+  int n_hist;            // its slices
+  int shift_history;     // move them one snapshot back first
 };
 
 constexpr unsigned DEPOSIT_ERR_BELOW_BOX = 4u;
 
 // CUB temporary storage for sorting n galaxies (bytes)
 size_t deposit_sort_bytes(int n);
-// Zeroes the REAL scratch, sorts, sums and writes the padded grids.
+// Clears the padded grids and shifts the history on `side` (forked from and
+// joined to s by the two events), sorts on s, sums and writes.
 cudaError_t launch_deposit(const DepositArgs& a, void* sort_tmp, size_t sort_bytes, const GridDims& gd,
-                           cudaStream_t s);
+                           cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
 // sm = {m0, a, b, c, d} of the Sobacchi & Mesinger (2013) fit
 void launch_Mvir_crit(double redshift, const double sm[5], double hubble_h, const float* J21_at_ion,
                       const float* z_at_ion, float* out, const GridDims& gd, cudaStream_t s);

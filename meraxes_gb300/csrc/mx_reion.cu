@@ -1473,7 +1473,7 @@ static int run_power_spectrum(mx_ctx* c, const float* dT, float* ps_k, float* ps
   }
   {
     Prof pr(c, "k_ps_field", 8.0 * (double)gd.N, s);
-    launch_ps_field(dT, mean_sum, a.volume, gd, field, s);
+    launch_ps_field(dT, mean_sum, gd, field, s);
   }
   {
     MX_CUFFT(cufftSetStream(c->r2c_plan, s));
@@ -1489,9 +1489,11 @@ static int run_power_spectrum(mx_ctx* c, const float* dT, float* ps_k, float* ps
   }
   MX_CUDA(cudaMemcpyAsync(c->h_ps_sums, c->d_ps_sums, sizeof(double) * 3 * a.nb, cudaMemcpyDeviceToHost, s));
   MX_CUDA(cudaStreamSynchronize(s));
-  // :228-240
+  // :228-240; the field's V / N squared, over 2 pi^2 V
+  const double n_cells = (double)(float)(double)gd.N;
+  const double to_power = (double)a.volume / n_cells / n_cells / (2.0 * k::PI * k::PI);
   for (int i = 0; i < a.nb; i++) {
-    const double p_box = c->h_ps_sums[i], k_ave = c->h_ps_sums[a.nb + i], ct = c->h_ps_sums[2 * a.nb + i];
+    const double p_box = c->h_ps_sums[i] * to_power, k_ave = c->h_ps_sums[a.nb + i], ct = c->h_ps_sums[2 * a.nb + i];
     ps_k[i] = (float)(k_ave / ct);
     ps_data[i] = (float)(p_box / ct);
     ps_error[i] = (float)((p_box / ct) / std::sqrt(ct));
@@ -1547,7 +1549,7 @@ static double run_ps_loss(mx_ctx* c, const float* dT, int nbins, const float* ed
   double loss = 0.0;
   double coef[PS_MAX_BINS] = { 0 };
   for (int b = 0; b < nbins; b++) {
-    const double sum = c->h_ps_sums[b + 1], ct = c->h_ps_sums[2 * a.nb + b + 1];
+    const double sum = c->h_ps_sums[b + 1] / pdiv, ct = c->h_ps_sums[2 * a.nb + b + 1];
     const double pb = ct > 0 ? sum / ct : 0.0;
     if (P)
       P[b] = (float)pb;
@@ -1989,10 +1991,6 @@ static void run_deposit(mx_ctx* c, int snapshot, const mx_galaxies& gal, const G
   const bool spin = p.flag_spin_temp != 0;
   if (gd.N >= 0xffffffffLL)
     throw CudaError{ MX_ENOTSUP, "construct_baryon_grids: 32-bit cell keys hold grids below 2^32 - 1 cells" };
-  if (spin && shift_history && sfr_hist)
-    for (int k = c->n_hist - 2; k >= 0; k--)
-      MX_CUDA(cudaMemcpyAsync(sfr_hist + (size_t)(k + 1) * gd.P, sfr_hist + (size_t)k * gd.P, sizeof(float) * gd.P,
-                              cudaMemcpyDeviceToDevice, s));
   DepositArgs a{};
   a.n = (int)gal.n;
   a.pos = gal.pos;
@@ -2012,18 +2010,17 @@ static void run_deposit(mx_ctx* c, int snapshot, const mx_galaxies& gal, const G
   a.keys = gs.keys;
   a.idx_in = gs.idx_in;
   a.idx = gs.idx;
-  // REAL sums in unfiltered-spectrum scratch slots 0-2
-  a.buf_stars = reinterpret_cast<float*>(c->d_unf);
-  a.buf_wsfr = reinterpret_cast<float*>(c->d_unf + gd.C);
-  a.buf_sfr = reinterpret_cast<float*>(c->d_unf + 2 * gd.C);
   a.err = c->d_err;
   a.stars = stars;
   a.weighted_sfr = wsfr;
   a.sfr = sfr;
   a.sfr_hist0 = sfr_hist;
+  a.n_hist = c->n_hist;
+  a.shift_history = shift_history ? 1 : 0;
   {
-    Prof pr(c, "deposit", (double)gal.n * 44.0 + 4.0 * gd.P * (spin ? 5 : 2), s);
-    MX_CUDA(launch_deposit(a, gs.sort_tmp, gs.sort_bytes, gd, s));
+    const double slices = (spin ? 4 : 2) + (shift_history && sfr_hist ? 2.0 * (c->n_hist - 1) : 0.0);
+    Prof pr(c, "deposit", (double)gal.n * 44.0 + 4.0 * gd.P * slices, s);
+    MX_CUDA(launch_deposit(a, gs.sort_tmp, gs.sort_bytes, gd, s, c->aux_stream, c->ev_a, c->ev_b));
   }
   unsigned int errw = 0;
   MX_CUDA(cudaMemcpyAsync(&errw, c->d_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));

@@ -1,8 +1,8 @@
 // 21 cm power spectrum of delta_T: Compute_PS (ComputePowerSpectrum.c:44-255).
 //
 //   1. mean of delta_T (two-stage fixed-order FP64 sum);
-//   2. the field (delta_T / mean - 1) * V / N * mean into the padded layout,
-//      with the reference's double arithmetic per cell;
+//   2. the field delta_T - mean into the padded layout (its factor V / N is
+//      applied to the sums);
 //   3. R2C (cuFFT, in mx_reion.cu);
 //   4. the binned sums over the half spectrum: every mode (kx, ky, kz <= D/2)
 //      is counted once, |k| in float as the reference computes it, bins of
@@ -22,12 +22,22 @@ namespace {
 // per host thread: a call counts its own launches when contexts run concurrently
 thread_local int ps_launches = 0;
 
+// SUM_BATCH cells of a thread's stride are read together
+constexpr int SUM_BATCH = 8;
 __global__ void k_ps_sum(const float* __restrict__ dT, long long N, double* partials)
 {
   __shared__ double sh[RED_THREADS / 32];
   CSum sum;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
-    sum.add(dT[i]);
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < N; i0 += SUM_BATCH * stride) {
+    float v[SUM_BATCH];
+#pragma unroll
+    for (int u = 0; u < SUM_BATCH; u++)
+      v[u] = i0 + u * stride < N ? dT[i0 + u * stride] : 0.0f;
+#pragma unroll
+    for (int u = 0; u < SUM_BATCH; u++)
+      sum.add(v[u]);
+  }
   double acc = sum.value();
   for (int o = 16; o > 0; o >>= 1)
     acc += __shfl_down_sync(0xffffffffu, acc, o);
@@ -61,17 +71,18 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) k_ps_finalize(const double* __
     sums[v] = s;
 }
 
-// ComputePowerSpectrum.c:94-110
-__global__ void k_ps_field(const float* __restrict__ dT, const double* __restrict__ sum, double n_cells, float volume,
-                           float n_cells_f, int D, int H, long long N, float* __restrict__ out)
+// The field of ComputePowerSpectrum.c:94-110, (dT / ave - 1) V / N ave, without
+// its constant factor V / N (the binned sums take it squared, in FP64): dT - ave
+// with ave in two floats, so that the difference is rounded once.  In FP64 as
+// written, the quotient per cell bound the pass (507 us at 200^3).
+__global__ void k_ps_field(const float* __restrict__ dT, const double* __restrict__ sum, double n_cells, int D, int H,
+                           long long N, float* __restrict__ out)
 {
   const double ave = sum[0] / n_cells;
+  const float hi = (float)ave, lo = (float)(ave - (double)hi);
   for (long long ir = blockIdx.x * (long long)blockDim.x + threadIdx.x; ir < N; ir += (long long)gridDim.x * blockDim.x) {
     const long long row = row_of(ir, D);
-    const long long ip = row * 2LL * H + (ir - row * D);
-    float v = (float)(((double)dT[ir] / ave - 1) * (double)volume / (double)n_cells_f);
-    v = (float)((double)v * ave);
-    out[ip] = v;
+    out[row * 2LL * H + (ir - row * D)] = __fsub_rn(__fsub_rn(dT[ir], hi), lo);
   }
 }
 
@@ -80,80 +91,80 @@ __device__ __forceinline__ float kcomp_ps(int n, int D, float delta_k)
   return (n > D / 2) ? __fmul_rn((float)(n - D), delta_k) : __fmul_rn((float)n, delta_k);
 }
 
-// ComputePowerSpectrum.c:160-215
+// ComputePowerSpectrum.c:160-215: sums of k^3 |X|^2, |k| and the modes of each
+// bin; the constant 1 / (2 pi^2 V) is applied to the sums by the caller.  Bound
+// by FP64 issue, now nine operations per mode (with that quotient, the count and
+// the cube's square in FP64 per mode, 371 us at 200^3).
 __global__ void __launch_bounds__(RED_THREADS) k_ps_bin(PsArgs a)
 {
-  double hp[PS_MAX_BINS], hk[PS_MAX_BINS], hc[PS_MAX_BINS];
-  for (int b = 0; b < a.nb; b++)
-    hp[b] = hk[b] = hc[b] = 0.0;
+  double hp[PS_MAX_BINS], hk[PS_MAX_BINS];
+  int hc[PS_MAX_BINS];
+  for (int b = 0; b < a.nb; b++) {
+    hp[b] = hk[b] = 0.0;
+    hc[b] = 0;
+  }
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (RED_THREADS / 32);
   const int D = a.D, H = D / 2 + 1;
   const long long rows = (long long)D * D;
-  const double pdiv = 2.0 * 3.14159265358979323846 * 3.14159265358979323846 * (double)a.volume;
   for (long long row = blockIdx.x * (RED_THREADS / 32) + (threadIdx.x >> 5); row < rows; row += warps) {
-    const int nx = (int)(row / D), ny = (int)(row % D);
+    const int nx = (int)((unsigned)row / (unsigned)D), ny = (int)row - nx * D;
     const float kx = kcomp_ps(nx, D, a.delta_k), ky = kcomp_ps(ny, D, a.delta_k);
     // k_x*k_x + k_y*k_y + k_z*k_z in the reference's float operations (no
     // fused multiply-add)
     const float kxy = __fadd_rn(__fmul_rn(kx, kx), __fmul_rn(ky, ky));
     const float2* __restrict__ spec = a.spec + row * H;
-    int cur = -1;
-    double sp = 0.0, sk = 0.0, sc = 0.0;
+    int cur = 0, count = 0;  // |k| grows along a lane's modes, and so does its bin
+    double sp = 0.0, sk = 0.0;
+    auto flush = [&]() {
+      if (count) {
+        hp[cur] += sp;
+        hk[cur] += sk;
+        hc[cur] += count;
+      }
+      sp = sk = 0.0;
+      count = 0;
+    };
     for (int nz = lane; nz < H; nz += 32) {
       const float kz = __fmul_rn((float)nz, a.delta_k);
       // (float)sqrt((double)s) of the reference equals sqrtf(s): the double
       // square root of a float has enough bits that rounding it again to
       // float gives the correctly rounded float root
       const float kmag = sqrtf(__fadd_rn(kxy, __fmul_rn(kz, kz)));
-      int b = -1;
-      if (kmag < a.edges[a.nb]) {
-        b = 0;
-        while (!(kmag < a.edges[b + 1]))
-          b++;
+      if (!(kmag < a.edges[a.nb]))
+        break;
+      if (!(kmag < a.edges[cur + 1])) {
+        flush();
+        do
+          cur++;
+        while (!(kmag < a.edges[cur + 1]));
       }
-      if (b != cur) {
-        if (cur >= 0) {
-          hp[cur] += sp;
-          hk[cur] += sk;
-          hc[cur] += sc;
-        }
-        cur = b;
-        sp = sk = sc = 0.0;
-      }
-      if (b >= 0) {
-        const float2 X = spec[nz];
-        const double k = (double)kmag;
-        const double m2 = (double)X.x * (double)X.x + (double)X.y * (double)X.y;
-        sp += k * k * k * m2 / pdiv;
-        sk += k;
-        sc += 1.0;
-      }
+      const float2 X = spec[nz];
+      const double k = (double)kmag, x = (double)X.x, y = (double)X.y;
+      sp = fma(k * k * k, fma(x, x, y * y), sp);
+      sk += k;
+      count++;
     }
-    if (cur >= 0) {
-      hp[cur] += sp;
-      hk[cur] += sk;
-      hc[cur] += sc;
-    }
+    flush();
   }
-  // block reduction per bin, fixed order: lanes by shuffles, warps in order
-  __shared__ double sh[3][RED_THREADS / 32];
+  // block reduction in a fixed order: the threads' values of one quantity
+  // through shared memory, a warp per bin (eight values per lane, then a tree);
+  // a tree over every warp's lanes took as many FP64 additions as the modes
+  extern __shared__ double sh[];  // nb x RED_THREADS
   const int warp = threadIdx.x >> 5;
-  for (int b = 0; b < a.nb; b++) {
-    double v[3] = { hp[b], hk[b], hc[b] };
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      for (int o = 16; o > 0; o >>= 1)
-        v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-      if (lane == 0)
-        sh[q][warp] = v[q];
-    }
+  for (int q = 0; q < 3; q++) {
+    for (int b = 0; b < a.nb; b++)
+      sh[b * RED_THREADS + threadIdx.x] = q == 0 ? hp[b] : (q == 1 ? hk[b] : (double)hc[b]);
     __syncthreads();
-    if (threadIdx.x < 3) {
-      double s = 0.0;
+    for (int b = warp; b < a.nb; b += RED_THREADS / 32) {
+      double v = 0.0;
+#pragma unroll
       for (int w = 0; w < RED_THREADS / 32; w++)
-        s += sh[threadIdx.x][w];
-      a.partials[(long long)blockIdx.x * 3 * a.nb + threadIdx.x * a.nb + b] = s;
+        v += sh[b * RED_THREADS + w * 32 + lane];
+      for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0)
+        a.partials[(long long)blockIdx.x * 3 * a.nb + q * a.nb + b] = v;
     }
     __syncthreads();
   }
@@ -212,16 +223,17 @@ void launch_ps_mean(const float* dT, long long N, double* partials, double* sum,
   ps_launches += 2;
 }
 
-void launch_ps_field(const float* dT, const double* sum, float volume, const GridDims& gd, float* out, cudaStream_t s)
+void launch_ps_field(const float* dT, const double* sum, const GridDims& gd, float* out, cudaStream_t s)
 {
-  const double n = (double)gd.N;
-  k_ps_field<<<RED_BLOCKS, RED_THREADS, 0, s>>>(dT, sum, n, volume, (float)n, gd.D, gd.H, gd.N, out);
+  k_ps_field<<<RED_BLOCKS, RED_THREADS, 0, s>>>(dT, sum, (double)gd.N, gd.D, gd.H, gd.N, out);
   ps_launches++;
 }
 
 void launch_ps_bin(const PsArgs& a, double* sums, cudaStream_t s)
 {
-  k_ps_bin<<<RED_BLOCKS, RED_THREADS, 0, s>>>(a);
+  const size_t smem = sizeof(double) * RED_THREADS * (size_t)a.nb;
+  cudaFuncSetAttribute(k_ps_bin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_ps_bin<<<RED_BLOCKS, RED_THREADS, smem, s>>>(a);
   k_ps_finalize<<<(3 * a.nb + FIN_WARPS - 1) / FIN_WARPS, 32 * FIN_WARPS, 0, s>>>(a.partials, RED_BLOCKS, 3 * a.nb, sums);
   ps_launches += 2;
 }

@@ -17,11 +17,13 @@ struct PsArgs
   float edges[PS_MAX_BINS + 1];  // edges[0] = 0, edges[b + 1] = ceiling of bin b
   float delta_k;
   float volume;                // (box / h)^3 in Mpc^3, as float
-  double* partials;            // RED_BLOCKS x 3 x nb: sum P, sum |k|, count
+  double* partials;            // RED_BLOCKS x 3 x nb: sum k^3 |X|^2, sum |k|, count
 };
 
 void launch_ps_mean(const float* dT, long long N, double* partials, double* sum, cudaStream_t s);
-void launch_ps_field(const float* dT, const double* sum, float volume, const GridDims& gd, float* out, cudaStream_t s);
+// dT - mean (padded); the sum of dT over the cells in *sum (device)
+void launch_ps_field(const float* dT, const double* sum, const GridDims& gd, float* out, cudaStream_t s);
+// sums: k^3 |X|^2, |k| and modes per bin
 void launch_ps_bin(const PsArgs& a, double* sums, cudaStream_t s);
 // power-spectrum loss: f = dT * scale (padded), gradient spectrum (in place:
 // Y_k = coef[bin] k^3 X_k, doubled on the kz = 0, D/2 planes), REAL = padded * scale
