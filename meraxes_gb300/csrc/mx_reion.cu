@@ -63,6 +63,14 @@ int hw_threads()
 }
 }  // namespace
 
+// Spectra of one cuFFT C2R execution of the unfused path: small transforms are
+// launch-bound and leave the GPU idle one by one, while the work area grows with
+// the batch (a few times this size).  42 radii of 5 fields, one radius at a time
+// -> in groups: 0.98 -> 0.54 ms at 50^3, 2.6 -> 2.2 at 100^3; from 144^3 on a
+// radius fills the GPU (6.2 ms both ways) and the group is one.
+constexpr long long C2R_GROUP_BYTES = 64LL << 20;
+constexpr int C2R_GROUP_MAX = 16;
+
 struct mx_ctx
 {
   mx_params p;
@@ -181,6 +189,27 @@ struct mx_ctx
   void make_shell_map();
   cufftHandle c2r_plan(long long batch);
   void ensure_mirror();
+  // groups of `unit` spectra per cuFFT execution of the unfused path
+  int c2r_group(int unit) const
+  {
+    const long long fit = std::min(C2R_GROUP_BYTES / (8 * gd.C * unit), work_fields / unit);
+    return (int)std::max<long long>(1, std::min<long long>(fit, C2R_GROUP_MAX));
+  }
+  // The C2R plans of a step: plans allocate their work areas when created,
+  // which a capture does not allow.
+  void make_c2r_plans()
+  {
+    const bool spin = p.flag_spin_temp != 0;
+    if (!fused_fft) {
+      const int G = 3 + (spin ? 1 : 0) + (p.flag_recombinations ? 1 : 0);
+      c2r_plan(G);
+      c2r_plan((long long)G * c2r_group(G));
+      if (spin)
+        c2r_plan(c2r_group(1));
+    }
+    if (spin && (!fused_fft || p.flag_pecvel > 0))
+      c2r_plan(1);
+  }
 };
 
 // Records CUDA events around one kernel (or cuFFT execution) on its stream
@@ -507,6 +536,25 @@ static void run_xy(mx_ctx* c, const XPassArgs& xa, cudaStream_t s)
   launch_fft_y(c->gd.D, xa.out, xa.C, xa.n * xa.G, xa.bands, c->y_threads, s);
 }
 
+// In-place C2R of n groups of `unit` consecutive spectra (unfused path): full
+// executions of c2r_group(unit) groups, the rest one group at a time (so that a
+// context makes two plans, whatever the number of radii).
+static void run_c2r(mx_ctx* c, float2* work, int n, int unit, cudaStream_t s)
+{
+  const GridDims& gd = c->gd;
+  const double bytes = 8.0 * (double)gd.C + 4.0 * (double)gd.N;
+  const int group = c->c2r_group(unit);
+  for (int i = 0; i < n;) {
+    const int k = n - i >= group ? group : 1;
+    const cufftHandle plan = c->c2r_plan((long long)k * unit);
+    MX_CUFFT(cufftSetStream(plan, s));
+    cufftComplex* w = (cufftComplex*)(work + (long long)i * unit * gd.C);
+    Prof pr(c, "cufft_c2r", bytes * k * unit, s);
+    MX_CUFFT(cufftExecC2R(plan, w, (cufftReal*)w));
+    i += k;
+  }
+}
+
 static void run_find_HII_bubbles(mx_ctx* c, int snapshot, const mx_grids* g, mx_globals* out, cudaStream_t s,
                                  FhbDownloads* dl = nullptr)
 {
@@ -703,15 +751,7 @@ static void run_find_HII_bubbles(mx_ctx* c, int snapshot, const mx_grids* g, mx_
       Prof pr(c, "k_filter", (double)G * B8C * (1 + nf), s);
       launch_filter((const float2* const*)c->d_in_ptrs, G, c->d_work, gd.C, fb, gd, (float)p.box_size, s);
     }
-    // one radius (G fields) per cuFFT execution keeps the cuFFT work area at
-    // the size of one radius' spectra
-    const cufftHandle plan = c->c2r_plan(G);
-    MX_CUFFT(cufftSetStream(plan, s));
-    for (int r = 0; r < nf; r++) {
-      cufftComplex* w = (cufftComplex*)(c->d_work + (long long)r * G * gd.C);
-      Prof pr(c, "cufft_c2r", (double)G * (B8C + B4N), s);
-      MX_CUFFT(cufftExecC2R(plan, w, (cufftReal*)w));
-    }
+    run_c2r(c, c->d_work, nf, G, s);
     if (dl && dl->state_in && r0 == 0)
       MX_CUDA(cudaStreamWaitEvent(s, dl->state_in, 0));
     ThresholdArgs ta;
@@ -1039,13 +1079,7 @@ static void compute_shells(mx_ctx* c, const ShellPlan& sp, float* sfr, float* sf
         Prof pr(c, "k_filter_ts", 8.0 * (double)gd.C * (1 + nb), s);
         launch_filter((const float2* const*)c->d_in_ptrs, 1, c->d_work, gd.C, fb, gd, (float)p.box_size, s);
       }
-      const cufftHandle plan = c->c2r_plan(1);
-      MX_CUFFT(cufftSetStream(plan, s));
-      for (int q = 0; q < nb; q++) {
-        cufftComplex* w = (cufftComplex*)(c->d_work + (long long)q * gd.C);
-        Prof pr(c, "cufft_c2r", 8.0 * (double)gd.C + 4.0 * (double)gd.N, s);
-        MX_CUFFT(cufftExecC2R(plan, w, (cufftReal*)w));
-      }
+      run_c2r(c, c->d_work, nb, 1, s);
       {
         Prof pr(c, "k_shell_extract", 8.0 * (double)gd.N * nb, s);
         launch_shell_extract((const float*)c->d_work, gd.P, nb, q0, c->d_shells, gd, s);
@@ -2104,15 +2138,7 @@ static void step_graph(mx_ctx* c, int snapshot, const mx_grids* dev, mx_globals*
   c->graph_keep.clear();
   cudaGraph_t graph = nullptr;
   int launches = 0;
-  // cuFFT plans allocate their work areas when created, which a capture
-  // does not allow: create the ones the step uses first
-  if (!c->fused_fft) {
-    c->c2r_plan(n_fields(c->p));
-    if (c->p.flag_spin_temp)
-      c->c2r_plan(1);
-  }
-  if (c->p.flag_spin_temp && c->p.flag_pecvel > 0)
-    c->c2r_plan(1);
+  c->make_c2r_plans();
   MX_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
   c->capturing = true;
   try {
@@ -3372,13 +3398,7 @@ int mx_batch_run_graph(mx_batch* b, mx_batch_item* items, int32_t n_items)
         throw CudaError{ MX_EINVAL, c->err };
       check_snapshot(c, it.snapshot);
       c->ensure_mirror();
-      if (!c->fused_fft) {
-        c->c2r_plan(n_fields(c->p));
-        if (c->p.flag_spin_temp)
-          c->c2r_plan(1);
-      }
-      if (c->p.flag_spin_temp && c->p.flag_pecvel > 0)
-        c->c2r_plan(1);
+      c->make_c2r_plans();
       step_copy_lists(c->p, &ins[i], &outs[i]);
       const mx_grids* h = it.grids;
       float* mx_grids::*all[] = { &mx_grids::deltax,   &mx_grids::stars,        &mx_grids::weighted_sfr,
