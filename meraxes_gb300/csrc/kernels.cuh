@@ -100,8 +100,7 @@ struct ThresholdArgs
 {
   const float* fields;   // batch base: field (r*G + g) at fields + (r*G+g)*P
   long long P;
-  int G;                 // fields per radius: dx, stars, wsfr, [x_e], [N_rec]
-  int idx_xe, idx_nr;    // field slot or -1
+  int G;                 // fields per radius: dx, stars, wsfr, [x_e if spin], [N_rec if recomb]
   int n_r;               // radii in this batch
   const RadiusParams* rp; // device array, n_r entries
   // The unfiltered last step is an identity transform: its fields are read

@@ -758,8 +758,6 @@ static void run_find_HII_bubbles(mx_ctx* c, int snapshot, const mx_grids* g, mx_
     ta.fields = (const float*)c->d_work;
     ta.P = gd.P;
     ta.G = G;
-    ta.idx_xe = idx_xe;
-    ta.idx_nr = idx_nr;
     ta.n_r = nb;
     ta.rp = c->d_rp + r0;
     for (int f = 0; f < MAX_FIELDS; f++)
