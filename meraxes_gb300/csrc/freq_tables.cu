@@ -19,13 +19,16 @@
 //
 // On 16 host threads the tables took 8.4 ms per snapshot, longer than the
 // shells' transforms of any grid below 512^3.  Here (40 shells, one E0)
-// k_tau_lower takes 171 us, 20 steps one after another, and k_freq_integrals
-// 354 us, bound by the bisections of the longest integral (30 and more rounds)
-// at the FP64 rate and latency; with the cross sections' formulas instead of
-// their polynomials they took 360 and 986 us.
+// k_tau_lower takes 134 us, 20 steps one after another, and k_freq_integrals
+// 297 us, the bisections of the longest integral (30 and more rounds), both bound by
+// the FP64 unit's latency (its pipe is 30 to 45% busy on the longest SM).  173 and
+// 366 us with one thread keeping the interval list, an FP64 error estimate for every
+// tau_X and the species one after another; 360 and 986 us with the cross sections'
+// formulas instead of their polynomials.
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <vector>
 
 #include "freq_tables.cuh"
 #include "gk61.h"
@@ -110,13 +113,20 @@ __device__ __forceinline__ void panel_sums(double f, const Rule& w, PanelSums& p
     p.asc[warp] = c;
 }
 
+// QUADPACK's error estimate: asc (200 err / asc)^1.5 up to asc, as a product
+// with one reciprocal root (a quotient and a root one after the other take twice
+// as long).
 __device__ double rescale_err(double err, double res_abs, double res_asc)
 {
   err = fabs(err);
   if (res_asc != 0 && err != 0) {
-    const double t = 200 * err / res_asc;
-    const double scale = t * sqrt(t);
-    err = scale < 1 ? res_asc * scale : res_asc;
+    const double x = 200 * err, m = x * res_asc;
+    if (!(x < res_asc))
+      err = res_asc;
+    else if (m > 1e-280)
+      err = x * x * rsqrt(m);
+    else
+      err = x * sqrt(x / res_asc);
   }
   if (res_abs > DBL_MIN / (50 * DBL_EPSILON)) {
     const double min_err = 50 * DBL_EPSILON * res_abs;
@@ -138,115 +148,170 @@ __device__ Panel panel_of(const PanelSums& s, double a, double b)
   return p;
 }
 
-// Interval list in QUADPACK's partially sorted order (qpsrt) and the running
-// state of one adaptive integral, kept by thread 0.
+// One panel of 64 threads whose error is clearly within eps of its result
+// (the estimate, taken in floats, a hundredth below the tolerance): *result is
+// the Kronrod sum.  false: the panel's sums decide.
+struct FastSums
+{
+  double part[2][2];
+  float asc[2], abs[2];
+};
+__device__ __forceinline__ bool settled(double f, const Rule& w, FastSums& p, double half, double eps, double* result)
+{
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 1;
+  const bool odd = lane & 1;
+  double s = odd ? w.wg * f : w.wk * f;
+  s += __shfl_xor_sync(0xffffffffu, odd ? w.wk * f : w.wg * f, 1);
+#pragma unroll
+  for (int o = 2; o < 32; o <<= 1)
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane < 2)
+    p.part[warp][lane] = s;
+  __syncthreads();
+  const double rk = p.part[0][0] + p.part[1][0], rg = p.part[0][1] + p.part[1][1];
+  const float wk = (float)w.wk;
+  float asc = wk * fabsf((float)(f - rk * 0.5)), abs = wk * fabsf((float)f);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    asc += __shfl_xor_sync(0xffffffffu, asc, o);
+    abs += __shfl_xor_sync(0xffffffffu, abs, o);
+  }
+  if (lane == 0) {
+    p.asc[warp] = asc;
+    p.abs[warp] = abs;
+  }
+  __syncthreads();
+  *result = rk * half;
+  const float h = fabsf((float)half), tol = 0.99f * (float)(eps * fabs(*result));
+  asc = (p.asc[0] + p.asc[1]) * h;
+  const float least = 1.2e-14f * (p.abs[0] + p.abs[1]) * h;  // 50 epsilon, rounded up
+  const float x = 200.0f * fabsf((float)((rk - rg) * half));
+  return x < 0.9f * asc && x * sqrtf(x / asc) < tol && least < 0.5f * asc && least < tol && asc > 1e-30f;
+}
+
+// Interval list in QUADPACK's order of errors (qpsrt, whole list) and the running
+// state of one adaptive integral, kept by warp 0 of the block.
 struct Qag
 {
   double a[FREQ_INTERVALS], b[FREQ_INTERVALS], r[FREQ_INTERVALS], e[FREQ_INTERVALS];
   int order[FREQ_INTERVALS];
-  int size, nrmax, i, rt1, rt2, etype, more;
-  double area, errsum, tol, epsrel, result;
+  int size, i, rt1, rt2, more;
+  double area, errsum, epsrel, result;
   PanelSums sums[2];
-  Panel panel[2];
 
-  __device__ void sort_errors()
+  // The list after interval imax = order[0] became imax (error emax) and n
+  // (error emin <= emax): emax goes behind the larger ones, emin before those
+  // that are not larger than it.  Errors are not negative: as integers they
+  // compare in the same order.  All lanes of a warp.
+  __device__ void sort_errors(int imax, int n, double emax, double emin)
   {
-    const int last = size - 1;
-    int i_nrmax = nrmax;
-    const int i_maxerr = order[i_nrmax];
-    if (last < 2) {
+    const int lane = threadIdx.x & 31;
+    const long long hi = __double_as_longlong(emax), lo = __double_as_longlong(emin);
+    int idx[FREQ_INTERVALS / 32], to[FREQ_INTERVALS / 32], larger = 0, between = 0;
+#pragma unroll
+    for (int c = 0; c < FREQ_INTERVALS / 32; c++) {
+      to[c] = -1;
+      if (32 * c < n - 1) {
+        const int t = 32 * c + lane;
+        const bool in = t < n - 1;
+        idx[c] = in ? order[t + 1] : 0;
+        const long long x = __double_as_longlong(e[idx[c]]);
+        larger += __popc(__ballot_sync(0xffffffffu, in && x > hi));
+        between += __popc(__ballot_sync(0xffffffffu, in && x <= hi && x > lo));
+        if (in)
+          to[c] = x > hi ? t : t + 1 + (lo >= x);
+      }
+    }
+    __syncwarp();
+    const bool tie = n >= 2 && lo >= hi;
+#pragma unroll
+    for (int c = 0; c < FREQ_INTERVALS / 32; c++)
+      if (to[c] >= 0)
+        order[to[c]] = idx[c];
+    if (lane == 0) {
+      order[larger + tie] = imax;
+      order[tie ? larger : larger + 1 + between] = n;
+      i = larger ? idx[0] : (tie ? n : imax);
+    }
+  }
+
+  // after the first panel (its sums in sums[0]); more: bisect on.  Warp 0.
+  __device__ void begin(double lo, double hi, double eps)
+  {
+    const Panel p = panel_of(sums[0], lo, hi);
+    if ((threadIdx.x & 31) == 0) {
+      const double tol = eps * fabs(p.result);
+      epsrel = eps;
+      result = p.result;
+      more = 1;
+      const double round_off = 50 * DBL_EPSILON * p.resabs;
+      if ((p.abserr <= round_off && p.abserr > tol) || (p.abserr <= tol && p.abserr != p.resasc) || p.abserr == 0.0)
+        more = 0;
+      a[0] = lo;
+      b[0] = hi;
+      r[0] = p.result;
+      e[0] = p.abserr;
       order[0] = 0;
-      order[1] = 1;
-      i = i_maxerr;
-      return;
+      size = 1;
+      i = rt1 = rt2 = 0;
+      area = p.result;
+      errsum = p.abserr;
     }
-    const double errmax = e[i_maxerr];
-    while (i_nrmax > 0 && errmax > e[order[i_nrmax - 1]]) {
-      order[i_nrmax] = order[i_nrmax - 1];
-      i_nrmax--;
-    }
-    const int top = last;
-    int ii = i_nrmax + 1;
-    while (ii < top && errmax < e[order[ii]]) {
-      order[ii - 1] = order[ii];
-      ii++;
-    }
-    order[ii - 1] = i_maxerr;
-    const double errmin = e[last];
-    int kk = top - 1;
-    while (kk > ii - 2 && errmin >= e[order[kk]]) {
-      order[kk + 1] = order[kk];
-      kk--;
-    }
-    order[kk + 1] = last;
-    i = order[i_nrmax];
-    nrmax = i_nrmax;
   }
 
-  // after the first panel; more: bisect on
-  __device__ void begin(const Panel& p, double lo, double hi, double eps)
+  // the two halves of interval i, their sums in sums[0] and sums[1].  Warp 0:
+  // its even lanes estimate the error of the one and its odd lanes of the other.
+  __device__ void step(double ai, double b1, double bi, int* fail)
   {
-    epsrel = eps;
-    result = p.result;
-    tol = epsrel * fabs(p.result);
-    more = 1;
-    const double round_off = 50 * DBL_EPSILON * p.resabs;
-    if ((p.abserr <= round_off && p.abserr > tol) || (p.abserr <= tol && p.abserr != p.resasc) || p.abserr == 0.0)
-      more = 0;
-    a[0] = lo;
-    b[0] = hi;
-    r[0] = p.result;
-    e[0] = p.abserr;
-    order[0] = 0;
-    size = 1;
-    nrmax = i = rt1 = rt2 = etype = 0;
-    area = p.result;
-    errsum = p.abserr;
-  }
-
-  // the two halves of interval i
-  __device__ void step(const Panel& p1, const Panel& p2, int* fail)
-  {
-    const double ai = a[i], bi = b[i], ri = r[i], ei = e[i];
-    const double b1 = 0.5 * (ai + bi);
-    const double area12 = p1.result + p2.result, err12 = p1.abserr + p2.abserr;
-    errsum += err12 - ei;
-    area += area12 - ri;
-    if (p1.resasc != p1.abserr && p2.resasc != p2.abserr) {
-      const double delta = ri - area12;
-      if (fabs(delta) <= 1.0e-5 * fabs(area12) && err12 >= 0.99 * ei)
-        rt1++;
-      if (size >= 10 && err12 > ei)
-        rt2++;
+    const int lane = threadIdx.x & 31, odd = lane & 1;
+    const Panel p = panel_of(sums[odd], odd ? b1 : ai, odd ? bi : b1);
+    auto of = [](double v, int l) { return __shfl_sync(0xffffffffu, v, l); };
+    const double r1 = of(p.result, 0), r2 = of(p.result, 1), e1 = of(p.abserr, 0), e2 = of(p.abserr, 1);
+    const unsigned limited = __ballot_sync(0xffffffffu, p.resasc == p.abserr) & 3u;
+    const int im = i, n = size;
+    const double ri = r[im], ei = e[im], area12 = r1 + r2, err12 = e1 + e2;
+    const double sum = errsum + (err12 - ei), whole = area + (area12 - ri);
+    int t1 = rt1, t2 = rt2;
+    if (!limited) {
+      if (fabs(ri - area12) <= 1.0e-5 * fabs(area12) && err12 >= 0.99 * ei)
+        t1++;
+      if (n >= 10 && err12 > ei)
+        t2++;
     }
-    tol = epsrel * fabs(area);
-    if (errsum > tol) {
-      if (rt1 >= 6 || rt2 >= 20)
-        etype = 2;
+    bool on = sum > epsrel * fabs(whole);
+    if (on) {
       const double tmp = (1 + 100 * DBL_EPSILON) * (fabs(b1) + 1000 * DBL_MIN);
-      if (fabs(ai) <= tmp && fabs(bi) <= tmp)
-        etype = 3;
+      if (t1 >= 6 || t2 >= 20 || (fabs(ai) <= tmp && fabs(bi) <= tmp))
+        on = false;
     }
-    const int imax = i, n = size;
-    const bool swap = p2.abserr > p1.abserr;
-    a[imax] = swap ? b1 : ai;
-    b[imax] = swap ? bi : b1;
-    r[imax] = swap ? p2.result : p1.result;
-    e[imax] = swap ? p2.abserr : p1.abserr;
-    a[n] = swap ? ai : b1;
-    b[n] = swap ? b1 : bi;
-    r[n] = swap ? p1.result : p2.result;
-    e[n] = swap ? p1.abserr : p2.abserr;
-    size++;
-    sort_errors();
-    more = !etype && errsum > tol;
-    if (more && size == FREQ_INTERVALS) {
-      *fail = 1;
-      more = 0;
+    if (on && n + 1 == FREQ_INTERVALS) {
+      if (lane == 0)
+        *fail = 1;
+      on = false;
     }
-    if (!more) {
+    const bool swap = e2 > e1;
+    __syncwarp();  // every lane has read the state
+    if (lane == 0) {
+      errsum = sum;
+      area = whole;
+      rt1 = t1;
+      rt2 = t2;
+      size = n + 1;
+      more = on;
+      a[im] = swap ? b1 : ai;
+      b[im] = swap ? bi : b1;
+      r[im] = swap ? r2 : r1;
+      e[im] = swap ? e2 : e1;
+      a[n] = swap ? ai : b1;
+      b[n] = swap ? b1 : bi;
+      r[n] = swap ? r1 : r2;
+      e[n] = swap ? e1 : e2;
+    }
+    if (on) {
+      sort_errors(im, n, swap ? e2 : e1, swap ? e1 : e2);
+    } else if (lane == 0) {
       double s = 0;
-      for (int q = 0; q < size; q++)
+      for (int q = 0; q <= n; q++)
         s += r[q];
       result = s;
     }
@@ -304,21 +369,38 @@ __device__ __forceinline__ bool xs_in_table(int q, int i)
 {
   return i >= (q == 0 ? XS_SUB / 2 : (q == 1 ? XS_SUB + 3 * XS_SUB / 8 : 2 * XS_SUB + XS_SUB / 2)) && i < XS_INTERVALS;
 }
-__device__ __forceinline__ double xs_poly(const double (&tab)[XS_INTERVALS][XS_N], const XsAt& p)
+// The three species' values at p from tab, or formula(q) below their tables.
+// Above 6 NU_HI all three are polynomials, evaluated side by side in pairs of
+// terms: the FP64 unit's latency, not its rate, bounds a chain of nine.
+template <class F>
+__device__ __forceinline__ void xs_values(const double (&tab)[3][XS_INTERVALS][XS_N], const XsAt& p, double (&s)[3],
+                                          const F& formula)
 {
-  const double2* c = reinterpret_cast<const double2*>(tab[p.i]);
-  double2 v[XS_N / 2];
+  static_assert(XS_N == 10);
+  const double t2 = p.t * p.t, t4 = t2 * t2, t8 = t4 * t4;
+  auto poly = [&](int q) {
+    const double2* c = reinterpret_cast<const double2*>(tab[q][p.i]);
+    double v[5];
 #pragma unroll
-  for (int j = 0; j < XS_N / 2; j++)
-    v[j] = __ldg(c + j);
-  double s = v[XS_N / 2 - 1].y;
+    for (int j = 0; j < 5; j++) {
+      const double2 u = __ldg(c + j);
+      v[j] = fma(u.y, p.t, u.x);
+    }
+    return fma(v[4], t8, fma(fma(v[3], t2, v[2]), t4, fma(v[1], t2, v[0])));
+  };
+  if (xs_in_table(2, p.i)) {
 #pragma unroll
-  for (int j = XS_N / 2 - 1; j >= 0; j--) {
-    s = fma(s, p.t, v[j].x);
-    if (j > 0)
-      s = fma(s, p.t, v[j - 1].y);
+    for (int q = 0; q < 3; q++)
+      s[q] = poly(q);
+  } else {
+#pragma unroll 1
+    for (int q = 0; q < 3; q++) {
+      const double v = xs_in_table(q, p.i) ? poly(q) : formula(q);
+      s[0] = q == 0 ? v : s[0];
+      s[1] = q == 1 ? v : s[1];
+      s[2] = q == 2 ? v : s[2];
+    }
   }
-  return s;
 }
 
 // ---------------------------------------------------------- optical depth
@@ -347,6 +429,7 @@ __device__ double tau_factor(const FreqArgs& a, double zhat, double fcoll1, doub
 __global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant__ FreqArgs a)
 {
   __shared__ Qag q;
+  __shared__ FastSums fast;
   const int r = blockIdx.x, j = threadIdx.x;
   const double x_e = a.sums[1] / a.total, fcoll1 = a.sums[0] / a.total;
   if (x_e > 0.9999) {
@@ -366,17 +449,18 @@ __global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant
       if (j >= 61)
         return 0.0;
       const double nuhat = nu0 * (1 + zhat);
-      const XsAt p = xs_at(nuhat);
-      double sig = 0;
-#pragma unroll
-      for (int q = 0; q < 3; q++)
-        sig += share[q] * (xs_in_table(q, p.i) ? xs_poly(a.tables->xs[q], p) : xs_formula(q, nuhat));
-      return factor * sig;
+      double xs[3];
+      xs_values(a.tables->xs, xs_at(nuhat), xs, [&](int q) { return xs_formula(q, nuhat); });
+      return factor * fma(share[2], xs[2], fma(share[1], xs[1], share[0] * xs[0]));
     };
-    panel_sums(value(z0, factor0), w, q.sums[0]);
+    const double f = value(z0, factor0);
+    double first;
+    if (settled(f, w, fast, 0.5 * (zp - zpp), 0.005, &first))
+      return first;
+    panel_sums(f, w, q.sums[0]);
     __syncthreads();
-    if (j == 0)
-      q.begin(panel_of(q.sums[0], zpp, zp), zpp, zp, 0.005);
+    if (j < 32)
+      q.begin(zpp, zp, 0.005);
     __syncthreads();
     while (q.more) {
       const double lo = q.a[q.i], hi = q.b[q.i], mid = 0.5 * (lo + hi);
@@ -387,8 +471,8 @@ __global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant
         panel_sums(value(z, tau_factor(a, z, fcoll1, x_e)), w, q.sums[h]);
       }
       __syncthreads();
-      if (j == 0)
-        q.step(panel_of(q.sums[0], lo, mid), panel_of(q.sums[1], mid, hi), &a.out->fail);
+      if (j < 32)
+        q.step(lo, mid, hi, &a.out->fail);
       __syncthreads();
     }
     return q.result;
@@ -475,48 +559,64 @@ __global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant
 // just below itself) between two x_HII rows.
 struct EnergyBin
 {
-  int n;  // -1: below the table
-  float dE, width;
+  int n;
+  float dE;
+  bool below;  // below the table
 };
-__device__ __forceinline__ EnergyBin energy_bin(const FreqDevTables& t, float En)
+// The bins of the three species' energies: a guess from the logarithm, one step
+// off at most where the table's steps round, and then the exact edges.
+__device__ __forceinline__ void energy_bins(const FreqDevTables& t, float (&En)[3], EnergyBin (&b)[3])
 {
-  EnergyBin b;
-  if (En > t.energy_cap) {
-    En = t.energy_top;
-  } else if (En < t.energy[0]) {
-    b.n = -1;
-    return b;
+  float4 at[3];
+  bool off = false;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    if (En[q] > t.energy_cap)
+      En[q] = t.energy_top;
+    b[q].below = En[q] < t.bin[0].z;
+    const bool fine = En[q] < 1008.88f;
+    const float l = logf(En[q] * (fine ? 0.1f : (float)(1 / 1008.88)));
+    const int n = fine ? (int)(l * (float)(1 / 1.98026273e-2)) : 232 + (int)(l * (float)(1 / 9.53101798e-2));
+    b[q].n = min(max(n, 0), k::NENERGY - 2);
+    at[q] = __ldg(&t.bin[b[q].n]);
+    off |= (b[q].n > 0 && En[q] < at[q].x) || (b[q].n < k::NENERGY - 2 && En[q] >= at[q].y);
   }
-  int n = En < 1008.88f ? (int)(logf(En * 0.1f) * (float)(1 / 1.98026273e-2))
-                        : 232 + (int)(logf(En * (float)(1 / 1008.88)) * (float)(1 / 9.53101798e-2));
-  n = min(max(n, 0), k::NENERGY - 2);
-  while (n > 0 && En < t.edge[n])
-    n--;
-  while (n < k::NENERGY - 2 && En >= t.edge[n + 1])
-    n++;
-  b.n = n;
-  b.width = t.energy[n + 1] - t.energy[n];
-  b.dE = En - t.energy[n];
-  return b;
+  if (off) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      int n = b[q].n;
+      while (n > 0 && En[q] < t.bin[n].x)
+        n--;
+      while (n < k::NENERGY - 2 && En[q] >= t.bin[n].y)
+        n++;
+      b[q].n = n;
+      at[q] = t.bin[n];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    b[q].dE = En[q] - at[q].z;
 }
-__device__ __forceinline__ float in_energy(const float* row, const EnergyBin& b)
+__device__ __forceinline__ float in_energy(const float2* row, const EnergyBin& b)
 {
-  float v = (row[b.n + 1] - row[b.n]) / b.width;
-  v *= b.dE;
-  return v + row[b.n];
+  const float2 v = __ldg(row + b.n);
+  return fmaf(v.y, b.dE, v.x);
 }
-__device__ float interp(const FreqDevTables& t, const float (*tab)[k::NENERGY], float below, const EnergyBin& b, int xi)
+__device__ __forceinline__ float interp(const FreqDevTables& t, const float2 (*tab)[k::NENERGY], float below,
+                                        const EnergyBin& b, int xi)
 {
-  if (b.n < 0)
-    return below;
-  if (xi < k::NXHII - 1)
-    return in_energy(tab[xi], b);
-  const int m0 = k::NXHII - 2;
-  const float x = (float)(t.xhii[k::NXHII - 1] * 0.999);
-  const float lo = in_energy(tab[m0], b), hi = in_energy(tab[m0 + 1], b);
-  float v = (hi - lo) / (t.xhii[m0 + 1] - t.xhii[m0]);
-  v *= x - t.xhii[m0];
-  return v + lo;
+  float v;
+  if (xi < k::NXHII - 1) {
+    v = in_energy(tab[xi], b);
+  } else {
+    const int m0 = k::NXHII - 2;
+    const float x = (float)(t.xhii[k::NXHII - 1] * 0.999);
+    const float lo = in_energy(tab[m0], b), hi = in_energy(tab[m0 + 1], b);
+    v = (hi - lo) / (t.xhii[m0 + 1] - t.xhii[m0]);
+    v *= x - t.xhii[m0];
+    v += lo;
+  }
+  return b.below ? below : v;
 }
 
 __device__ __forceinline__ double integrand(const FreqArgs& a, double nu, int flag, int xi, double spec)
@@ -525,25 +625,28 @@ __device__ __forceinline__ double integrand(const FreqArgs& a, double nu, int fl
   const double xe = t.xhii[xi];
   const double nus[3] = { k::NU_HI, k::NU_HEI, k::NU_HEII };
   const double share[3] = { a.f_h * (1 - xe), a.f_he * (1 - xe), a.f_he * xe };
-  const XsAt p = xs_at(nu);
   const double eV = nu * (1.0 / k::NU_OVER_EV);
-  double s = 0;
+  float En[3];
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+    En[q] = (float)(eV - nus[q] / k::NU_OVER_EV);
+  EnergyBin b[3];
+  energy_bins(t, En, b);
+  double c[3], xs[3];
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    const EnergyBin b = energy_bin(t, (float)(eV - nus[q] / k::NU_OVER_EV));
-    double c = share[q];
     if (flag == 0)
-      c *= (double)interp(t, t.fheat, 1.0f, b, xi) * (nu - nus[q]);
+      c[q] = (double)interp(t, t.fheat, 1.0f, b[q], xi) * (nu - nus[q]);
     else if (flag == 1)
-      c *= (double)(interp(t, t.nion[0], 0.0f, b, xi) + interp(t, t.nion[1], 0.0f, b, xi) +
-                    interp(t, t.nion[2], 0.0f, b, xi) + 1);
+      c[q] = (double)(interp(t, t.nion[0], 0.0f, b[q], xi) + interp(t, t.nion[1], 0.0f, b[q], xi) +
+                      interp(t, t.nion[2], 0.0f, b[q], xi) + 1);
     else
-      c *= (double)interp(t, t.nlya, 0.0f, b, xi);
-    const double xs = xs_in_table(q, p.i) ? xs_poly(t.xs_spec[q], p)
-                                          : xs_formula(q, nu) * exp((-a.alpha - 1) * log(nu * (1.0 / k::NU_HI)));
-    s = fma(c, xs, s);
+      c[q] = (double)interp(t, t.nlya, 0.0f, b[q], xi);
+    c[q] *= share[q];
   }
-  return s * spec;
+  xs_values(t.xs_spec, xs_at(nu), xs,
+            [&](int q) { return xs_formula(q, nu) * exp((-a.alpha - 1) * log(nu * (1.0 / k::NU_HI))); });
+  return fma(c[2], xs[2], fma(c[1], xs[1], c[0] * xs[0])) * spec;
 }
 
 __global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_constant__ FreqArgs a)
@@ -574,20 +677,14 @@ __global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_con
     __syncthreads();
   };
   sums(lower, a.numax);
-  if (threadIdx.x == 0)
-    q.begin(panel_of(q.sums[0], lower, a.numax), lower, a.numax, 0.01);
+  if (threadIdx.x < 32)
+    q.begin(lower, a.numax, 0.01);
   __syncthreads();
   while (q.more) {
     const double lo = q.a[q.i], hi = q.b[q.i], mid = 0.5 * (lo + hi);
     sums(h ? mid : lo, h ? hi : mid);
-    if (threadIdx.x < 2) {
-      // the two panels' error estimates side by side, then the bookkeeping
-      const int u = threadIdx.x;
-      q.panel[u] = panel_of(q.sums[u], u ? mid : lo, u ? hi : mid);
-      __syncwarp(3u);
-      if (u == 0)
-        q.step(q.panel[0], q.panel[1], &a.out->fail);
-    }
+    if (threadIdx.x < 32)
+      q.step(lo, mid, hi, &a.out->fail);
     __syncthreads();
   }
   if (threadIdx.x < a.S) {
@@ -642,13 +739,20 @@ static void fill_xs(double alpha, FreqDevTables* t)
 void fill_freq_dev_tables(const HeatTables& ht, double alpha, FreqDevTables* t)
 {
   fill_xs(alpha, t);
-  std::memcpy(t->energy, ht.energy, sizeof(t->energy));
   std::memcpy(t->xhii, ht.xhii, sizeof(t->xhii));
-  std::memcpy(t->fheat, ht.fheat, sizeof(t->fheat));
-  std::memcpy(t->nlya, ht.nlya, sizeof(t->nlya));
-  std::memcpy(t->nion[0], ht.nion_hi, sizeof(t->nion[0]));
-  std::memcpy(t->nion[1], ht.nion_hei, sizeof(t->nion[1]));
-  std::memcpy(t->nion[2], ht.nion_heii, sizeof(t->nion[2]));
+  // a value and the slope to the next one, as interp_tab forms it
+  auto rows = [&](const float (&v)[k::NXHII][k::NENERGY], float2 (&out)[k::NXHII][k::NENERGY]) {
+    for (int x = 0; x < k::NXHII; x++)
+      for (int n = 0; n < k::NENERGY; n++) {
+        out[x][n].x = v[x][n];
+        out[x][n].y = n + 1 < k::NENERGY ? (v[x][n + 1] - v[x][n]) / (ht.energy[n + 1] - ht.energy[n]) : 0.0f;
+      }
+  };
+  rows(ht.fheat, t->fheat);
+  rows(ht.nlya, t->nlya);
+  rows(ht.nion_hi, t->nion[0]);
+  rows(ht.nion_hei, t->nion[1]);
+  rows(ht.nion_heii, t->nion[2]);
   // the last energy's 0.999 as interp_tab compares (in double) and takes it:
   // the largest float not above it, and its float
   const double cap = 0.999 * ht.energy[k::NENERGY - 1];
@@ -657,10 +761,10 @@ void fill_freq_dev_tables(const HeatTables& ht, double alpha, FreqDevTables* t)
   // loc_energy does not decrease with the energy: bisect the float at which
   // it reaches n
   const float top = ht.energy[k::NENERGY - 1];
-  t->edge[0] = 0.0f;
+  std::vector<float> edge(k::NENERGY + 1, 0.0f);
   for (int n = 1; n <= k::NENERGY; n++) {
     if (loc_energy(top) < n) {
-      t->edge[n] = INFINITY;
+      edge[n] = INFINITY;
       continue;
     }
     float lo = ht.energy[0], hi = top;
@@ -670,8 +774,10 @@ void fill_freq_dev_tables(const HeatTables& ht, double alpha, FreqDevTables* t)
       const float mid = lo + 0.5f * (hi - lo);
       (loc_energy(mid) >= n ? hi : lo) = mid;
     }
-    t->edge[n] = hi;
+    edge[n] = hi;
   }
+  for (int n = 0; n < k::NENERGY; n++)
+    t->bin[n] = make_float4(edge[n], edge[n + 1], ht.energy[n], 0.0f);
 }
 
 FreqArgs make_freq_args(const mx_params& p, const Derived& d, const std::vector<double>& zz, const double* stored_fcoll,

@@ -22,12 +22,12 @@ constexpr int XS_SUB = 16, XS_OCTAVES = 17, XS_INTERVALS = XS_SUB * XS_OCTAVES, 
 struct FreqDevTables
 {
   double xs[3][XS_INTERVALS][XS_N], xs_spec[3][XS_INTERVALS][XS_N];
-  float energy[k::NENERGY];
+  float4 bin[k::NENERGY];  // smallest energy of index n (loc_energy), of n + 1; energy n; unused
   float energy_cap, energy_top;  // energies above cap are looked up at top
-  float edge[k::NENERGY + 1];  // smallest energy whose index (loc_energy) is n
   float xhii[k::NXHII];
-  float fheat[k::NXHII][k::NENERGY], nlya[k::NXHII][k::NENERGY];
-  float nion[3][k::NXHII][k::NENERGY];
+  // value at an energy, slope to the next
+  float2 fheat[k::NXHII][k::NENERGY], nlya[k::NXHII][k::NENERGY];
+  float2 nion[3][k::NXHII][k::NENERGY];
 };
 void fill_freq_dev_tables(const HeatTables& ht, double alpha, FreqDevTables* t);
 
