@@ -418,11 +418,6 @@ void launch_finalize(const double* partials, int nvals, double* out, cudaStream_
 }
 
 // ============================================================ grid helpers
-__global__ void k_fill(float* p, long long n, float v)
-{
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    p[i] = v;
-}
 // The state that find_HII_bubbles starts from (find_HII_bubbles.c:102-116), one
 // launch for the three grids; n2 = cells / 2 (grid sizes are even, device grids
 // 8-byte aligned).  J_21 may be NULL.
@@ -455,38 +450,64 @@ void launch_fill_real_in_padded(float* p, const GridDims& gd, float v, cudaStrea
 }
 
 // =============================================================== ComputeTs
-// ComputeTs.c:321-322 / 311-312: the first slab_n_complex floats of the
-// padded sfr grid are rescaled or cleared (the reference loops over
-// slab_n_complex float elements of a 2*slab_n_complex array).
-__global__ void k_sfr_scale_half(float* sfr, long long n, double w)
+// SFR-history operations on the padded sfr grid, all of a shell in one pass, two
+// cells of a row per thread.  SCALE and ZERO apply to the first slab_n_complex
+// floats of the padded array (the reference loops over that many float elements of
+// a 2*slab_n_complex array, ComputeTs.c:311-322), padding included; LOAD and ADD
+// read a history slice with REAL indexing and write with PADDED indexing
+// (load_reion_sfr_grids, reionization.c:1756-1784).  Bound by HBM: a LOAD and an
+// ADD move three grids instead of five in two passes.  Seven shells' operations at
+// 256^3 take 0.34 ms (3.6 TB/s, partly from L2); one operation at a time, a float
+// per thread, 0.58 ms in 11 launches.
+__global__ void __launch_bounds__(256) k_sfr_ops(float* __restrict__ sfr, const __grid_constant__ SfrOpArgs a, int D,
+                                                 int H, long long N, long long nhalf)
 {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    sfr[i] = (float)((double)sfr[i] * w);
-}
-void launch_sfr_scale_half(float* sfr, long long nhalf, double w, cudaStream_t s)
-{
-  k_sfr_scale_half<<<blocks_for(nhalf, 256), 256, 0, s>>>(sfr, nhalf, w);
-  g_launches++;
-}
-void launch_sfr_zero_half(float* sfr, long long nhalf, cudaStream_t s)
-{
-  k_fill<<<blocks_for(nhalf, 256), 256, 0, s>>>(sfr, nhalf, 0.0f);
-  g_launches++;
-}
-// load_reion_sfr_grids, reionization.c:1756-1784: the history slice is read
-// with REAL indexing and written with PADDED indexing.
-__global__ void k_sfr_load(float* sfr, const float* slice, float w, int acc, int D, int H, long long N)
-{
-  for (long long ir = blockIdx.x * (long long)blockDim.x + threadIdx.x; ir < N; ir += (long long)gridDim.x * blockDim.x) {
-    const long long ip = pad_of(ir, D, H);
-    const float v = __fmul_rn(slice[ir], w);
-    sfr[ip] = acc ? __fadd_rn(sfr[ip], v) : v;
+  const long long n2 = N / 2;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2; i += (long long)gridDim.x * blockDim.x) {
+    const long long ir = 2 * i, ip = pad_of(ir, D, H);
+    auto half_op = [&](const SfrOpArgs::Op& op, long long at, float v) {
+      if (at >= nhalf || op.kind > SfrOp::ZERO_HALF)
+        return v;
+      return op.kind == SfrOp::SCALE_HALF ? (float)((double)v * op.dweight) : 0.0f;
+    };
+    float2* cell = reinterpret_cast<float2*>(sfr + ip);
+    if (a.loads || ip < nhalf) {
+      float2 v = a.op[0].kind == SfrOp::LOAD ? make_float2(0.f, 0.f) : *cell;
+      for (int q = 0; q < a.n; q++) {
+        const SfrOpArgs::Op& op = a.op[q];
+        if (op.kind >= SfrOp::LOAD) {
+          const float2 u = __ldg(reinterpret_cast<const float2*>(op.slice + ir));
+          const float x = __fmul_rn(u.x, op.weight), y = __fmul_rn(u.y, op.weight);
+          v = op.kind == SfrOp::ADD ? make_float2(__fadd_rn(v.x, x), __fadd_rn(v.y, y)) : make_float2(x, y);
+        } else {
+          v = make_float2(half_op(op, ip, v.x), half_op(op, ip + 1, v.y));
+        }
+      }
+      *cell = v;
+    }
+    if (a.halves && ir + 2 == (row_of(ir, D) + 1) * D)
+      for (long long at = ip + 2; at < ip + 2 + 2 * H - D && at < nhalf; at++) {
+        float v = sfr[at];
+        for (int q = 0; q < a.n; q++)
+          v = half_op(a.op[q], at, v);
+        sfr[at] = v;
+      }
   }
 }
-void launch_sfr_load(float* sfr, const float* slice, float w, int accumulate, const GridDims& gd, cudaStream_t s)
+void launch_sfr_ops(float* sfr, const SfrOp* ops, int n, const float* histories, const GridDims& gd, cudaStream_t s)
 {
-  k_sfr_load<<<blocks_for(gd.N, 256), 256, 0, s>>>(sfr, slice, w, accumulate, gd.D, gd.H, gd.N);
-  g_launches++;
+  for (int q0 = 0; q0 < n; q0 += SfrOpArgs::MAX) {
+    SfrOpArgs a{};
+    a.n = std::min(n - q0, SfrOpArgs::MAX);
+    for (int q = 0; q < a.n; q++) {
+      const SfrOp& op = ops[q0 + q];
+      const bool reads = op.kind >= SfrOp::LOAD;
+      a.op[q] = { op.kind, op.weight, op.dweight, reads ? histories + (long long)op.slice * gd.P : nullptr };
+      (reads ? a.loads : a.halves) = 1;
+    }
+    k_sfr_ops<<<blocks_for(gd.N / 2, 256), 256, 0, s>>>(sfr, a, gd.D, gd.H, gd.N, gd.C);
+    g_launches++;
+  }
 }
 
 // Two cells of a row per thread: the grids are 8-byte aligned and D is even.  45

@@ -145,10 +145,22 @@ void launch_fhb_init(float* xH, float* r_bubble, float* J21, const GridDims& gd,
 void launch_fill_real_in_padded(float* p, const GridDims& gd, float v, cudaStream_t s);
 
 // ---------------------------------------------------------------- ComputeTs
-// SFR-history operations on the PADDED sfr grid (ComputeTs.c:288-377).
-void launch_sfr_scale_half(float* sfr, long long nhalf, double w, cudaStream_t s);
-void launch_sfr_zero_half(float* sfr, long long nhalf, cudaStream_t s);
-void launch_sfr_load(float* sfr, const float* slice, float w, int accumulate, const GridDims& gd, cudaStream_t s);
+// SFR-history operations on the PADDED sfr grid (ComputeTs.c:288-377), in order;
+// histories: slices of P floats.
+struct SfrOpArgs
+{
+  static constexpr int MAX = 16;
+  struct Op
+  {
+    int kind;
+    float weight;
+    double dweight;
+    const float* slice;
+  } op[MAX];
+  int n, loads, halves;  // any LOAD or ADD, any SCALE_HALF or ZERO_HALF
+};
+struct SfrOp;
+void launch_sfr_ops(float* sfr, const SfrOp* ops, int n, const float* histories, const GridDims& gd, cudaStream_t s);
 
 // Shell value extraction: shells[r*N + real] = max(filtered_real, 0).
 void launch_shell_extract(const float* filtered, long long P, int n, int r0, float* shells, const GridDims& gd,

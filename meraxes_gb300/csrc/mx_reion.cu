@@ -986,17 +986,18 @@ static void compute_shells(mx_ctx* c, const ShellPlan& sp, float* sfr, float* sf
   const float delta_k = (float)(2.0 * k::PI / (float)p.box_size);
   int r = 0;
   while (r < S) {
-    for (const SfrOp& op : sp.ops[r]) {
-      if (up && op.kind >= SfrOp::LOAD)
-        MX_CUDA(cudaStreamWaitEvent(s, (*up->slices)[op.slice], 0));
-      Prof pr(c, "k_sfr_history", op.kind <= SfrOp::ZERO_HALF ? 8.0 * (double)nhalf : 12.0 * (double)gd.N, s);
-      if (op.kind == SfrOp::SCALE_HALF)
-        launch_sfr_scale_half(sfr, nhalf, op.dweight, s);
-      else if (op.kind == SfrOp::ZERO_HALF)
-        launch_sfr_zero_half(sfr, nhalf, s);
-      else
-        launch_sfr_load(sfr, sfr_histories + (long long)op.slice * gd.P, op.weight,
-                        op.kind == SfrOp::ADD, gd, s);
+    if (!sp.ops[r].empty()) {
+      const std::vector<SfrOp>& ops = sp.ops[r];
+      int loads = 0;
+      for (const SfrOp& op : ops)
+        if (op.kind >= SfrOp::LOAD) {
+          loads++;
+          if (up)
+            MX_CUDA(cudaStreamWaitEvent(s, (*up->slices)[op.slice], 0));
+        }
+      const int own = ops[0].kind == SfrOp::LOAD ? 1 : 2;  // reads and writes of sfr itself
+      Prof pr(c, "k_sfr_history", loads ? 4.0 * (double)gd.N * (loads + own) : 8.0 * (double)nhalf, s);
+      launch_sfr_ops(sfr, ops.data(), (int)ops.size(), sfr_histories, gd, s);
     }
     // shells r..r_end-1 share this spectrum (no operations in between)
     int r_end = r + 1;
