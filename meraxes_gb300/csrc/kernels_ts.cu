@@ -173,6 +173,99 @@ __device__ float kappa_f(const TsDevConst& c, int which, float T)
   return expf(ans);
 }
 
+// The kappa splines in shared memory, the cubic of each interval beside its node
+// and, for 64 steps of ln T, the interval that a step begins in: three binary
+// searches through global memory took a fifth of the per-cell update's time.
+struct KappaTab
+{
+  static constexpr int STEPS = 64, NODES = 27;
+  float4 p[3][NODES];  // y, and the coefficients of dx, dx^2, dx^3
+  float x[3][NODES + 1];
+  float x_last[3], y_last[3], slope[3], step[3];  // slope of the extrapolation above, steps per ln T
+  int last[3];                                    // last interval
+  unsigned char begin[3][STEPS];
+};
+__device__ void fill_kappa(KappaTab& t, const TsDevConst& c)
+{
+  for (int i = threadIdx.x; i < 3 * KappaTab::NODES; i += blockDim.x) {
+    const int w = i / KappaTab::NODES, q = i % KappaTab::NODES, n = c.nk[w];
+    const float *x = c.fkx[w], *y = c.fky[w], *cc = c.fkc[w];
+    if (q < n)
+      t.x[w][q] = x[q];
+    if (q < n - 1) {
+      const float h = x[q + 1] - x[q];
+      const float ih = __fdividef(1.0f, h);
+      const float b = (y[q + 1] - y[q]) * ih - h * (cc[q + 1] + 2.0f * cc[q]) * (1.0f / 3.0f);
+      t.p[w][q] = make_float4(y[q], b, cc[q], (cc[q + 1] - cc[q]) * ih * (1.0f / 3.0f));
+    }
+    if (q == n - 1) {
+      t.x_last[w] = x[q];
+      t.y_last[w] = y[q];
+      t.slope[w] = w == 0 ? 0.381f : (y[q] - y[q - 1]) / (x[q] - x[q - 1]);
+      t.step[w] = KappaTab::STEPS / (x[q] - x[0]);
+      t.last[w] = n - 2;
+    }
+  }
+  for (int i = threadIdx.x; i < 3 * KappaTab::STEPS; i += blockDim.x) {
+    const int w = i / KappaTab::STEPS, q = i % KappaTab::STEPS, n = c.nk[w];
+    const float* x = c.fkx[w];
+    // a hundredth of a step early, for the rounding of the step's number
+    const float from = x[0] + (x[n - 1] - x[0]) * ((q - 0.01f) / KappaTab::STEPS);
+    int lo = 0;
+    while (lo < n - 2 && x[lo + 1] <= from)
+      lo++;
+    t.begin[w][q] = (unsigned char)lo;
+  }
+}
+// kappa at lt = ln T as kappa_f, and d ln kappa / d ln T (the spline's derivative
+// inside the table, the extrapolations' slopes outside it)
+template <bool GRAD = false>
+__device__ __forceinline__ float kappa_s(const KappaTab& t, int w, float lt, float* dln = nullptr)
+{
+  const float x0 = t.x[w][0];
+  int lo = t.begin[w][(int)fminf(fmaxf((lt - x0) * t.step[w], 0.0f), (float)(KappaTab::STEPS - 1))];
+  while (lo < t.last[w] && t.x[w][lo + 1] <= lt)
+    lo++;
+  const float4 p = t.p[w][lo];
+  const float dx = lt - t.x[w][lo];
+  float ans = p.x + dx * (p.y + dx * (p.z + dx * p.w));
+  if constexpr (GRAD)
+    *dln = p.y + dx * (2.0f * p.z + 3.0f * p.w * dx);
+  if (lt < x0) {
+    ans = t.p[w][0].x;
+    if constexpr (GRAD)
+      *dln = 0.0f;
+  } else if (lt > t.x_last[w]) {
+    ans = t.y_last[w] + t.slope[w] * (lt - t.x_last[w]);
+    if constexpr (GRAD)
+      *dln = t.slope[w];
+  }
+  return expf(ans);
+}
+
+// a * b + c of both halves, each rounded as fmaf
+__device__ __forceinline__ float2 fma2(float a, float2 b, float2 c)
+{
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %2};\n\tmov.b64 y, {%3, %4};\n\tmov.b64 z, {%5, %6};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
+// Node below xcall in the x_HII table, whose bracket the tables are taken in
+// (ComputeTs.c:761-773).  Upwards: the gas outside ionised regions is nearly
+// neutral, and the table's lower nodes are its.
+__device__ __forceinline__ int xhii_node(const float* xhii, float xcall)
+{
+  int lo = 0;
+  while (lo < NXHII - 2 && xcall >= xhii[lo + 1])
+    lo++;
+  return lo;
+}
+
 // alpha_A (Abel et al. 1997 fit), XRayHeatingFunctions.c:1450-1458, in Horner form
 __device__ float alpha_A_f(float T)
 {
@@ -195,13 +288,14 @@ __device__ float alpha_A_f(float T)
 // quotients are reciprocals or quotients of __fdividef (2 ulp), well inside
 // that 1e-5 band around the criterion; get_Ts_grad repeats the same
 // operations, so the adjoint runs the forward's iteration count.
-__device__ bool get_Ts_f(const TsDevConst& c, float delta, float TK, float xe, float Jalpha, float* TS_out,
-                         float* xalpha)
+template <class K>
+__device__ bool get_Ts_f(const TsDevConst& c, const K& kappa, float delta, float TK, float xe, float Jalpha,
+                         float* TS_out, float* xalpha)
 {
   const float Trad = c.ftrad;
   const float opd = 1.0f + delta;
-  const float xc = c.fxc[0] * ((1.0f - xe) * opd) * kappa_f(c, 0, TK) +
-                   c.fxc[1] * (xe * opd) * kappa_f(c, 1, TK) + c.fxc[2] * (xe * opd) * kappa_f(c, 2, TK);
+  const float xc = c.fxc[0] * ((1.0f - xe) * opd) * kappa(0) + c.fxc[1] * (xe * opd) * kappa(1) +
+                   c.fxc[2] * (xe * opd) * kappa(2);
   float TS, xa = 0.0f;
   const float iTK = __fdividef(1.0f, TK);
   const float iTrad = __fdividef(1.0f, Trad);
@@ -251,6 +345,12 @@ __device__ bool get_Ts_f(const TsDevConst& c, float delta, float TK, float xe, f
 // engine's cost per copy made the S separate row copies the bound of the
 // ring.  The map applies when every tile is whole, the cell coordinate fits
 // a signed 32-bit index and S fits a box dimension.
+//
+// Bound by the latency and the shared-memory loads of its arithmetic at 16 warps
+// per SM (the two tables' rows for each shell and cell), then by HBM: 40 shells at
+// 256^3 take 1.41 ms (2.2 TB/s), at 512^3 11.2 ms.  With the kappa splines and the
+// x_HII table searched in global memory 1.70 and 13.6 ms; with those in shared memory
+// and scalar multiply-adds 1.53 and 12.1 ms.
 constexpr int EV_TILE = RED_THREADS;
 
 bool ev_shell_map_ok(long long N, int S) { return N % EV_TILE == 0 && N < (1LL << 31) && S >= 1 && S <= 256; }
@@ -295,6 +395,11 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
   float4* s_P = reinterpret_cast<float4*>(sm);  // NXHII * S
   float* stages = sm + ev_ring_offset(S);       // 2 * S * EV_TILE
   __shared__ uint64_t bars[STAGES];
+  __shared__ KappaTab s_kappa;
+  __shared__ float s_xhii[NXHII];
+  fill_kappa(s_kappa, c);
+  if (threadIdx.x < NXHII)
+    s_xhii[threadIdx.x] = c.xhii[threadIdx.x];
   for (int i = threadIdx.x; i < NXHII * S; i += blockDim.x) {
     const int x = i / S, r = i % S;
     s_P[i] = make_float4(c.fKH[r] * c.ftab[0][x][r], c.fKI[r] * c.ftab[1][x][r], c.fKL[r] * c.ftab[2][x][r],
@@ -316,12 +421,13 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
   CSum sum[4];
   // the cell state of tile k + 1 is read while tile k is computed
   float n_delta = 0.f, n_xe = 0.f, n_T = 1.f;
+  long long n_ip = 0;
   auto read_state = [&](int k) {
     const long long ir = (blockIdx.x + (long long)k * gridDim.x) * EV_TILE + threadIdx.x;
     if (k < my_tiles && ir < N) {
-      const long long ip = pad_index(ir, D, H);
-      n_delta = a.deltax[ip];
-      n_xe = a.x_e_prev[ip];
+      n_ip = pad_index(ir, D, H);
+      n_delta = a.deltax[n_ip];
+      n_xe = a.x_e_prev[n_ip];
       n_T = a.Tk[ir];
     }
   };
@@ -330,7 +436,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
     const long long tile = blockIdx.x + (long long)k * gridDim.x;
     const long long ir = tile * EV_TILE + threadIdx.x;
     const bool valid = ir < N;
-    const long long ip = valid ? pad_index(ir, D, H) : 0;
+    const long long ip = n_ip;
     float delta = 0.f, xe = 0.f, T = 1.f;
     if (valid) {
       delta = n_delta;
@@ -340,15 +446,12 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
     read_state(k + 1);
     // interpolation bracket in x_HII (ComputeTs.c:761-773)
     float xcall = xe;
-    if (xcall > c.xhii[NXHII - 1] * 0.999f)
-      xcall = c.xhii[NXHII - 1] * 0.999f;
-    else if (xcall < c.xhii[0])
-      xcall = 1.001f * c.xhii[0];
-    int lo = NXHII - 1;
-    while (lo > 0 && xcall < c.xhii[lo])
-      lo--;
-    const int hi = lo + 1;
-    const float w = __fdividef(xcall - c.xhii[lo], c.xhii[hi] - c.xhii[lo]);
+    if (xcall > s_xhii[NXHII - 1] * 0.999f)
+      xcall = s_xhii[NXHII - 1] * 0.999f;
+    else if (xcall < s_xhii[0])
+      xcall = 1.001f * s_xhii[0];
+    const int lo = xhii_node(s_xhii, xcall), hi = lo + 1;
+    const float w = __fdividef(xcall - s_xhii[lo], s_xhii[hi] - s_xhii[lo]);
     float heat = 0.f, ion = 0.f, lya = 0.f, star = 0.f;
     if (light) {
       const bool arrived = bulk::mbar_wait(&bars[k % STAGES], (unsigned)(k / STAGES) & 1u, full);
@@ -364,22 +467,22 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
       const float* st = stages + (size_t)(k % STAGES) * S * EV_TILE + threadIdx.x;
       const float4* Plo = s_P + lo * S;
       const float4* Phi = s_P + hi * S;
-      float hl = 0.f, il = 0.f, ll = 0.f, hh = 0.f, ih = 0.f, lh = 0.f;
+      // heat and ionisation, Ly-alpha and stars at the lower node, the same (stars
+      // unused) at the upper one: a packed multiply-add for each pair
+      float2 low_hi{}, low_ls{}, up_hi{}, up_ls{};
 #pragma unroll 4
       for (int r = 0; r < S; r++) {
         const float sf = st[r * EV_TILE];
         const float4 pl = Plo[r], ph = Phi[r];
-        hl = fmaf(sf, pl.x, hl);
-        il = fmaf(sf, pl.y, il);
-        ll = fmaf(sf, pl.z, ll);
-        star = fmaf(sf, pl.w, star);
-        hh = fmaf(sf, ph.x, hh);
-        ih = fmaf(sf, ph.y, ih);
-        lh = fmaf(sf, ph.z, lh);
+        low_hi = fma2(sf, make_float2(pl.x, pl.y), low_hi);
+        low_ls = fma2(sf, make_float2(pl.z, pl.w), low_ls);
+        up_hi = fma2(sf, make_float2(ph.x, ph.y), up_hi);
+        up_ls = fma2(sf, make_float2(ph.z, ph.w), up_ls);
       }
-      heat = fmaf(w, hh - hl, hl);
-      ion = fmaf(w, ih - il, il);
-      lya = fmaf(w, lh - ll, ll);
+      star = low_ls.y;
+      heat = fmaf(w, up_hi.x - low_hi.x, low_hi.x);
+      ion = fmaf(w, up_hi.y - low_hi.y, low_hi.y);
+      lya = fmaf(w, up_ls.x - low_ls.x, low_ls.x);
       // every thread has read this tile's stage: refill it with tile k + STAGES
       __syncthreads();
       if (threadIdx.x == 0 && k + STAGES < my_tiles)
@@ -411,7 +514,8 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
     if (T < 0.0f)
       T = c.ftk_floor;
     float TS, xalpha;
-    if (!get_Ts_f(c, delta, T, xe, Jalpha, &TS, &xalpha))
+    const float lt = logf(T);
+    if (!get_Ts_f(c, [&](int i) { return kappa_s(s_kappa, i, lt); }, delta, T, xe, Jalpha, &TS, &xalpha))
       TS = get_Ts_d(c, c.zp, delta, T, xe, Jalpha, &xalpha, a.err);
     a.x_e_prev[ip] = xe;
     a.Tk[ir] = T;
@@ -457,35 +561,6 @@ int launch_evolve(const EvolveArgs& a, const GridDims& gd, const void* shell_map
 // ======================================================================
 namespace {
 
-// d ln kappa / d ln T of kappa_f (the spline's derivative inside the table,
-// the extrapolation slopes outside it).
-__device__ float dlnkappa_dlnT(const TsDevConst& c, int which, float T)
-{
-  const int n = c.nk[which];
-  const float* x = c.fkx[which];
-  const float* y = c.fky[which];
-  const float* cc = c.fkc[which];
-  const float lt = logf(T);
-  if (lt < x[0])
-    return 0.0f;
-  if (lt > x[n - 1])
-    return which == 0 ? 0.381f : (y[n - 1] - y[n - 2]) / (x[n - 1] - x[n - 2]);
-  int lo = 0, hi = n - 1;
-  while (hi > lo + 1) {
-    const int mid = (lo + hi) >> 1;
-    if (x[mid] > lt)
-      hi = mid;
-    else
-      lo = mid;
-  }
-  const float h = x[lo + 1] - x[lo];
-  const float ih = __fdividef(1.0f, h);
-  const float dx = lt - x[lo];
-  const float b = (y[lo + 1] - y[lo]) * ih - h * (cc[lo + 1] + 2.0f * cc[lo]) * (1.0f / 3.0f);
-  const float d = (cc[lo + 1] - cc[lo]) * ih * (1.0f / 3.0f);
-  return b + dx * (2.0f * cc[lo] + 3.0f * d * dx);
-}
-
 // Value and gradient (d/dTK, d/dxe, d/dJ) of get_Ts_f, by forward-mode
 // differentiation of the same iteration (the number of iterations is that of
 // the FP32 forward; its stopping test is not differentiated).
@@ -494,15 +569,17 @@ struct TsGrad
   float TS, dT, dxe, dJ;
 };
 
-__device__ TsGrad get_Ts_grad(const TsDevConst& c, float delta, float TK, float xe, float J)
+__device__ TsGrad get_Ts_grad(const TsDevConst& c, const KappaTab& kt, float delta, float TK, float xe, float J)
 {
   const float Trad = c.ftrad;
   const float opd = 1.0f + delta;
   float k[3], dk[3];
+  const float lt = logf(TK);
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    k[i] = kappa_f(c, i, TK);
-    dk[i] = k[i] * dlnkappa_dlnT(c, i, TK) / TK;  // d kappa / d TK
+    float dln;
+    k[i] = kappa_s<true>(kt, i, lt, &dln);
+    dk[i] = k[i] * dln / TK;  // d kappa / d TK
   }
   const float xc = c.fxc[0] * ((1.0f - xe) * opd) * k[0] + c.fxc[1] * (xe * opd) * k[1] + c.fxc[2] * (xe * opd) * k[2];
   const float xc_T = c.fxc[0] * ((1.0f - xe) * opd) * dk[0] + c.fxc[1] * (xe * opd) * dk[1] + c.fxc[2] * (xe * opd) * dk[2];
@@ -604,6 +681,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_evolve_adjoint(AdjointArgs a, i
   float4* s_dP = s_P + NXHII * S;                            // NXHII * S (d/dE0; w unused)
   float* stages = sm + (2 * ev_tables_floats(S) + 31) / 32 * 32;  // 2 * S * EV_TILE, 128-byte aligned
   __shared__ uint64_t bars[2];
+  __shared__ KappaTab s_kappa;
+  __shared__ float s_xhii[NXHII];
+  fill_kappa(s_kappa, c);
+  if (threadIdx.x < NXHII)
+    s_xhii[threadIdx.x] = c.xhii[threadIdx.x];
   for (int i = threadIdx.x; i < NXHII * S; i += blockDim.x) {
     const int x = i / S, r = i % S;
     s_P[i] = make_float4(c.fKH[r] * c.ftab[0][x][r], c.fKI[r] * c.ftab[1][x][r], c.fKL[r] * c.ftab[2][x][r],
@@ -657,15 +739,12 @@ __global__ void __launch_bounds__(RED_THREADS) k_evolve_adjoint(AdjointArgs a, i
       a.grad_stars[ip] = stars_bar;
     // x_HII bracket (ComputeTs.c:761-773)
     float xcall = xe;
-    if (xcall > c.xhii[NXHII - 1] * 0.999f)
-      xcall = c.xhii[NXHII - 1] * 0.999f;
-    else if (xcall < c.xhii[0])
-      xcall = 1.001f * c.xhii[0];
-    int lo = NXHII - 1;
-    while (lo > 0 && xcall < c.xhii[lo])
-      lo--;
-    const int hi = lo + 1;
-    const float w = __fdividef(xcall - c.xhii[lo], c.xhii[hi] - c.xhii[lo]);
+    if (xcall > s_xhii[NXHII - 1] * 0.999f)
+      xcall = s_xhii[NXHII - 1] * 0.999f;
+    else if (xcall < s_xhii[0])
+      xcall = 1.001f * s_xhii[0];
+    const int lo = xhii_node(s_xhii, xcall), hi = lo + 1;
+    const float w = __fdividef(xcall - s_xhii[lo], s_xhii[hi] - s_xhii[lo]);
     float heat = 0.f, ion = 0.f, lya = 0.f, star = 0.f, dheat = 0.f, dion = 0.f, dlya = 0.f;
     const float* st = nullptr;
     if (light) {
@@ -735,7 +814,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_evolve_adjoint(AdjointArgs a, i
       Tn = c.ftk_floor;
       T_free = false;
     }
-    const TsGrad tg = get_Ts_grad(c, delta, Tn, xn, Jalpha);
+    const TsGrad tg = get_Ts_grad(c, s_kappa, delta, Tn, xn, Jalpha);
     // backward
     const float Tn_bar = TS_bar * tg.dT;
     xe_new_bar += TS_bar * tg.dxe;
@@ -800,7 +879,7 @@ __global__ void k_homog_f32(HomogArgs a, int D, int H, long long N)
     a.x_e_prev[ip] = a.xe0;
     a.Tk[ir] = a.tk0;
     float TS, xa;
-    if (!get_Ts_f(c, delta, a.tk0, a.xe0, 0.0f, &TS, &xa))
+    if (!get_Ts_f(c, [&](int i) { return kappa_f(c, i, a.tk0); }, delta, a.tk0, a.xe0, 0.0f, &TS, &xa))
       TS = get_Ts_d(c, c.zp, delta, a.tk0, a.xe0, 0.0f, &xa, a.err);
     a.TS[ir] = TS;
     const float cf = fminf(a.stars[ip] * kcf / (1.0f + delta), 1.0f);
