@@ -630,10 +630,14 @@ __device__ __forceinline__ int band_radius(const unsigned* start, int n, unsigne
 // 256^3 6202, 5456, 5923).
 template <int D>
 constexpr bool X_TILE_128 = D == 64 || D == 128;
+// Grids with a factor 3 hold 8 points a thread at most: three blocks of 384 threads
+// fit an SM without spills (56 registers; the y-pass and the forward passes four at
+// 40), whose loads hide each other's latency: 192^3, 41 radii of 5 fields and the
+// shells, x 3.0 -> 2.3 ms, y 2.6 -> 2.3 ms against two and three blocks.
 template <int D, int XTHREADS>
 constexpr int x_min_blocks()
 {
-  return XTHREADS == 128 ? 4 : (XTHREADS == 256 && D < 512 ? 3 : 2);
+  return XTHREADS == 128 ? 4 : ((XTHREADS == 256 && D < 512) || XTHREADS == TILE_THREADS_3 ? 3 : 2);
 }
 // BANDED: only the tiles with a mode inside the radius's band (Bands), radius
 // by radius; their lines outside it are not read.
@@ -755,7 +759,7 @@ struct YPassArgs
   Bands bands;
 };
 template <int D, int YTHREADS, bool BANDED>
-__global__ void __launch_bounds__(YTHREADS, YTHREADS == 256 ? 3 : 2) k_fft_y(const __grid_constant__ YPassArgs a)
+__global__ void __launch_bounds__(YTHREADS, YTHREADS == TILE_THREADS_3 ? 4 : (YTHREADS == 256 ? 3 : 2)) k_fft_y(const __grid_constant__ YPassArgs a)
 {
   using P = TilePlan<D>;
   constexpr int HP = Pitch<D>::HP;
@@ -1600,7 +1604,7 @@ __global__ void __launch_bounds__(T) k_fft_z_r2c(const __grid_constant__ FwdArgs
 // the first nt tiles of 16 kz columns of n_outer rows (all x, or the |ky| that
 // are read); the inverse y-pass's engine with conjugated input and output.
 template <int D, int T, int AXIS>
-__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_fwd_cols(float2* data, long long C, int nt, int n_outer)
+__global__ void __launch_bounds__(T, T == TILE_THREADS_3 ? 4 : (T == 256 ? 3 : 2)) k_fft_fwd_cols(float2* data, long long C, int nt, int n_outer)
 {
   using P = TilePlan<D>;
   constexpr int HP = Pitch<D>::HP;
