@@ -626,8 +626,9 @@ __device__ __forceinline__ int band_radius(const unsigned* start, int n, unsigne
 // autotuner picks).  A tile of a small grid has few points: 128 threads hold
 // D / 8 of them each, all in flight at once, and more tiles fit on an SM whose
 // barriers and loads are independent of each other (us for 41 radii of 5
-// fields with 128, 256, 512 threads: 64^3 125, 126, 184; 128^3 726, 836, 1047;
-// 256^3 6202, 5456, 5923).
+// fields with 128, 256, 512 threads: 64^3 124, 127, 185; 128^3 726, 711, 1045;
+// 256^3 6202, 5030, 5927).  256 threads run four blocks to an SM below 512^3 (64
+// registers, at 256^3 with 24 bytes spilled; three blocks: 128^3 830, 256^3 5432).
 template <int D>
 constexpr bool X_TILE_128 = D == 64 || D == 128;
 // Grids with a factor 3 hold 8 points a thread at most: three blocks of 384 threads
@@ -637,7 +638,7 @@ constexpr bool X_TILE_128 = D == 64 || D == 128;
 template <int D, int XTHREADS>
 constexpr int x_min_blocks()
 {
-  return XTHREADS == 128 ? 4 : ((XTHREADS == 256 && D < 512) || XTHREADS == TILE_THREADS_3 ? 3 : 2);
+  return XTHREADS == 128 || (XTHREADS == 256 && D < 512) ? 4 : (XTHREADS == TILE_THREADS_3 ? 3 : 2);
 }
 // BANDED: only the tiles with a mode inside the radius's band (Bands), radius
 // by radius; their lines outside it are not read.
