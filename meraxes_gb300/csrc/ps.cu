@@ -72,17 +72,18 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) k_ps_finalize(const double* __
 }
 
 // The field of ComputePowerSpectrum.c:94-110, (dT / ave - 1) V / N ave, without
-// its constant factor V / N (the binned sums take it squared, in FP64): dT - ave
-// with ave in two floats, so that the difference is rounded once.  In FP64 as
-// written, the quotient per cell bound the pass (507 us at 200^3).
+// its constant factor V / N (the binned sums take it squared, in FP64): dT less ave
+// as a float.  What that leaves out of ave is the same in every cell and enters the
+// k = 0 mode alone, whose power is k^3 = 0 times it; taken in, it would round in
+// every ionised cell (dT = 0) to the same side.  In FP64 as written, the quotient
+// per cell bound the pass (507 us at 200^3).
 __global__ void k_ps_field(const float* __restrict__ dT, const double* __restrict__ sum, double n_cells, int D, int H,
                            long long N, float* __restrict__ out)
 {
-  const double ave = sum[0] / n_cells;
-  const float hi = (float)ave, lo = (float)(ave - (double)hi);
+  const float ave = (float)(sum[0] / n_cells);
   for (long long ir = blockIdx.x * (long long)blockDim.x + threadIdx.x; ir < N; ir += (long long)gridDim.x * blockDim.x) {
     const long long row = row_of(ir, D);
-    out[row * 2LL * H + (ir - row * D)] = __fsub_rn(__fsub_rn(dT[ir], hi), lo);
+    out[row * 2LL * H + (ir - row * D)] = __fsub_rn(dT[ir], ave);
   }
 }
 
