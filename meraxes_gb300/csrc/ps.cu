@@ -75,12 +75,14 @@ __global__ void __launch_bounds__(32 * FIN_WARPS) k_ps_finalize(const double* __
 // its constant factor V / N (the binned sums take it squared, in FP64): dT less ave
 // as a float.  What that leaves out of ave is the same in every cell and enters the
 // k = 0 mode alone, whose power is k^3 = 0 times it; taken in, it would round in
-// every ionised cell (dT = 0) to the same side.  In FP64 as written, the quotient
-// per cell bound the pass (507 us at 200^3).
+// every ionised cell (dT = 0) to the same side.  A mean of 0 (a fully ionised box)
+// makes every cell's quotient infinite or NaN and the field NaN, as written there.
+// In FP64 as written, the quotient per cell bound the pass (507 us at 200^3).
 __global__ void k_ps_field(const float* __restrict__ dT, const double* __restrict__ sum, double n_cells, int D, int H,
                            long long N, float* __restrict__ out)
 {
-  const float ave = (float)(sum[0] / n_cells);
+  const double mean = sum[0] / n_cells;
+  const float ave = mean == 0.0 ? __int_as_float(0x7fffffff) : (float)mean;
   for (long long ir = blockIdx.x * (long long)blockDim.x + threadIdx.x; ir < N; ir += (long long)gridDim.x * blockDim.x) {
     const long long row = row_of(ir, D);
     out[row * 2LL * H + (ir - row * D)] = __fsub_rn(dT[ir], ave);
