@@ -15,6 +15,7 @@
 //                    50 sub-cells per cell, a thread per cell (fixed point,
 //                    order-independent deposits).
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 
 #include "pecvel.cuh"
@@ -32,13 +33,18 @@ constexpr double MPC_CM = 3.086e24;
 // result equals (float)(c * (double)x) unless that lies within 2^-48 of a tie.
 // Two FP32 operations instead of two conversions and a product at the FP64
 // rate (the FP64 form took 0.50 ms in k_vel_convert and, with its quotient,
-// 0.41 ms in k_vel_grad_k at 256^3).
+// 0.41 ms in k_vel_grad_k at 256^3).  An infinite x keeps its sign and stays
+// infinite, as in FP64: x lo alone would be NaN or of the other sign.
 struct Scale2
 {
   float hi, lo;
   Scale2() = default;
   __host__ explicit Scale2(double c) : hi((float)c), lo((float)(c - (double)(float)c)) {}
-  __device__ __forceinline__ float operator()(float x) const { return __fmaf_rn(x, hi, __fmul_rn(x, lo)); }
+  __device__ __forceinline__ float operator()(float x) const
+  {
+    const float p = __fmul_rn(x, lo);
+    return __fmaf_rn(x, hi, fabsf(x) <= FLT_MAX ? p : 0.0f);
+  }
 };
 
 // The unit factors in the reference's order, each rounded to float.
