@@ -307,8 +307,11 @@ __device__ __noinline__ void rsd_column_sequential(const RsdArgs& a, long long c
 // 24-bit sources, relative to the column's largest.  The sums are exact but for
 // the last of these roundings (1e-9 of a source at 256 cells), a column's
 // deposits stay below 2^63, and the result does not depend on their order.  n1
-// and n2 may come from FP32, because the series is continuous where they step (a
-// count off by one within rounding of a step moves 1e-6 of a sub-cell).
+// and n2 come from FP32: the series is continuous where they step, and a count off
+// by one within rounding of a step moves 1.5e-6 |B| of a sub-cell.  Where the
+// sub-cells lie more than two widths apart (|B| > 2; up to 8192 between
+// neighbours of opposite far displacements, which would move 1e-2), one exact
+// comparison each mends the counts.
 // A column with an infinite source or a displacement of RSD_FAR cells or more
 // (or NaN) takes the sequential routine.
 //
@@ -350,8 +353,20 @@ __device__ __forceinline__ void rsd_half(unsigned long long* acc, int kk, int D,
       // sub-cells below the boundary c + 1
       const long long U = ((c + 1) * RSD_CELL - lo) >> 1;
       const float u = (float)U * 0x1p-40f;
-      const int n1 = (int)fminf(fmaxf(floorf((u - 1.0f) * inv_step) + 1.0f, 0.0f), (float)n);
-      const int n2 = max(n1, (int)fminf(fmaxf(ceilf(u * inv_step), 0.0f), (float)n));
+      int n1 = (int)fminf(fmaxf(floorf((u - 1.0f) * inv_step) + 1.0f, 0.0f), (float)n);
+      int n2 = (int)fminf(fmaxf(ceilf(u * inv_step), 0.0f), (float)n);
+      if (step > 2 * RSD_ONE) {
+        // whole: U - i step >= 1; at least partly below: U - i step > 0
+        if (n1 < n && U - n1 * step >= RSD_ONE)
+          n1++;
+        else if (n1 > 0 && U - (n1 - 1) * step < RSD_ONE)
+          n1--;
+        if (n2 < n && U - n2 * step > 0)
+          n2++;
+        else if (n2 > 0 && U - (n2 - 1) * step <= 0)
+          n2--;
+      }
+      n2 = max(n1, n2);
       const int m = n2 - n1;
       const long long below = n1 * RSD_ONE + (m * U - ((n1 + n2 - 1) * m / 2) * step);
       const int mass = (int)((below + (1LL << (39 - bits))) >> (40 - bits));
