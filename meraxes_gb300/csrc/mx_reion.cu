@@ -1518,7 +1518,7 @@ static int run_power_spectrum(mx_ctx* c, const float* dT, float* ps_k, float* ps
   a.partials = c->d_ps_partials;
   {
     Prof pr(c, "k_ps_bin", 8.0 * (double)gd.C, s);
-    launch_ps_bin(a, c->d_ps_sums, s);
+    MX_CUDA(launch_ps_bin(a, c->d_ps_sums, s));
   }
   MX_CUDA(cudaMemcpyAsync(c->h_ps_sums, c->d_ps_sums, sizeof(double) * 3 * a.nb, cudaMemcpyDeviceToHost, s));
   MX_CUDA(cudaStreamSynchronize(s));
@@ -1574,7 +1574,7 @@ static double run_ps_loss(mx_ctx* c, const float* dT, int nbins, const float* ed
   a.spec = c->d_unf;
   {
     Prof pr(c, "k_ps_bin", 8.0 * (double)gd.C, s);
-    launch_ps_bin(a, c->d_ps_sums, s);
+    MX_CUDA(launch_ps_bin(a, c->d_ps_sums, s));
   }
   MX_CUDA(cudaMemcpyAsync(c->h_ps_sums, c->d_ps_sums, sizeof(double) * 3 * a.nb, cudaMemcpyDeviceToHost, s));
   MX_CUDA(cudaStreamSynchronize(s));

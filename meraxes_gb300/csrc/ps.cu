@@ -232,13 +232,21 @@ void launch_ps_field(const float* dT, const double* sum, const GridDims& gd, flo
   ps_launches++;
 }
 
-void launch_ps_bin(const PsArgs& a, double* sums, cudaStream_t s)
+cudaError_t launch_ps_bin(const PsArgs& a, double* sums, cudaStream_t s)
 {
   const size_t smem = sizeof(double) * RED_THREADS * (size_t)a.nb;
-  cudaFuncSetAttribute(k_ps_bin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit belongs to the function, not to the call: every caller sets the same
+  // one, or a call on another thread with fewer bins could lower it before this
+  // launch and make the launch fail
+  constexpr size_t smem_max = sizeof(double) * RED_THREADS * (size_t)PS_MAX_BINS;
+  const cudaError_t e =
+    cudaFuncSetAttribute(k_ps_bin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+  if (e != cudaSuccess)
+    return e;
   k_ps_bin<<<RED_BLOCKS, RED_THREADS, smem, s>>>(a);
   k_ps_finalize<<<(3 * a.nb + FIN_WARPS - 1) / FIN_WARPS, 32 * FIN_WARPS, 0, s>>>(a.partials, RED_BLOCKS, 3 * a.nb, sums);
   ps_launches += 2;
+  return cudaSuccess;
 }
 
 void launch_ps_scale(const float* dT, float scale, const GridDims& gd, float* out, cudaStream_t s)

@@ -24,7 +24,7 @@ void launch_ps_mean(const float* dT, long long N, double* partials, double* sum,
 // dT - mean (padded); the sum of dT over the cells in *sum (device)
 void launch_ps_field(const float* dT, const double* sum, const GridDims& gd, float* out, cudaStream_t s);
 // sums: k^3 |X|^2, |k| and modes per bin
-void launch_ps_bin(const PsArgs& a, double* sums, cudaStream_t s);
+cudaError_t launch_ps_bin(const PsArgs& a, double* sums, cudaStream_t s);
 // power-spectrum loss: f = dT * scale (padded), gradient spectrum (in place:
 // Y_k = coef[bin] k^3 X_k, doubled on the kz = 0, D/2 planes), REAL = padded * scale
 void launch_ps_scale(const float* dT, float scale, const GridDims& gd, float* out, cudaStream_t s);
