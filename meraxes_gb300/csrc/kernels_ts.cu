@@ -529,14 +529,29 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
   block_sum_store<4>(acc, a.partials);
 }
 
+// Shared memory of the per-cell kernels, forward and adjoint, with S shells.  The
+// function's limit is set to the size for MAX_SHELLS by every call: it belongs to
+// the function in the device's context, and a call with fewer shells on another
+// thread must not lower it between this call's set and its launch.
+template <int STAGES>
+static constexpr size_t ev_smem(int S)
+{
+  return sizeof(float) * (ev_ring_offset(S) + STAGES * (size_t)S * EV_TILE);
+}
+static constexpr size_t adjoint_smem(int S)
+{
+  return sizeof(float) * ((2 * ev_tables_floats(S) + 31) / 32 * 32 + 2 * (size_t)S * EV_TILE);
+}
+
 // Grid: every SM's resident blocks once (the blocks loop over their tiles),
 // at most RED_BLOCKS (the partial-sum slots).
 template <int STAGES>
 static int launch_evolve_t(const EvolveArgs& a, const GridDims& gd, const bulk::TensorMap& map, int use_map,
                            cudaStream_t s)
 {
-  const size_t smem = sizeof(float) * (ev_ring_offset(a.n_shells) + STAGES * (size_t)a.n_shells * EV_TILE);
-  cudaFuncSetAttribute(k_evolve_f32<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = ev_smem<STAGES>(a.n_shells);
+  cudaFuncSetAttribute(k_evolve_f32<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)ev_smem<STAGES>(MAX_SHELLS));
   int dev = 0, sms = 152, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -852,9 +867,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_evolve_adjoint(AdjointArgs a, i
 
 void launch_evolve_adjoint(const AdjointArgs& a, const GridDims& gd, const void* shell_map, cudaStream_t s)
 {
-  const size_t smem =
-    sizeof(float) * ((2 * ev_tables_floats(a.n_shells) + 31) / 32 * 32 + 2 * (size_t)a.n_shells * EV_TILE);
-  cudaFuncSetAttribute(k_evolve_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = adjoint_smem(a.n_shells);
+  cudaFuncSetAttribute(k_evolve_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adjoint_smem(MAX_SHELLS));
   bulk::TensorMap map{};
   if (shell_map)
     std::memcpy(&map, shell_map, sizeof(map));
