@@ -166,7 +166,10 @@ int mx_create(const mx_params* params, const char* tables_dir, mx_ctx** out);
 /* mx_create with the transform work buffer capped at max_work_bytes (it
  * holds at least the fields of one filter radius), for several contexts on
  * one GPU, e.g. a batch of independent boxes.  mx_create takes up to 45% of
- * the free device memory for it.  No reference counterpart. */
+ * the free device memory for it.  Not under the cap: the unfiltered spectra, the
+ * shells, and the work areas of the cuFFT plans, which the first calls make (at
+ * most 128 MB, and six spectra).  Results do not depend on the cap.  No reference
+ * counterpart. */
 int mx_create_limited(const mx_params* params, const char* tables_dir, size_t max_work_bytes, mx_ctx** out);
 void mx_destroy(mx_ctx* ctx);
 

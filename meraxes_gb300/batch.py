@@ -121,7 +121,9 @@ class BatchRunner:
             torch.cuda.synchronize()
             free1, _ = torch.cuda.mem_get_info()
             # context + this size's box inputs and the step's copies (about 40 grids)
-            self.ctx_bytes[D] = (free0 - free1) + 40 * 4 * D ** 3
+            # + the cuFFT plans' work areas, which the first calls make (mx_create_limited)
+            plans = (128 << 20) + 6 * 8 * D * D * (D // 2 + 1)
+            self.ctx_bytes[D] = (free0 - free1) + 40 * 4 * D ** 3 + plans
         free, _ = torch.cuda.mem_get_info()
         budget = self.memory_fraction * free / max(len(self.sizes), 1)
         for D in self.sizes:

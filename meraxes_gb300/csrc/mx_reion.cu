@@ -64,10 +64,14 @@ int hw_threads()
 }  // namespace
 
 // Spectra of one cuFFT C2R execution of the unfused path: small transforms are
-// launch-bound and leave the GPU idle one by one, while the work area grows with
-// the batch (a few times this size).  42 radii of 5 fields, one radius at a time
-// -> in groups: 0.98 -> 0.54 ms at 50^3, 2.6 -> 2.2 at 100^3; from 144^3 on a
-// radius fills the GPU (6.2 ms both ways) and the group is one.
+// launch-bound and leave the GPU idle one by one, while a plan's work area grows
+// with the batch (none for sizes of factors 2, 3, 5, 7, 11, as large as the spectra
+// for others).  42 radii of 5 fields, one radius at a time -> in groups: 0.98 -> 0.54
+// ms at 50^3, 2.6 -> 2.2 at 100^3; from 144^3 on a radius fills the GPU (6.2 ms both
+// ways) and the group is one.  A spectrum's result does not depend on the batch of
+// the plan that it goes through: the same bits for every even size from 2 to 206 in
+// batches of 1 to 80 (cuFFT 12.0), so nor on the group, which follows the memory that
+// the context has.
 constexpr long long C2R_GROUP_BYTES = 64LL << 20;
 constexpr int C2R_GROUP_MAX = 16;
 
