@@ -232,6 +232,10 @@ int32_t mx_n_sfr_histories(const mx_ctx* ctx);
  * y-pass of its fused inverse transforms (256 or 512; 384 with a factor 3; 0
  * and 0 when the grid uses cuFFT).  No reference counterpart. */
 int mx_fft_block_sizes(const mx_ctx* ctx, int32_t* x_threads, int32_t* y_threads);
+/* Threads that transform one tile of the x-pass: those of a block, or 128 where
+ * two tiles share a block of 256 (0 when the grid uses cuFFT).  No reference
+ * counterpart. */
+int32_t mx_fft_x_tile_threads(const mx_ctx* ctx);
 /* Resident blocks per SM that the threshold z-pass's registers are budgeted
  * for (2, or 3 with MX_ZPASS_BLOCKS=3; 0 when the grid does not run that
  * kernel).  No reference counterpart. */

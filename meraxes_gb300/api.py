@@ -93,8 +93,12 @@ class ReionGridStep:
         n = self.lib.mx_filter_radii(self.ctx, buf, 1024)
         return list(buf[:n])
 
+    def fft_x_tile_threads(self) -> int:
+        """Threads per tile of the x-pass (mx_fft_x_tile_threads)."""
+        return int(self.lib.mx_fft_x_tile_threads(self.ctx))
+
     def zpass_blocks(self) -> int:
-        """Resident blocks per SM the threshold z-pass was tuned for (0: not run)."""
+        """Resident blocks per SM that the threshold z-pass is compiled for (0: not run)."""
         return int(self.lib.mx_zpass_blocks_per_sm(self.ctx))
 
     def set_graph(self, on: bool = True):

@@ -2670,6 +2670,8 @@ int mx_set_redshifts(mx_ctx* ctx, const double* zz, int32_t n_snaps)
 
 int32_t mx_n_sfr_histories(const mx_ctx* ctx) { return ctx ? ctx->n_hist : -1; }
 
+int32_t mx_fft_x_tile_threads(const mx_ctx* ctx) { return ctx && ctx->fused_fft ? ctx->x_threads : 0; }
+
 int32_t mx_zpass_blocks_per_sm(const mx_ctx* ctx)
 {
   if (!ctx)
