@@ -2443,10 +2443,15 @@ int mx_create_limited(const mx_params* params, const char* tables_dir, size_t ma
 // (the thread count changes only which thread runs which column transform,
 // not the arithmetic).  Which one is faster depends on the grid size: a tile
 // of a small grid has few points, at 512^3 the larger block keeps more loads in
-// flight.  The context times them on its own scratch at creation (zero spectra
-// of its fields, up to 16 radii or 1 GB, best of three launches) and keeps the
-// fastest.  MX_XPASS_THREADS / MX_YPASS_THREADS fix a choice; MX_AUTOTUNE=0
-// keeps the defaults (x 512, y 256).
+// flight.  Up to 256^3 512 threads are slower in both passes (excursion sets with x
+// 256, x 512, y 512: 64^3 343, 373, 393 us, 256^3 16.8, 17.7, 17.9 ms; the step at
+// 128^3 4.31, 4.69, 4.79 ms), so only what may win is timed: x tiles of 128 and 256
+// threads at 64^3 and 128^3, both passes with 256 and 512 at 512^3, nothing at 32^3
+// and 256^3.  The context times them on its own scratch at creation (zero spectra of
+// its fields, up to eight radii or 1 GB, best of three launches) and keeps the
+// fastest: all candidates at every size made the creation of a context without
+// tables 4.7 ms at 128^3 and 1.6 at 64^3, now 1.6 and 1.0.  MX_XPASS_THREADS /
+// MX_YPASS_THREADS fix a choice; MX_AUTOTUNE=0 keeps the defaults (x 512, y 256).
 static void tune_fft(mx_ctx* c)
 {
   auto env_threads = [](const char* name) {
@@ -2473,12 +2478,19 @@ static void tune_fft(mx_ctx* c)
   if ((fx && fy) || (at && std::string(at) == "0") || !c->fused_fft)
     return;
   const GridDims& gd = c->gd;
+  const bool wide = gd.D > 256, narrow = fft_x_threads_ok(gd.D, 128);
+  if (!fx)
+    c->x_threads = 256;
+  if (!fy)
+    c->y_threads = 256;
+  if (!wide && (fx || !narrow))
+    return;
   cudaStream_t s = c->stream;
   const int G = n_fields(c->p);
   MX_CUDA(cudaMemsetAsync(c->d_unf, 0, sizeof(float2) * c->unf_C * G, s));
   const long long spectrum_bytes = (long long)sizeof(float2) * c->work_C;
   const int n =
-    (int)std::max<long long>(1, std::min<long long>({ c->work_fields / G, (1LL << 30) / (spectrum_bytes * G), 16 }));
+    (int)std::max<long long>(1, std::min<long long>({ c->work_fields / G, (1LL << 30) / (spectrum_bytes * G), 8 }));
   XPassArgs xa;
   for (int f = 0; f < MAX_FIELDS; f++)
     xa.in[f] = f < G ? c->d_unf + (long long)f * c->unf_C : nullptr;
@@ -2512,14 +2524,14 @@ static void tune_fft(mx_ctx* c)
   };
   float tx = 1e30f, ty = 1e30f;
   for (const int t : { 128, 256, 512 }) {
-    if (!fx && fft_x_threads_ok(gd.D, t)) {
+    if (!fx && fft_x_threads_ok(gd.D, t) && (t == 256 || t == (wide ? 512 : 128))) {
       const float ms = best_ms([&] { launch_fft_x_filter(gd.D, xa, t, s); });
       if (ms < tx) {
         tx = ms;
         c->x_threads = t;
       }
     }
-    if (!fy && t >= 256) {
+    if (!fy && wide && t >= 256) {
       const float ms = best_ms([&] { launch_fft_y(gd.D, c->d_work, c->work_C, n * G, Bands{}, t, s); });
       if (ms < ty) {
         ty = ms;
