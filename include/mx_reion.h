@@ -236,6 +236,10 @@ int mx_fft_block_sizes(const mx_ctx* ctx, int32_t* x_threads, int32_t* y_threads
  * two tiles share a block of 256 (0 when the grid uses cuFFT).  No reference
  * counterpart. */
 int32_t mx_fft_x_tile_threads(const mx_ctx* ctx);
+/* Sets of frequency-integral tables (one per ComputeTs, three per adjoint) that
+ * the context built on host threads, because an integral needed more intervals
+ * than the device holds.  No reference counterpart. */
+int32_t mx_freq_fallbacks(const mx_ctx* ctx);
 /* Resident blocks per SM that the threshold z-pass's registers are budgeted
  * for (2, or 3 with MX_ZPASS_BLOCKS=3; 0 when the grid does not run that
  * kernel).  No reference counterpart. */

@@ -27,7 +27,7 @@ EXPORTS = [
     "mx_lightcone_init", "mx_ConstructLightcone", "mx_ConstructLightcone_device",
     "mx_construct_baryon_grids", "mx_construct_baryon_grids_device", "mx_calculate_Mvir_crit",
     "mx_calculate_Mvir_crit_device", "mx_set_xray_params", "mx_ps_loss_device", "mx_adjoint_device",
-    "mx_create_limited", "mx_fft_block_sizes", "mx_fft_x_tile_threads", "mx_zpass_blocks_per_sm", "mx_set_step_graph", "mx_batch_create", "mx_batch_run",
+    "mx_create_limited", "mx_fft_block_sizes", "mx_fft_x_tile_threads", "mx_freq_fallbacks", "mx_zpass_blocks_per_sm", "mx_set_step_graph", "mx_batch_create", "mx_batch_run",
     "mx_batch_run_graph", "mx_batch_destroy",
     "mx_batch_last_error",
 ]
@@ -86,6 +86,8 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
         L.mx_fft_block_sizes.restype = ctypes.c_int
         L.mx_fft_x_tile_threads.argtypes = [P]
         L.mx_fft_x_tile_threads.restype = ctypes.c_int32
+        L.mx_freq_fallbacks.argtypes = [P]
+        L.mx_freq_fallbacks.restype = ctypes.c_int32
         L.mx_zpass_blocks_per_sm.argtypes = [P]
         L.mx_zpass_blocks_per_sm.restype = ctypes.c_int32
         L.mx_set_step_graph.argtypes = [P, ctypes.c_int32]

@@ -97,6 +97,10 @@ class ReionGridStep:
         """Threads per tile of the x-pass (mx_fft_x_tile_threads)."""
         return int(self.lib.mx_fft_x_tile_threads(self.ctx))
 
+    def freq_fallbacks(self) -> int:
+        """Table sets of ComputeTs that were built on host threads (mx_freq_fallbacks)."""
+        return int(self.lib.mx_freq_fallbacks(self.ctx))
+
     def zpass_blocks(self) -> int:
         """Resident blocks per SM that the threshold z-pass is compiled for (0: not run)."""
         return int(self.lib.mx_zpass_blocks_per_sm(self.ctx))

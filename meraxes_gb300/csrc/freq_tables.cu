@@ -39,7 +39,6 @@ namespace {
 // per host thread: a call counts its own launches when contexts run concurrently
 thread_local int freq_launches = 0;
 
-constexpr int FREQ_INTERVALS = 128;
 constexpr int TAU_THREADS = 64;
 constexpr int INT_THREADS = 128;
 
@@ -261,7 +260,7 @@ struct Qag
 
   // the two halves of interval i, their sums in sums[0] and sums[1].  Warp 0:
   // its even lanes estimate the error of the one and its odd lanes of the other.
-  __device__ void step(double ai, double b1, double bi, int* fail)
+  __device__ void step(double ai, double b1, double bi, int limit, int* fail)
   {
     const int lane = threadIdx.x & 31, odd = lane & 1;
     const Panel p = panel_of(sums[odd], odd ? b1 : ai, odd ? bi : b1);
@@ -284,7 +283,7 @@ struct Qag
       if (t1 >= 6 || t2 >= 20 || (fabs(ai) <= tmp && fabs(bi) <= tmp))
         on = false;
     }
-    if (on && n + 1 == FREQ_INTERVALS) {
+    if (on && n + 1 >= limit) {
       if (lane == 0)
         *fail = 1;
       on = false;
@@ -472,7 +471,7 @@ __global__ void __launch_bounds__(TAU_THREADS) k_tau_lower(const __grid_constant
       }
       __syncthreads();
       if (j < 32)
-        q.step(lo, mid, hi, &a.out->fail);
+        q.step(lo, mid, hi, a.intervals, &a.out->fail);
       __syncthreads();
     }
     return q.result;
@@ -684,7 +683,7 @@ __global__ void __launch_bounds__(INT_THREADS) k_freq_integrals(const __grid_con
     const double lo = q.a[q.i], hi = q.b[q.i], mid = 0.5 * (lo + hi);
     sums(h ? mid : lo, h ? hi : mid);
     if (threadIdx.x < 32)
-      q.step(lo, mid, hi, &a.out->fail);
+      q.step(lo, mid, hi, a.intervals, &a.out->fail);
     __syncthreads();
   }
   if (threadIdx.x < a.S) {

@@ -9,6 +9,7 @@
 namespace mx {
 
 constexpr int FREQ_SETS = 3;  // X-ray thresholds E0 of one call (the adjoint needs three)
+constexpr int FREQ_INTERVALS = 128;  // intervals of one adaptive integral that the kernels hold
 constexpr int FREQ_TAB = 3 * k::NXHII;  // rows of a set: tab[(flag * 14 + x) * S + r]
 
 // Cross sections as polynomials: a sixteenth of an octave in nu / NU_HI per
@@ -47,6 +48,7 @@ struct FreqArgs
   const double* sums;           // device: sum of f_coll and of x_e over the cells
   double total;                 // cells
   int S, n_sets;
+  int intervals;  // at most FREQ_INTERVALS; fewer in a test of the host fallback
   double zp, zpp[MAX_SHELLS];
   double E0[FREQ_SETS];    // NuXrayGalThreshold [eV]
   double spec[FREQ_SETS];  // (NU_HI / E0)^(-alpha - 1)

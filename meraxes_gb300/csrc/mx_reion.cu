@@ -151,6 +151,8 @@ struct mx_ctx
   FreqDevTables* d_ft_tables = nullptr;
   FreqDevResult* d_ft = nullptr;
   FreqDevResult* h_ft = nullptr;  // pinned copy
+  int freq_intervals = FREQ_INTERVALS;  // MX_FREQ_INTERVALS
+  int freq_fallbacks = 0;               // table sets built on host threads
   // device mirror used by the host-pointer entry points
   mx_grids mirror{};
   std::vector<void*> mirror_allocs;
@@ -1103,6 +1105,7 @@ static void launch_tables(mx_ctx* c, const ShellPlan& sp, int snapshot, const st
   a.sums = c->d_sums;
   a.total = (double)c->gd.N;
   a.n_sets = (int)E0.size();
+  a.intervals = c->freq_intervals;
   for (int i = 0; i < a.n_sets; i++) {
     a.E0[i] = E0[i];
     a.spec[i] = std::pow(k::NU_HI / (E0[i] * k::NU_OVER_EV), -a.alpha - 1);
@@ -1118,10 +1121,12 @@ static void launch_tables(mx_ctx* c, const ShellPlan& sp, int snapshot, const st
 static void take_tables(mx_ctx* c, const mx_params& p, const ShellPlan& sp, int snapshot, int i, double x_e_ave,
                         FreqTables* ft)
 {
-  if (c->h_ft->fail)
+  if (c->h_ft->fail) {
     build_freq_integrals(p, c->d, c->ht, c->zz, c->stored_fcoll, snapshot, sp, x_e_ave, c->nthreads, ft);
-  else
+    c->freq_fallbacks++;
+  } else {
     ft->tab.assign(c->h_ft->tab[i], c->h_ft->tab[i] + (size_t)FREQ_TAB * sp.S);
+  }
 }
 
 // ComputeTs's host work inside a captured step: a host node of the graph
@@ -2582,6 +2587,8 @@ static int create_ctx(const mx_params* params, const char* tables_dir, size_t wo
   c->nthreads = std::max(1, std::min(64, hw_threads()));
   if (const char* env = std::getenv("MX_HOST_THREADS"))
     c->nthreads = std::max(1, std::atoi(env));
+  if (const char* env = std::getenv("MX_FREQ_INTERVALS"))
+    c->freq_intervals = std::max(2, std::min(FREQ_INTERVALS, std::atoi(env)));
   if (const char* env = std::getenv("MX_TS_EARLY_SHELLS"))
     c->early_shells = std::atoi(env) != 0;
 
@@ -2683,6 +2690,8 @@ int mx_set_redshifts(mx_ctx* ctx, const double* zz, int32_t n_snaps)
 int32_t mx_n_sfr_histories(const mx_ctx* ctx) { return ctx ? ctx->n_hist : -1; }
 
 int32_t mx_fft_x_tile_threads(const mx_ctx* ctx) { return ctx && ctx->fused_fft ? ctx->x_threads : 0; }
+
+int32_t mx_freq_fallbacks(const mx_ctx* ctx) { return ctx ? ctx->freq_fallbacks : 0; }
 
 int32_t mx_zpass_blocks_per_sm(const mx_ctx* ctx)
 {
