@@ -53,14 +53,14 @@ _C256, _N256 = 256 * 256 * 129, 256 ** 3
 PAD_512_OVER_256 = (272 / 257) / (144 / 129)
 DRAM_PER_ALGORITHMIC = {
     # 5 unfiltered spectra read, 20 written; algorithmic 8 C G (1 + n_radii)
-    "fft_x_filter": (0.377542e9 + 1.452510e9) / (8 * _C256 * 5 * 5) * PAD_512_OVER_256,
+    "fft_x_filter": (0.378534e9 + 1.470662e9) / (8 * _C256 * 5 * 5) * PAD_512_OVER_256,
     # 20 spectra read and written; algorithmic 16 C per spectrum
-    "fft_y": (1.509980e9 + 1.447947e9) / (16 * _C256 * 20) * PAD_512_OVER_256,
+    "fft_y": (1.510010e9 + 1.449974e9) / (16 * _C256 * 20) * PAD_512_OVER_256,
     # 20 spectra read (the state read of 8 B per cell taken out)
-    "fft_z_threshold": (1.644234e9 + 3.307264e6 - 8 * _N256) / (8 * _C256 * 20) * PAD_512_OVER_256,
-    # 19 shells: spectra read, shells written
-    "fft_z_store": (1.434571e9 + 1.234466e9) / ((8 * _C256 + 4 * _N256) * 19),
-    "k_evolve": (2.887466e9 + 0.196168e9) / (46 * 4 * _N256),
+    "fft_z_threshold": (1.644290e9 + 3.681792e6 - 8 * _N256) / (8 * _C256 * 20) * PAD_512_OVER_256,
+    # 20 shells: 43 tiles of 16 columns per row read, shells written
+    "fft_z_store": (0.360848e9 + 1.283363e9) / (8 * 16 * 256 * 256 * 43 + 4 * _N256 * 20),
+    "k_evolve": (2.887166e9 + 0.196635e9) / (46 * 4 * _N256),
 }
 THRESHOLD_STATE_BYTES_PER_CELL = 8
 

@@ -213,8 +213,9 @@ int mx_batch_run(mx_batch* batch, mx_batch_item* items, int32_t n_items);
  * context (kept between runs while its position's configuration stays the
  * same, with the per-box history cleared); one capture puts each item's
  * host->device copies, its step (ComputeTs -> find_HII_bubbles -> 21cm box,
- * with the frequency tables built by a host node) and its device->host copies
- * on a branch of the graph, and a single cudaGraphLaunch runs every box.  The
+ * a host node fills the constants that the frequency tables enter) and its
+ * device->host copies on a branch of the graph, and a single cudaGraphLaunch runs
+ * every box.  The
  * host grids must be page-locked (cudaHostAlloc / cudaHostRegister), as the
  * graph's copy nodes need pinned memory; other grids return MX_EINVAL.
  * Results equal those of mx_step per box.  No reference counterpart (the
@@ -269,7 +270,8 @@ int mx_step_device(mx_ctx* ctx, int32_t snapshot, const mx_grids* dev, mx_global
 /* With on != 0, each later mx_step_device call captures the whole step
  * (ComputeTs, find_HII_bubbles, the 21cm box) into one CUDA graph on the
  * context's stream and launches it on `stream`; ComputeTs's frequency tables
- * are built by a host node of the graph while the shells are smoothed.  The
+ * are built on a branch of the graph, whose host node fills the constants that they
+ * enter, while the shells are smoothed.  The
  * grids and globals equal those of the uncaptured step bit for bit.  Each
  * call captures anew (kernel arguments depend on the snapshot); per-kernel
  * profiling records its events as event nodes of the graph.  No reference

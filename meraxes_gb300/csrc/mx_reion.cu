@@ -182,7 +182,8 @@ struct mx_ctx
   // the device land in pinned slots of h_stage and the code that uses them
   // (`finishers`) runs after the graph has completed; host data uploaded by
   // the step is staged in h_stage too, so that it outlives the capture.
-  // ComputeTs's frequency tables are built by a host node of the graph.
+  // A host node of the graph fills the constants that ComputeTs's frequency
+  // tables enter.
   bool graph_on = false;
   bool capturing = false;
   unsigned char* h_stage = nullptr;  // pinned, STAGE_BYTES
