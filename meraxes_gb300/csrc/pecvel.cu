@@ -28,53 +28,85 @@ thread_local int pv_launches = 0;
 constexpr double FRACT_FLOAT_ERR_D = 1e-7;
 constexpr double MPC_CM = 3.086e24;
 
-// The float nearest to c x, c a double held as two floats (c = hi + lo): one
-// rounding of the exact x hi + x lo but for the last place of x lo, so the
-// result equals (float)(c * (double)x) unless that lies within 2^-48 of a tie.
-// Two FP32 operations instead of two conversions and a product at the FP64
-// rate (the FP64 form took 0.50 ms in k_vel_convert and, with its quotient,
-// 0.41 ms in k_vel_grad_k at 256^3).  An infinite x keeps its sign and stays
-// infinite, as in FP64: x lo alone would be NaN or of the other sign.
-struct Scale2
+// Products of a float with double factors one after another, each rounded to float.
+// A factor is held as two floats and a power of two, c = (hi + lo) 2^e with hi in
+// [1/2, 1]: the product is one rounding of the exact x hi + x lo but for the last place
+// of x lo, so it equals (float)(c * (double)x) unless that lies within 2^-48 of a tie.
+// That holds while x lo and the products are normal floats (the powers of two wait for
+// the end): for `least` <= |x| <= `most` on the way in (1e-19 to 1e37 km/s for the
+// units, from 1e-29 for the gradient).  Zeros are kept, and what lies outside
+// (infinities and NaN too) takes the products in FP64, out of line.  Two FP32 operations
+// a factor instead of two conversions and a product at the FP64 rate (the FP64 form took
+// 0.50 ms in k_vel_convert and, with its quotient, 0.41 ms in k_vel_grad_k at 256^3, this
+// one 79 and 31 us).
+template <int N>
+struct Scales
 {
-  float hi, lo;
-  Scale2() = default;
-  __host__ explicit Scale2(double c) : hi((float)c), lo((float)(c - (double)(float)c)) {}
+  float hi[N], lo[N], pow2, least = 0.0f, most = FLT_MAX;
+  double c[N];
+
+  __host__ explicit Scales(const double (&factors)[N])
+  {
+    double product = 1.0, mantissas = 1.0;
+    int exponents = 0;
+    for (int i = 0; i < N; i++) {
+      int e;
+      const double m = std::frexp(factors[i], &e);
+      c[i] = factors[i];
+      hi[i] = (float)m;
+      lo[i] = (float)(m - (double)hi[i]);
+      product *= c[i];
+      mantissas *= m;
+      exponents += e;
+      // lo is 2^-26 of hi or nothing, and every product is within the floats
+      least = std::max({ least, (float)(0x1p-99 / mantissas), (float)(0x1p-125 / product) });
+      most = std::min(most, (float)std::min(0x1p127 / product, (double)FLT_MAX));
+    }
+    pow2 = std::ldexp(1.0f, exponents);
+  }
+  __device__ __forceinline__ bool takes(float x) const
+  {
+    const float a = fabsf(x);
+    return (a >= least && a <= most) || x == 0.0f;
+  }
   __device__ __forceinline__ float operator()(float x) const
   {
-    const float p = __fmul_rn(x, lo);
-    return __fmaf_rn(x, hi, fabsf(x) <= FLT_MAX ? p : 0.0f);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      x = __fmaf_rn(x, hi[i], __fmul_rn(x, lo[i]));
+    return __fmul_rn(x, pow2);
   }
 };
-
-// The unit factors in the reference's order, each rounded to float.
-struct VelScales
+template <int N>
+__device__ __noinline__ float scales_fp64(const Scales<N>& s, float x)
 {
-  Scale2 f[3];
-  int n;
-};
+  for (int i = 0; i < N; i++)
+    x = (float)(s.c[i] * (double)x);
+  return x;
+}
 
-__global__ void k_vel_convert(float* vel, VelScales sc, int D, int H, long long N)
+// the unit factors in the reference's order
+template <int NF>
+__global__ void k_vel_convert(float* vel, const __grid_constant__ Scales<NF> units, int D, int H, long long N)
 {
   for (long long ir = blockIdx.x * (long long)blockDim.x + threadIdx.x; ir < N; ir += (long long)gridDim.x * blockDim.x) {
     const long long row = row_of(ir, D);
     const long long ip = row * 2LL * H + (ir - row * D);
-    float v = vel[ip];
-    for (int i = 0; i < sc.n; i++)
-      v = sc.f[i](v);
-    vel[ip] = v;
+    const float v = vel[ip];
+    vel[ip] = units.takes(v) ? units(v) : scales_fp64(units, v);
   }
 }
 
 // c /= N; c *= h (each rounded to float); c *= (0 + i k_z) as a float complex
-// product.  1/N = inv_n * pow2 with inv_n in [1, 2), so that the low part of
-// the factor stays a normal float.
-__global__ void k_vel_grad_k(float2* spec, int H, long long C, Scale2 inv_n, float pow2, Scale2 hubble_h, float delta_k)
+// product
+__global__ void k_vel_grad_k(float2* spec, int H, long long C, const __grid_constant__ Scales<2> scales, float delta_k)
 {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < C; i += (long long)gridDim.x * blockDim.x) {
     float2 v = spec[i];
-    v.x = hubble_h(inv_n(v.x) * pow2);
-    v.y = hubble_h(inv_n(v.y) * pow2);
+    if (scales.takes(v.x) && scales.takes(v.y))
+      v = make_float2(scales(v.x), scales(v.y));
+    else
+      v = make_float2(scales_fp64(scales, v.x), scales_fp64(scales, v.y));
     const int nz = (int)(i % H);
     const float kz = __fmul_rn((float)nz, delta_k);
     // (a + i b)(0 + i k): real a*0 - b*k, imaginary a*k + b*0
@@ -452,23 +484,18 @@ __global__ void __launch_bounds__(RSD_THREADS)
 
 void launch_vel_convert(float* vel, int trees_id, float redshift, const GridDims& gd, cudaStream_t s)
 {
-  VelScales sc{};
-  if (trees_id == 1)
-    sc.f[sc.n++] = Scale2(std::sqrt(1. / (1. + redshift)) / 1000.);
-  else if (trees_id == 0 || trees_id == 2)
-    sc.f[sc.n++] = Scale2(1. + redshift);
-  sc.f[sc.n++] = Scale2(1000. * 100. / MPC_CM);
-  sc.f[sc.n++] = Scale2(1. / (1. / (1. + redshift)));
-  k_vel_convert<<<RED_BLOCKS, RED_THREADS, 0, s>>>(vel, sc, gd.D, gd.H, gd.N);
+  const double first = trees_id == 1 ? std::sqrt(1. / (1. + redshift)) / 1000. : 1. + redshift;
+  const double mpc = 1000. * 100. / MPC_CM, comoving = 1. / (1. / (1. + redshift));
+  if (trees_id >= 0 && trees_id <= 2)
+    k_vel_convert<<<RED_BLOCKS, RED_THREADS, 0, s>>>(vel, Scales<3>({ first, mpc, comoving }), gd.D, gd.H, gd.N);
+  else
+    k_vel_convert<<<RED_BLOCKS, RED_THREADS, 0, s>>>(vel, Scales<2>({ mpc, comoving }), gd.D, gd.H, gd.N);
   pv_launches++;
 }
 
 void launch_vel_grad_k(float2* spec, const GridDims& gd, double hubble_h, float delta_k, cudaStream_t s)
 {
-  int e;
-  const double m = std::frexp(1.0 / (double)gd.N, &e);
-  k_vel_grad_k<<<RED_BLOCKS, RED_THREADS, 0, s>>>(spec, gd.H, gd.C, Scale2(2.0 * m), std::ldexp(1.0f, e - 1),
-                                                  Scale2(hubble_h), delta_k);
+  k_vel_grad_k<<<RED_BLOCKS, RED_THREADS, 0, s>>>(spec, gd.H, gd.C, Scales<2>({ 1.0 / (double)gd.N, hubble_h }), delta_k);
   pv_launches++;
 }
 
